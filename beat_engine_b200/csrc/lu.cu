@@ -29,6 +29,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "internal.cuh"
 
@@ -978,38 +979,54 @@ __global__ void __launch_bounds__(256, 2) panel_update_kernel(Cx<float> *A, int6
 }
 
 // ---------------------------------------------------------------------------
-// Sub-panel factorisation on one thread-block cluster.  CP_CTAS CTAs hold all
-// rows of a w-column sub-panel (256-byte rows) in shared memory; rows never
-// move: each row carries its logical position, and an interchange only swaps
-// two positions.  Per column j:
-//   1. wait on this CTA's mbarrier until every CTA's candidate for column j
-//      (magnitude, position, and the whole candidate row, finished through
-//      step j - 1) has landed in this CTA's shared memory;
-//   2. every warp picks the same winner from the CP_CTAS candidates
+// Sub-panel factorisation on one thread-block cluster of C CTAs (16, or 1 for
+// few rows).  A thread keeps RPT whole 256-byte rows (32 c64 or 16 c128
+// columns, 64 registers each), as pairs of columns with the real and the
+// imaginary parts packed (one FP32 instruction then updates both columns), so
+// eliminating a column touches shared memory only for the broadcast pivot row.
+// Rows past RPT per thread (EXTRA) stay in shared memory.  Rows never move:
+// each carries its logical position, and an interchange only swaps two
+// positions.
+//
+// The loop over columns advances two at a time: the even column is the first
+// half of the thread's first pair, the odd one the second half, and the odd
+// step shifts the pairs down by one as it updates them, so the register
+// indices are compile-time constants in a loop body of fixed length.  Four
+// phases of W / 4 columns drop the finished pairs from the body.  Per column j:
+//   1. C > 1: wait on this CTA's mbarrier until every CTA's candidate for
+//      column j (key: magnitude, position, reciprocal of the pivot; and the
+//      whole candidate row) has landed; every warp picks the same winner
 //      (redux.sync on the magnitude bits, then the smallest position);
-//   3. look-ahead: multipliers of column j and column j + 1 of every
-//      remaining row, each thread's best row, each warp's best row finished
-//      through step j into a staging buffer by the warp's lanes;
-//   4. one CTA barrier, the CTA's best row among the warps' rows, and warp q
-//      pushes it to CTA q (one 16-byte st.async per lane, complete_tx on the
-//      receiver's mbarrier);
-//   5. the remaining columns of step j are eliminated while the pushes fly.
-// Candidate slots and mbarriers rotate over three columns: a CTA still
-// eliminating column j - 1 reads that column's slot after it has pushed its
-// candidate for column j, so a peer that holds every candidate for j may push
-// j + 1, but never j + 2, before the slot of j - 1 is free.  The staging
-// buffers and the warp results alternate with the column parity: the one CTA
-// barrier of a column separates their writers from the previous readers.
-// Every wait is bounded.
+//   2. the multiplier and column j + 1 of each row; each warp's best row's key
+//      to shared memory; a CTA barrier; every warp picks the CTA's best;
+//   3. the best row's thread writes the row as it stands before this step to
+//      the staging buffer, and its warp's lanes finish it there, a pair each;
+//      a second CTA barrier; the warps push it to every CTA (16 bytes per
+//      lane, st.async, complete_tx on the receiver's mbarrier).  With C = 1 the
+//      staging buffer is what every thread reads next: no exchange;
+//   4. every thread eliminates the rest of step j while the pushes fly.
+// Multipliers and retired pivot rows go to a shared-memory copy of the
+// sub-panel, which the bulk-copy engine loaded and stores at the end; rank 0
+// keeps the pivot rows' multipliers (L11) and inverts them during that store.
+//
+// Slots and mbarriers rotate over three columns: a CTA's slowest warps read
+// the slot of column j after the CTA pushed its candidate for j + 1, and finish
+// before it pushes j + 2; a peer pushes j + 3, which reuses the slot, only once
+// it holds every candidate for j + 2.  Staging buffers and warp keys alternate
+// with the column parity, separated by the column's CTA barriers.  Every wait
+// is bounded.
+//
+// Bound: the dependent chain of one pivot per column (the exchange between
+// CTAs, two argmax reductions, two barriers), at about five cycles an
+// instruction: one warp per scheduler while the rows allow it, and no more
+// on the chain than the candidate's own row.  Measured on a B200, the whole
+// factorisation, against rows kept in shared memory by 512 threads of 16 CTAs
+// whatever their number: FP32 N = 162 0.60 -> 0.41 ms, N = 1,390 4.17 -> 2.65,
+// N = 10,242 38.1 -> 32.2; FP64 N = 998 3.04 -> 2.83.
 // ---------------------------------------------------------------------------
-constexpr int CP_CTAS = 16, CP_THREADS = 512, CP_WARPS = CP_THREADS / 32, CP_RMAX = 2, CP_ROW_BYTES = 272,
-              CP_SLOTS = 3;
-static_assert(CP_WARPS == CP_CTAS, "warp q pushes to CTA q");
+constexpr int CP_CTAS = 16, CP_THREADS = 256, CP_WARPS = CP_THREADS / 32, CP_ROW_BYTES = 272, CP_SLOTS = 3;
+constexpr int CP_ONE_CTA = 256;  // rows up to which one CTA alone factors the sub-panel
 constexpr int CP_NONE = 0x7fffffff;  // position of "no candidate"
-
-struct alignas(16) PivKey {
-    uint32_t w[4];  // magnitude bits (lo, hi), position, unused
-};
 
 __device__ __forceinline__ uint32_t cl_rank() {
     uint32_t r;
@@ -1073,120 +1090,179 @@ __device__ __forceinline__ void st_async16(uint32_t addr, uint4 v, uint32_t bar)
 }
 
 // ordered bits of a non-negative magnitude (0 also stands for "none")
-__device__ __forceinline__ uint64_t mag_bits(float v) { return (uint64_t)__float_as_uint(v); }
+__device__ __forceinline__ uint32_t mag_bits(float v) { return __float_as_uint(v); }
 __device__ __forceinline__ uint64_t mag_bits(double v) { return (uint64_t)__double_as_longlong(v); }
-template <typename T> __device__ __forceinline__ T mag_value(uint64_t b);
-template <> __device__ __forceinline__ float mag_value<float>(uint64_t b) { return __uint_as_float((uint32_t)b); }
-template <> __device__ __forceinline__ double mag_value<double>(uint64_t b) { return __longlong_as_double((long long)b); }
+__device__ __forceinline__ float mag_value(uint32_t b) { return __uint_as_float(b); }
+__device__ __forceinline__ double mag_value(uint64_t b) { return __longlong_as_double((long long)b); }
 
 // lane holding the largest magnitude, the smallest position among equals
 // (all 32 lanes take part; the result is the same in every lane)
-template <typename T> __device__ __forceinline__ int warp_argbest(uint64_t m, int pos) {
+template <typename M> __device__ __forceinline__ int warp_argbest(M m, int pos) {
     bool tie;
-    if (sizeof(T) == 8) {
+    if constexpr (sizeof(M) == 8) {
         const uint32_t hi = (uint32_t)(m >> 32), lo = (uint32_t)m;
         const uint32_t mhi = __reduce_max_sync(0xffffffffu, hi);
         const uint32_t mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
         tie = hi == mhi && lo == mlo;
     } else {
-        const uint32_t mm = __reduce_max_sync(0xffffffffu, (uint32_t)m);
-        tie = (uint32_t)m == mm;
+        tie = m == __reduce_max_sync(0xffffffffu, m);
     }
     const unsigned ties = __ballot_sync(0xffffffffu, tie);
-    if (__popc(ties) == 1) return __ffs(ties) - 1;  // one largest magnitude: no position to compare
+    if ((ties & (ties - 1u)) == 0u) return __ffs(ties) - 1;  // one largest magnitude: no position to compare
     const int mpos = __reduce_min_sync(0xffffffffu, tie ? pos : CP_NONE);
     return __ffs(__ballot_sync(0xffffffffu, tie && pos == mpos)) - 1;
 }
 
-// 16 bytes of a row: 2 c64 or 1 c128 entries
-__device__ __forceinline__ float4 v16_ld(const Cx<float> *p) { return *reinterpret_cast<const float4 *>(p); }
-__device__ __forceinline__ double2 v16_ld(const Cx<double> *p) { return *reinterpret_cast<const double2 *>(p); }
-__device__ __forceinline__ void v16_st(Cx<float> *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
-__device__ __forceinline__ void v16_st(Cx<double> *p, double2 v) { *reinterpret_cast<double2 *>(p) = v; }
-__device__ __forceinline__ float4 v16_cms(float4 x, Cx<float> l, float4 u) {
-    const Cx<float> a = cms(Cx<float>{x.x, x.y}, l, Cx<float>{u.x, u.y});
-    const Cx<float> b = cms(Cx<float>{x.z, x.w}, l, Cx<float>{u.z, u.w});
-    return make_float4(a.re, a.im, b.re, b.im);
+// Two columns of a row, real and imaginary parts as packed pairs, and a
+// multiplier for them.  FP32 packs a pair into one 64-bit register operand
+// (fma.rn.f32x2).  In shared memory a pair is (re0, re1, im0, im1).
+template <typename T> struct ColPair;
+template <typename T> struct ColMult;
+template <> struct alignas(16) ColPair<float> { unsigned long long re, im; };
+template <> struct alignas(16) ColPair<double> { double re[2], im[2]; };
+template <> struct ColMult<float> { unsigned long long nr, i, ni; };  // (-l.re, -l.re), (l.im, l.im), (-l.im, -l.im)
+template <> struct ColMult<double> { double r, i; };
+__device__ __forceinline__ unsigned long long f2_pack(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
 }
-__device__ __forceinline__ double2 v16_cms(double2 x, Cx<double> l, double2 u) {
-    const Cx<double> a = cms(Cx<double>{x.x, x.y}, l, Cx<double>{u.x, u.y});
-    return make_double2(a.re, a.im);
+__device__ __forceinline__ void f2_unpack(unsigned long long v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
-
-// row[c] -= l prow[c] for c in [c0, w); row and prow 16-byte aligned, w even
-// for c64 entries
-template <typename T> __device__ __forceinline__ void row_update(Cx<T> *row, const Cx<T> *prow, Cx<T> l, int c0, int w) {
-    constexpr int E = 16 / sizeof(Cx<T>);
-    int c = c0;
-    if (E == 2 && (c & 1) && c < w) {
-        row[c] = cms(row[c], l, prow[c]);
-        ++c;
-    }
-    for (; c < w; c += 4 * E) {
-        decltype(v16_ld(row)) x[4], u[4];
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ ColPair<float> pair_ld(const unsigned char *p, float) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(p);
+    return ColPair<float>{v.x, v.y};
+}
+__device__ __forceinline__ ColPair<double> pair_ld(const unsigned char *p, double) {
+    const double2 a = reinterpret_cast<const double2 *>(p)[0], b = reinterpret_cast<const double2 *>(p)[1];
+    return ColPair<double>{{a.x, a.y}, {b.x, b.y}};
+}
+__device__ __forceinline__ void pair_st(unsigned char *p, const ColPair<float> &v) {
+    *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(v.re, v.im);
+}
+__device__ __forceinline__ void pair_st(unsigned char *p, const ColPair<double> &v) {
+    reinterpret_cast<double2 *>(p)[0] = make_double2(v.re[0], v.re[1]);
+    reinterpret_cast<double2 *>(p)[1] = make_double2(v.im[0], v.im[1]);
+}
+template <int H> __device__ __forceinline__ Cx<float> pair_get(const ColPair<float> &v) {
+    float r0, r1, i0, i1;
+    f2_unpack(v.re, r0, r1);
+    f2_unpack(v.im, i0, i1);
+    return H ? Cx<float>{r1, i1} : Cx<float>{r0, i0};
+}
+template <int H> __device__ __forceinline__ Cx<double> pair_get(const ColPair<double> &v) {
+    return Cx<double>{v.re[H], v.im[H]};
+}
+__device__ __forceinline__ ColPair<float> pair_make(Cx<float> a, Cx<float> b) {
+    return ColPair<float>{f2_pack(a.re, b.re), f2_pack(a.im, b.im)};
+}
+__device__ __forceinline__ ColPair<double> pair_make(Cx<double> a, Cx<double> b) {
+    return ColPair<double>{{a.re, b.re}, {a.im, b.im}};
+}
+__device__ __forceinline__ ColMult<float> pair_mult(Cx<float> l) {
+    return ColMult<float>{f2_pack(-l.re, -l.re), f2_pack(l.im, l.im), f2_pack(-l.im, -l.im)};
+}
+__device__ __forceinline__ ColMult<double> pair_mult(Cx<double> l) { return ColMult<double>{l.re, l.im}; }
+// x - l u
+__device__ __forceinline__ ColPair<float> pair_cms(const ColPair<float> &x, const ColMult<float> &l,
+                                                   const ColPair<float> &u) {
+    return ColPair<float>{f2_fma(l.i, u.im, f2_fma(l.nr, u.re, x.re)), f2_fma(l.ni, u.re, f2_fma(l.nr, u.im, x.im))};
+}
+__device__ __forceinline__ ColPair<double> pair_cms(const ColPair<double> &x, const ColMult<double> &l,
+                                                    const ColPair<double> &u) {
+    ColPair<double> d;
 #pragma unroll
-        for (int t = 0; t < 4; ++t)
-            if (c + t * E < w) {
-                x[t] = v16_ld(row + c + t * E);
-                u[t] = v16_ld(prow + c + t * E);
-            }
-#pragma unroll
-        for (int t = 0; t < 4; ++t)
-            if (c + t * E < w) v16_st(row + c + t * E, v16_cms(x[t], l, u[t]));
+    for (int h = 0; h < 2; ++h) {
+        d.re[h] = fma(l.i, u.im[h], fma(-l.r, u.re[h], x.re[h]));
+        d.im[h] = fma(-l.i, u.re[h], fma(-l.r, u.im[h], x.im[h]));
     }
+    return d;
 }
 
 template <typename T> struct ClusterPanelArgs {
     Cx<T> *A;
     int64_t ld;
-    int n, k, w;  // sub-panel: rows [k, n), columns [k, k + w)
+    int n, k;     // sub-panel: rows [k, n), columns [k, k + W), W = 256 / sizeof(Cx<T>)
     int rpc;      // rows per CTA
     int *ipiv;
     int *status;
-    Cx<T> *dinv;  // inverse of the unit lower w x w diagonal block (nullptr: not wanted)
-    int xc0, xc1; // the panel's columns: the interchanges go to [xc0, xc1) outside [k, k + w) as well
+    Cx<T> *dinv;  // inverse of the unit lower W x W diagonal block (nullptr: not wanted)
+    int xc0, xc1; // the panel's columns: the interchanges go to [xc0, xc1) outside [k, k + W) as well
                   // (xc0 == xc1: the caller swaps the other columns itself)
     uint64_t timeout_ns;
 };
 
-// values per thread that the interchange of the panel's other columns holds
-// between its read and write phases: moved rows (<= 2 w) x columns (< nb)
-template <typename T> struct CpMove { static constexpr int V = sizeof(T) == 4 ? 12 : 8; };
-constexpr int CP_MAXMOVED = 64;
+template <typename T> struct CpShape {
+    static constexpr int W = 256 / sizeof(Cx<T>);        // columns
+    static constexpr int NP = W / 2;                      // column pairs
+    static constexpr int PB = 256 / NP;                   // bytes of a pair
+    static constexpr int KB = sizeof(T) == 4 ? 16 : 32;   // bytes of a key: magnitude, position, reciprocal
+    // a slot's row: NP pairs, then the pairs a phase's last columns read past the row's end (unused values)
+    static constexpr int RSL = 256 + (NP / 4 - 1) * PB;
+    // The interchange of the panel's other columns: at most 2 W moved rows, MVC
+    // 16-byte chunks (or fewer) each, MVT values per thread of 128 or more
+    static constexpr int MVC = sizeof(T) == 4 ? 64 : 128, MVT = 2 * W * MVC / 128;
+    // shared memory for rpc rows on C CTAs, `extra` of them not in registers
+    static size_t smem(int rpc, int C, int extra) {
+        return (size_t)rpc * CP_ROW_BYTES + (size_t)(RSL + KB) * (CP_SLOTS * C + 2) +
+               sizeof(Cx<T>) * 2 * W * (W + 1) + sizeof(int) * (size_t)extra;
+    }
+};
 
-template <typename T>
-__global__ void __launch_bounds__(CP_THREADS) cluster_panel_kernel(ClusterPanelArgs<T> a) {
+template <typename T, int RPT, bool EXTRA>
+__global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPanelArgs<T> a) {
+    using S = CpShape<T>;
+    using M = decltype(mag_bits(T(0)));
+    constexpr int W = S::W, NPM = S::NP, PB = S::PB, KB = S::KB, RSL = S::RSL;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int RS = CP_ROW_BYTES / sizeof(Cx<T>);  // padded row stride (entries)
-    const int w = a.w, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    Cx<T> *P = reinterpret_cast<Cx<T> *>(smem_raw);                                    // rpc x RS
-    Cx<T> *slot_row = P + (size_t)a.rpc * RS;                                           // [CP_SLOTS][CP_CTAS][w]
-    Cx<T> *wbuf = slot_row + CP_SLOTS * CP_CTAS * w;                                    // [2][CP_WARPS][w]
-    Cx<T> *ublk = wbuf + 2 * CP_WARPS * w;                                              // w x (w + 1): L11^-1 (CTA 0)
-    PivKey *slot_key = reinterpret_cast<PivKey *>(ublk + w * (w + 1));                 // [CP_SLOTS][CP_CTAS]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, NT = (int)blockDim.x, NW = NT >> 5;
+    const uint32_t rank = cl_rank();
+    const int C = (int)gridDim.x;  // one cluster
+    unsigned char *slot_row = smem_raw;                            // [CP_SLOTS][C][RSL]
+    unsigned char *stage = slot_row + (size_t)CP_SLOTS * C * RSL;  // [2][RSL]
+    unsigned char *slot_key = stage + 2 * RSL;                     // [CP_SLOTS][C][KB]
+    unsigned char *stage_key = slot_key + (size_t)CP_SLOTS * C * KB;  // [2][KB]
+    Cx<T> *l11 = reinterpret_cast<Cx<T> *>(stage_key + 2 * KB);    // W x (W + 1): L11 (rank 0)
+    Cx<T> *y11 = l11 + W * (W + 1);                                // W x (W + 1): its inverse
+    unsigned char *P = reinterpret_cast<unsigned char *>(y11 + W * (W + 1));  // rpc rows of CP_ROW_BYTES, complex
+    int *xpos = reinterpret_cast<int *>(P + (size_t)a.rpc * CP_ROW_BYTES);    // EXTRA: positions of those rows
+    struct alignas(16) Key {  // a warp's best row
+        M m;
+        int pos, li;
+    };
     __shared__ uint64_t mbar[CP_SLOTS];
     __shared__ uint64_t ldbar;  // the sub-panel's rows landed in shared memory
-    __shared__ uint64_t red_m[2][CP_WARPS];
-    __shared__ int red_pos[2][CP_WARPS];
+    __shared__ Key red[2][CP_WARPS];
     __shared__ int s_abort[2];
-    const uint32_t rank = cl_rank();
     const int gr0 = a.k + (int)rank * a.rpc;
     const int nrows = max(0, min(a.rpc, a.n - gr0));
-    const int jmax = min(w, a.n - a.k);
-    const int nd = w * (int)sizeof(Cx<T>) / 16;  // data lanes of a push
-    const unsigned step_bytes = CP_CTAS * (unsigned)(w * sizeof(Cx<T>) + sizeof(PivKey));
-    const uint32_t row_bytes = (uint32_t)(w * sizeof(Cx<T>));
+    const int jmax = min(W, a.n - a.k);
+    const unsigned step_bytes = (unsigned)C * (256 + KB);
+    auto row_at = [&](int i) { return reinterpret_cast<Cx<T> *>(P + (size_t)i * CP_ROW_BYTES); };
     if (tid == 0) {
         mb_init(&ldbar, 1);
         for (int b = 0; b < CP_SLOTS; ++b) mb_init(&mbar[b], 1);
         mb_init_fence();
-        mb_arrive_expect(&ldbar, (unsigned)nrows * row_bytes);
+        mb_arrive_expect(&ldbar, (unsigned)nrows * 256u);
         for (int b = 0; b < CP_SLOTS; ++b) mb_arrive_expect(&mbar[b], step_bytes);  // columns 0, 1, 2
         s_abort[0] = s_abort[1] = 0;
     }
     __syncthreads();
-    for (int i = tid; i < nrows; i += CP_THREADS)  // rows in flight all at once
-        bulk_g2s(sm_addr(P + (size_t)i * RS), a.A + (int64_t)(gr0 + i) * a.ld + a.k, row_bytes, sm_addr(&ldbar));
+    for (int i = tid; i < nrows; i += NT)  // rows in flight all at once
+        bulk_g2s(sm_addr(row_at(i)), a.A + (int64_t)(gr0 + i) * a.ld + a.k, 256u, sm_addr(&ldbar));
+    // the warp's share of the pushes: CTAs warp, warp + NW, ...; a peer's
+    // shared::cluster address is this CTA's plus a constant
+    constexpr int PUSH = 4;  // NW >= 4
+    uint32_t peer[PUSH];
+#pragma unroll
+    for (int i = 0; i < PUSH; ++i)
+        peer[i] = warp + i * NW < C ? cl_map(sm_addr(smem_raw), warp + i * NW) - sm_addr(smem_raw) : 0u;
     if (!mb_try(&ldbar, 0u)) {
         const uint64_t t0 = global_ns();
         while (!mb_try(&ldbar, 0u))
@@ -1195,286 +1271,411 @@ __global__ void __launch_bounds__(CP_THREADS) cluster_panel_kernel(ClusterPanelA
                 break;
             }
     }
-    int mp[CP_RMAX];  // logical position of local rows tid + r * CP_THREADS (-1: none)
+    // logical positions of this thread's register rows (local rows tid + r NT;
+    // -1: none) and, in xpos, of the shared-memory rows (local rows x0 + i)
+    const int x0 = RPT * NT, nx = EXTRA ? max(0, nrows - x0) : 0;
+    int mp[RPT];
+    ColPair<T> A[RPT][NPM];
 #pragma unroll
-    for (int r = 0; r < CP_RMAX; ++r) {
-        const int i = tid + r * CP_THREADS;
+    for (int r = 0; r < RPT; ++r) {
+        const int i = tid + r * NT;
         mp[r] = i < nrows ? gr0 + i : -1;
-    }
-
-    // the warp's best row (given each thread's best) into the staging buffer
-    // `pb`, finished through step jprev (multiplier in column jprev, written by
-    // its owner lane), and the warp's result into red_*[pb]
-    auto warp_stage = [&](uint64_t m, int pos, int li, int pb, int jprev, const Cx<T> *prow_prev) -> int {
-        const int wl = warp_argbest<T>(m, pos);
-        const int wpos = __shfl_sync(0xffffffffu, pos, wl);
-        const int wli = __shfl_sync(0xffffffffu, li, wl);
-        const uint64_t wm = __shfl_sync(0xffffffffu, m, wl);
-        __syncwarp();
-        if (wpos != CP_NONE) {
-            Cx<T> *row = P + (size_t)wli * RS;
-            Cx<T> *dst = wbuf + (size_t)(pb * CP_WARPS + warp) * w;
-            for (int c = lane; c < w; c += 32) {
-                Cx<T> x = row[c];
-                if (jprev >= 0 && c >= jprev + 2) {
-                    x = cms(x, row[jprev], prow_prev[c]);
-                    row[c] = x;
-                }
-                dst[c] = x;
-            }
-        }
-        if (lane == 0) {
-            red_m[pb][warp] = wm;
-            red_pos[pb][warp] = wpos;
-        }
-        return wpos != CP_NONE ? wli : -1;
-    };
-    // after the CTA barrier: the CTA's best among the warps' rows; warp q
-    // pushes it (slot of column s) to CTA q
-    auto push = [&](int s, int pb) {
-        const uint64_t m = lane < CP_WARPS ? red_m[pb][lane] : 0ull;
-        const int pos = lane < CP_WARPS ? red_pos[pb][lane] : CP_NONE;
-        const int bw = warp_argbest<T>(m, pos);
-        const uint64_t cm = __shfl_sync(0xffffffffu, m, bw);
-        const int cpos = __shfl_sync(0xffffffffu, pos, bw);
-        const int ps = s % CP_SLOTS;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        uint32_t dst = 0;
-        if (lane < nd) {
-            if (cpos != CP_NONE) v = reinterpret_cast<const uint4 *>(wbuf + (size_t)(pb * CP_WARPS + bw) * w)[lane];
-            dst = sm_addr(slot_row + (size_t)(ps * CP_CTAS + rank) * w) + 16u * lane;
-        } else if (lane == nd) {
-            v = make_uint4((uint32_t)cm, (uint32_t)(cm >> 32), (uint32_t)cpos, 0u);
-            dst = sm_addr(&slot_key[ps * CP_CTAS + rank]);
-        }
-        if (lane <= nd) st_async16(cl_map(dst, warp), v, cl_map(sm_addr(&mbar[ps]), warp));
-    };
-
-    // candidate of column 0
-    {
-        uint64_t m = 0;
-        int pos = CP_NONE, li = -1;
 #pragma unroll
-        for (int r = 0; r < CP_RMAX; ++r) {
-            const int i = tid + r * CP_THREADS;
-            if (mp[r] >= 0) {
-                const uint64_t mr = mag_bits(cabs1(P[i * RS]));
-                if (pos == CP_NONE || mr > m || (mr == m && mp[r] < pos)) {
-                    m = mr;
-                    pos = mp[r];
-                    li = i;
-                }
-            }
+        for (int q = 0; q < NPM; ++q) {
+            const Cx<T> z{T(0), T(0)};
+            A[r][q] = mp[r] >= 0 ? pair_make(row_at(i)[2 * q], row_at(i)[2 * q + 1]) : pair_make(z, z);
         }
-        warp_stage(m, pos, li, 1, -1, nullptr);
-        __syncthreads();
-        cl_sync();  // every CTA's mbarriers are initialised before any remote store
-        if (jmax > 0) push(0, 1);
     }
+    if (EXTRA)
+        for (int i = tid; i < nx; i += NT) xpos[i] = gr0 + x0 + i;  // read and swapped by the same thread
 
-    for (int j = 0; j < jmax; ++j) {
-        const int jr = a.k + j, par = j % CP_SLOTS, pb = j & 1;
-        if (!mb_try(&mbar[par], (unsigned)(j / CP_SLOTS) & 1u)) {
-            const uint64_t t0 = global_ns();
-            while (!mb_try(&mbar[par], (unsigned)(j / CP_SLOTS) & 1u)) {
-                if (global_ns() - t0 > a.timeout_ns) {
-                    s_abort[pb] = 1;
-                    atomicOr(a.status, (int)DEV_BARRIER_TIMEOUT);
-                    break;
-                }
+    // a thread's best row: magnitude, position, local row, the entry itself and
+    // the multiplier that finishes the row
+    struct Best {
+        M m = 0;
+        int pos = CP_NONE, li = 0;
+        Cx<T> y{T(0), T(0)}, l{T(0), T(0)};
+        __device__ __forceinline__ void offer(Cx<T> y1, Cx<T> l1, int pos1, int li1) {
+            const M m1 = mag_bits(cabs1(y1));
+            if (pos == CP_NONE || m1 > m || (m1 == m && pos1 < pos)) {
+                m = m1;
+                pos = pos1;
+                li = li1;
+                y = y1;
+                l = l1;
             }
         }
-        if (tid == 0 && !s_abort[pb]) mb_arrive_expect(&mbar[par], step_bytes);  // next phase: column j + 3
-        // the same winner in every warp
-        int p, wc;
-        T wv;
-        {
-            const PivKey kq = slot_key[par * CP_CTAS + (lane & (CP_CTAS - 1))];
-            const uint64_t m = lane < CP_CTAS ? ((uint64_t)kq.w[1] << 32 | kq.w[0]) : 0ull;
-            const int pos = lane < CP_CTAS ? (int)kq.w[2] : CP_NONE;
-            wc = warp_argbest<T>(m, pos) & (CP_CTAS - 1);
-            p = __shfl_sync(0xffffffffu, pos, wc);
-            wv = mag_value<T>(__shfl_sync(0xffffffffu, m, wc));
+    };
+    Key cand{0, CP_NONE, 0};  // the CTA's best row for the next column
+    // The CTA's candidate for column s (each thread's best in `b`) to the
+    // staging buffer, and from there to every CTA.  prow: the pivot row of step
+    // s - 1, which finishes the candidate's pairs from `first` on (nullptr: the
+    // rows are as loaded).  SH, NP: this thread's pairs, A[r][i] at pair
+    // (s >> 1) + i - SH.
+    auto publish = [&](auto shc, auto npc, int s, int slot, const Best &b, const unsigned char *prow) -> bool {
+        constexpr int SH = decltype(shc)::value, NP = decltype(npc)::value;
+        const int pb = s & 1, base = s >> 1;
+        const int wl = warp_argbest(b.m, b.pos);
+        if (lane == wl) red[pb][warp] = Key{b.m, b.pos, b.li};
+        __syncthreads();
+        if (s_abort[pb ^ 1]) return false;  // set before the barrier: uniform
+        const int bw = [&] {
+            const Key r = lane < NW ? red[pb][lane] : Key{0, CP_NONE, 0};
+            return warp_argbest(r.m, r.pos);
+        }();
+        cand = red[pb][bw];
+        unsigned char *buf = stage + pb * RSL;
+        if (warp == bw && cand.pos != CP_NONE) {
+            if (lane == wl) {
+                if (EXTRA && cand.li >= x0) {
+                    const Cx<T> *row = row_at(cand.li);
+                    for (int q = base; q < NPM; ++q) pair_st(buf + q * PB, pair_make(row[2 * q], row[2 * q + 1]));
+                }
+#pragma unroll
+                for (int r = 0; r < RPT; ++r)
+                    if (cand.li == tid + r * NT) {
+#pragma unroll
+                        for (int i = SH; i < NP; ++i)  // (past the row's end: the slot's padding)
+                            pair_st(buf + (base + i - SH) * PB, A[r][i]);
+                    }
+                const T den = b.y.re * b.y.re + b.y.im * b.y.im;
+                const T rd = den > T(0) ? rcp_rn(den) : T(0);
+                M *km = reinterpret_cast<M *>(stage_key + pb * KB);
+                km[0] = cand.m;
+                reinterpret_cast<int *>(km + 1)[0] = cand.pos;
+                *reinterpret_cast<Cx<T> *>(stage_key + pb * KB + KB / 2) = Cx<T>{b.y.re * rd, -b.y.im * rd};
+            }
+            if (prow) {  // a lane per pair: even s, from pair s / 2 on; odd s, after the pair that holds column s
+                const Cx<T> l{__shfl_sync(0xffffffffu, b.l.re, wl), __shfl_sync(0xffffffffu, b.l.im, wl)};
+                __syncwarp();
+                if (lane >= base + (s & 1) && lane < NPM)
+                    pair_st(buf + lane * PB, pair_cms(pair_ld(buf + lane * PB, T(0)), pair_mult(l),
+                                                      pair_ld(prow + lane * PB, T(0))));
+            }
         }
+        __syncthreads();
+        if (C == 1) return true;
+        // to every CTA: the row's first s / 2 pairs (multipliers, complex
+        // entries) from the sub-panel's copy, the rest and the key staged
+        if (lane < 16 + KB / 16) {
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            uint32_t dst;
+            if (lane < 16) {
+                const unsigned char *src = lane * 16 < base * PB ? P + (size_t)cand.li * CP_ROW_BYTES : buf;
+                if (cand.pos != CP_NONE) v = reinterpret_cast<const uint4 *>(src)[lane];
+                dst = sm_addr(slot_row) + (uint32_t)(slot * C + rank) * RSL + 16u * lane;
+            } else {
+                if (cand.pos != CP_NONE)
+                    v = reinterpret_cast<const uint4 *>(stage_key + pb * KB)[lane - 16];
+                else if (lane == 16)
+                    (sizeof(M) == 4 ? v.y : v.z) = (uint32_t)CP_NONE;
+                dst = sm_addr(slot_key) + (uint32_t)(slot * C + rank) * KB + 16u * (lane - 16);
+            }
+            const uint32_t bar = sm_addr(&mbar[slot]);
+#pragma unroll
+            for (int i = 0; i < PUSH; ++i)
+                if (warp + i * NW < C) st_async16(dst + peer[i], v, bar + peer[i]);
+        }
+        return true;
+    };
+
+    int par = 0;            // slot of the current column
+    unsigned phase = 0;     // parity of its mbarrier phase
+    bool stop = false;
+    // one column; ODD: the pivot column is the second of the first pair
+    auto step = [&](auto npc, auto oddc, int j) {
+        constexpr int NP = decltype(npc)::value;
+        constexpr int ODD = decltype(oddc)::value;
+        const int jr = a.k + j, pb = j & 1;
+        const unsigned char *prow = stage + pb * RSL, *pkey = stage_key + pb * KB;
+        const unsigned char *lrow = P + (size_t)cand.li * CP_ROW_BYTES;  // the pivot row's multipliers
+        int p = cand.pos;
+        M wm = cand.m;
+        if (C > 1) {
+            if (!mb_try(&mbar[par], phase)) {
+                const uint64_t t0 = global_ns();
+                while (!mb_try(&mbar[par], phase)) {
+                    if (global_ns() - t0 > a.timeout_ns) {
+                        s_abort[pb] = 1;
+                        atomicOr(a.status, (int)DEV_BARRIER_TIMEOUT);
+                        break;
+                    }
+                }
+            }
+            if (tid == 0 && !s_abort[pb]) mb_arrive_expect(&mbar[par], step_bytes);  // next phase: column j + 3
+            // the same winner in every warp
+            const M *km = reinterpret_cast<const M *>(slot_key + (size_t)(par * C + (lane & (C - 1))) * KB);
+            const M m = lane < C ? km[0] : M(0);
+            const int pos = lane < C ? reinterpret_cast<const int *>(km + 1)[0] : CP_NONE;
+            const int wc = warp_argbest(m, pos) & (C - 1);
+            prow = lrow = slot_row + (size_t)(par * C + wc) * RSL;
+            pkey = slot_key + (size_t)(par * C + wc) * KB;
+            wm = reinterpret_cast<const M *>(pkey)[0];
+            p = reinterpret_cast<const int *>(pkey + sizeof(M))[0];
+        }
+        const Cx<T> inv = *reinterpret_cast<const Cx<T> *>(pkey + KB / 2);
+        const unsigned char *up = prow + (j >> 1) * PB;  // the pair A[r][0] stands for
+        // the pivot row's column j + 1
+        const Cx<T> un = pair_get<1 - ODD>(pair_ld(up + ODD * PB, T(0)));
         if (p < jr || p >= a.n) {  // no candidate (or a damaged slot): keep the row in place
             p = jr;
-            wv = T(0);
+            wm = 0;
         }
-        const Cx<T> *prow = slot_row + (size_t)(par * CP_CTAS + wc) * w;
-        if (tid == 0) {
-            if (!(wv > T(0))) atomicOr(a.status, (int)DEV_ZERO_PIVOT);
-            if (rank == 0) a.ipiv[jr] = p;
-        }
-        const Cx<T> pv = prow[j];
-        const T den = pv.re * pv.re + pv.im * pv.im;
-        const T rd = den > T(0) ? rcp_rn(den) : T(0);
-        const Cx<T> inv{pv.re * rd, -pv.im * rd};
-        // interchange of positions jr and p; the pivot row retires at jr
+        const bool more = j + 1 < jmax;
+        // the interchange of positions jr and p (the pivot row retires at
+        // jr), then the look-ahead: multiplier and column j + 1 of each row
+        // (a row that is not active has multiplier 0 and keeps its values)
+        Cx<T> l[RPT];
+        Best best;
 #pragma unroll
-        for (int r = 0; r < CP_RMAX; ++r) {
+        for (int r = 0; r < RPT; ++r) {
             if (mp[r] == p)
                 mp[r] = jr;
             else if (mp[r] == jr)
                 mp[r] = p;
+            const bool act = mp[r] > jr;
+            const Cx<T> x = pair_get<ODD>(A[r][0]);
+            l[r] = cmul(x, inv);
+            if (!act) l[r] = Cx<T>{T(0), T(0)};
+            const Cx<T> y = cms(ODD ? pair_get<0>(A[r][NP > 1 ? 1 : 0]) : pair_get<1>(A[r][0]), l[r], un);
+            // the first column is final (the multiplier, or the pivot row's own entry)
+            if constexpr (!ODD) A[r][0] = pair_make(act ? l[r] : x, y);
+            if (act && more) best.offer(y, l[r], mp[r], tid + r * NT);
+            if (act) row_at(tid + r * NT)[j] = l[r];  // read by the push of the candidate that holds it
         }
-        // look-ahead: multipliers and column j + 1, with each thread's best row
-        const bool more = j + 1 < jmax;
-        uint64_t m = 0;
-        int pos = CP_NONE, li = -1;
-        {
-            Cx<T> xj[CP_RMAX], xn[CP_RMAX];
-#pragma unroll
-            for (int r = 0; r < CP_RMAX; ++r)
-                if (mp[r] > jr) {
-                    const Cx<T> *row = P + (size_t)(tid + r * CP_THREADS) * RS;
-                    xj[r] = row[j];
-                    if (more) xn[r] = row[j + 1];
-                }
-            const Cx<T> u = more ? prow[j + 1] : Cx<T>{T(0), T(0)};
-#pragma unroll
-            for (int r = 0; r < CP_RMAX; ++r)
-                if (mp[r] > jr) {
-                    const int i = tid + r * CP_THREADS;
-                    Cx<T> *row = P + (size_t)i * RS;
-                    const Cx<T> l = cmul(xj[r], inv);
-                    row[j] = l;
+        if (EXTRA)
+            for (int i = tid; i < nx; i += NT) {
+                int xp = xpos[i];
+                if (xp == p || xp == jr) xpos[i] = xp = xp == p ? jr : p;
+                if (xp > jr) {
+                    Cx<T> *row = row_at(x0 + i);
+                    const Cx<T> l1 = cmul(row[j], inv);
+                    row[j] = l1;
                     if (more) {
-                        const Cx<T> y = cms(xn[r], l, u);
-                        row[j + 1] = y;
-                        const uint64_t mr = mag_bits(cabs1(y));
-                        if (pos == CP_NONE || mr > m || (mr == m && mp[r] < pos)) {
-                            m = mr;
-                            pos = mp[r];
-                            li = i;
-                        }
+                        const Cx<T> y1 = cms(row[j + 1], l1, un);
+                        if (!ODD) row[j + 1] = y1;
+                        best.offer(y1, l1, xp, x0 + i);
                     }
                 }
+            }
+        const int nslot = par == CP_SLOTS - 1 ? 0 : par + 1;
+        if (more && !publish(oddc, npc, j + 1, nslot, best, prow)) {
+            stop = true;
+            return;
         }
-        int staged = -1;  // local row finished by this warp for the push
-        if (more) staged = warp_stage(m, pos, li, pb, j, prow);
-        __syncthreads();
-        if (s_abort[pb]) break;  // read after the barrier: uniform
-        if (more) push(j + 1, pb);
-        // rest of step j
-        const int c0 = more ? j + 2 : j + 1;
+        // the rest of this step; a retiring pivot row goes to the sub-panel's copy first
 #pragma unroll
-        for (int r = 0; r < CP_RMAX; ++r) {
-            const int i = tid + r * CP_THREADS;
-            if (mp[r] > jr && i != staged) {
-                Cx<T> *row = P + (size_t)i * RS;
-                row_update(row, prow, row[j], c0, w);
+        for (int r = 0; r < RPT; ++r)
+            if (mp[r] == jr) {
+                Cx<T> *row = row_at(tid + r * NT);
+#pragma unroll
+                for (int i = 0; i < NP; ++i) {
+                    const int q = (j >> 1) + i;
+                    if (q < NPM) {
+                        row[2 * q] = pair_get<0>(A[r][i]);
+                        row[2 * q + 1] = pair_get<1>(A[r][i]);
+                    }
+                }
             }
+        ColMult<T> lm[RPT];
+#pragma unroll
+        for (int r = 0; r < RPT; ++r) lm[r] = pair_mult(l[r]);
+#pragma unroll
+        for (int i = 1; i < NP; ++i) {
+            const ColPair<T> u = pair_ld(up + i * PB, T(0));
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) A[r][i - ODD] = pair_cms(A[r][i], lm[r], u);
         }
-        if (rank == 0 && warp == CP_WARPS - 1 && a.dinv && lane < w) {
-            // row j of the inverse of the unit lower diagonal block, whose row
-            // j is prow[0:j]:  Y[j][c] = delta_jc - sum_{t<j} prow[t] Y[t][c]
-            Cx<T> s0{T(lane == j), T(0)}, s1{T(0), T(0)}, s2{T(0), T(0)}, s3{T(0), T(0)};
-            int t = 0;
-            for (; t + 4 <= j; t += 4) {
-                s0 = cms(s0, prow[t], ublk[t * (w + 1) + lane]);
-                s1 = cms(s1, prow[t + 1], ublk[(t + 1) * (w + 1) + lane]);
-                s2 = cms(s2, prow[t + 2], ublk[(t + 2) * (w + 1) + lane]);
-                s3 = cms(s3, prow[t + 3], ublk[(t + 3) * (w + 1) + lane]);
+        if (EXTRA)
+            for (int i = tid; i < nx; i += NT) {
+                if (xpos[i] <= jr) continue;
+                Cx<T> *row = row_at(x0 + i);
+                const Cx<T> l1 = row[j];
+#pragma unroll 4
+                for (int q = (j >> 1) + 1; q < NPM; ++q) {
+                    const ColPair<T> u = pair_ld(prow + q * PB, T(0));
+                    row[2 * q] = cms(row[2 * q], l1, pair_get<0>(u));
+                    row[2 * q + 1] = cms(row[2 * q + 1], l1, pair_get<1>(u));
+                }
             }
-            for (; t < j; ++t) s0 = cms(s0, prow[t], ublk[t * (w + 1) + lane]);
-            ublk[j * (w + 1) + lane] = Cx<T>{(s0.re + s1.re) + (s2.re + s3.re), (s0.im + s1.im) + (s2.im + s3.im)};
+        // the pivot's index; L11's row j (complex entries in the pairs before
+        // j / 2, then the first half of pair j / 2)
+        if (rank == 0 && warp == NW - 1) {
+            if (lane == 0) {
+                if (!(mag_value(wm) > T(0))) atomicOr(a.status, (int)DEV_ZERO_PIVOT);
+                a.ipiv[jr] = p;
+            }
+            if (lane < W)
+                l11[j * (W + 1) + lane] = lane >= j                    ? Cx<T>{T(lane == j), T(0)}
+                                          : (lane >> 1) < (j >> 1) ? reinterpret_cast<const Cx<T> *>(lrow)[lane]
+                                                                       : pair_get<0>(pair_ld(up, T(0)));
         }
+        if (!more) {
+            stop = true;
+            return;
+        }
+        par = nslot;
+        phase ^= nslot == 0 ? 1u : 0u;
+    };
+    // candidate of column 0
+    {
+        Best best;
+        const Cx<T> z{T(0), T(0)};
+#pragma unroll
+        for (int r = 0; r < RPT; ++r)
+            if (mp[r] >= 0) best.offer(pair_get<0>(A[r][0]), z, mp[r], tid + r * NT);
+        if (EXTRA)
+            for (int i = tid; i < nx; i += NT) best.offer(row_at(x0 + i)[0], z, xpos[i], x0 + i);
+        if (C > 1) cl_sync();  // every CTA's mbarriers are initialised before any remote store
+        publish(std::integral_constant<int, 0>{}, std::integral_constant<int, NPM>{}, 0, 0, best, nullptr);
     }
+    auto run_phase = [&](auto npc, int j0) {
+#pragma unroll 1
+        for (int j = j0; j < j0 + W / 4 && !stop; j += 2) {
+            step(npc, std::integral_constant<int, 0>{}, j);
+            if (!stop) step(npc, std::integral_constant<int, 1>{}, j + 1);
+        }
+    };
+    run_phase(std::integral_constant<int, NPM>{}, 0);
+    run_phase(std::integral_constant<int, NPM * 3 / 4>{}, W / 4);
+    run_phase(std::integral_constant<int, NPM / 2>{}, W / 2);
+    run_phase(std::integral_constant<int, NPM / 4>{}, W * 3 / 4);
+
     // each row to its final position, by the bulk-copy engine
     fence_proxy_async_smem();
     __syncthreads();
+    auto each_row = [&](auto &&fn) {
 #pragma unroll
-    for (int r = 0; r < CP_RMAX; ++r) {
-        const int i = tid + r * CP_THREADS;
-        if (i < nrows && mp[r] >= a.k && mp[r] < a.n)
-            bulk_s2g(a.A + (int64_t)mp[r] * a.ld + a.k, sm_addr(P + (size_t)i * RS), row_bytes);
-    }
+        for (int r = 0; r < RPT; ++r)
+            if (mp[r] >= a.k && mp[r] < a.n) fn(tid + r * NT, mp[r]);
+        if (EXTRA)
+            for (int i = tid; i < nx; i += NT)
+                if (xpos[i] >= a.k && xpos[i] < a.n) fn(x0 + i, xpos[i]);
+    };
+    each_row([&](int i, int pos) { bulk_s2g(a.A + (int64_t)pos * a.ld + a.k, sm_addr(row_at(i)), 256u); });
     // the same interchanges on the panel's other columns: every CTA reads its
     // moved rows there before the cluster barrier and writes them at their
     // final positions after it (a permutation: every destination is some moved
     // row's origin, read before the barrier)
-    __shared__ int mv_src[CP_MAXMOVED], mv_dst[CP_MAXMOVED], mv_n;
-    constexpr int MV = CpMove<T>::V;
-    Cx<T> mvv[MV];
-    const int nleft = a.k - a.xc0, nother = (a.xc1 > a.xc0) ? nleft + (a.xc1 - a.k - w) : 0;
-    int nitems = 0;
+    __shared__ int mv_src[2 * W], mv_dst[2 * W], mv_n;
+    constexpr int MVC = S::MVC, MVT = S::MVT, E = 16 / sizeof(Cx<T>);
+    const int nleft = (a.k - a.xc0) / E, nother = a.xc1 > a.xc0 ? nleft + max(0, a.xc1 - a.k - W) / E : 0;
+    const int mc = tid % MVC, mr0 = tid / MVC, mrs = NT / MVC;
+    const int mcol = mc < nleft ? a.xc0 + mc * E : a.k + W + (mc - nleft) * E;
+    uint4 mvv[MVT];
+    int nmoved = 0;
     if (nother > 0) {
         if (tid == 0) mv_n = 0;
         __syncthreads();
-#pragma unroll
-        for (int r = 0; r < CP_RMAX; ++r) {
-            const int i = tid + r * CP_THREADS;
-            if (i < nrows && mp[r] >= a.k && mp[r] < a.n && mp[r] != gr0 + i) {
+        each_row([&](int i, int pos) {
+            if (pos != gr0 + i) {
                 const int slot = atomicAdd(&mv_n, 1);
-                if (slot < CP_MAXMOVED) {
+                if (slot < 2 * W) {
                     mv_src[slot] = gr0 + i;
-                    mv_dst[slot] = mp[r];
+                    mv_dst[slot] = pos;
                 }
+            }
+        });
+        __syncthreads();
+        nmoved = mc < nother ? min(mv_n, 2 * W) : 0;
+#pragma unroll
+        for (int u = 0; u < MVT; ++u)
+            if (mr0 + u * mrs < nmoved)
+                mvv[u] = *reinterpret_cast<const uint4 *>(a.A + (int64_t)mv_src[mr0 + u * mrs] * a.ld + mcol);
+    }
+    if (rank == 0 && a.dinv) {
+        // The inverse of L11 (identity past jmax): the 8 x 8 diagonal blocks'
+        // by substitution, a column per lane, then doubling: with the b x b
+        // diagonal blocks inverted, Y21 = -Y22 (L21 Y11) for each pair of
+        // them, L21 Y11 kept above l11's diagonal.
+        for (int e = tid; e < W * W; e += NT) {
+            const int i = e / W, c = e % W;
+            if (i / 8 != c / 8) y11[i * (W + 1) + c] = Cx<T>{T(0), T(0)};
+            if (i >= jmax) l11[i * (W + 1) + c] = Cx<T>{T(i == c), T(0)};
+        }
+        __syncthreads();
+        if (tid < W) {
+            const int d = tid & ~7;
+            const Cx<T> *L = l11 + d * (W + 1) + d;
+            Cx<T> v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                v[i] = Cx<T>{T(i == (tid & 7)), T(0)};
+#pragma unroll
+                for (int t = 0; t < i; ++t) v[i] = cms(v[i], L[i * (W + 1) + t], v[t]);
+                y11[(d + i) * (W + 1) + tid] = v[i];
             }
         }
         __syncthreads();
-        nitems = min(mv_n, CP_MAXMOVED) * nother;
-        if (mv_n > CP_MAXMOVED || nitems > MV * CP_THREADS) {  // the host sizes the panel so that this cannot happen
-            if (tid == 0) atomicOr(a.status, (int)DEV_BARRIER_TIMEOUT);
-            nitems = 0;
-        }
-#pragma unroll
-        for (int u = 0; u < MV; ++u) {
-            const int it = tid + u * CP_THREADS;
-            if (it < nitems) {
-                const int row = it / nother, cc = it % nother;
-                const int col = cc < nleft ? a.xc0 + cc : a.k + w + (cc - nleft);
-                mvv[u] = a.A[(int64_t)mv_src[row] * a.ld + col];
+#pragma unroll 1
+        for (int b = 8, lb = 3; b < W; b *= 2, ++lb)
+#pragma unroll 1
+            for (int pass = 0; pass < 2; ++pass) {
+                for (int e = tid; e < W / 2 * b; e += NT) {
+                    const int d = (e >> (2 * lb)) * 2 * b, i = (e >> lb) & (b - 1), c = e & (b - 1);
+                    const Cx<T> *left = (pass ? y11 + (d + b + i) * (W + 1) + d + b : l11 + (d + b + i) * (W + 1) + d);
+                    const Cx<T> *right = (pass ? l11 + b : y11) + d * (W + 1) + d + c;
+                    Cx<T> s0{T(0), T(0)}, s1{T(0), T(0)};
+#pragma unroll 4
+                    for (int t = 0; t < b; t += 2) {
+                        s0 = cms(s0, left[t], right[t * (W + 1)]);
+                        s1 = cms(s1, left[t + 1], right[(t + 1) * (W + 1)]);
+                    }
+                    const Cx<T> v{s0.re + s1.re, s0.im + s1.im};  // -(left right)
+                    if (pass == 0)
+                        l11[(d + i) * (W + 1) + d + b + c] = Cx<T>{-v.re, -v.im};
+                    else
+                        y11[(d + b + i) * (W + 1) + d + c] = v;
+                }
+                __syncthreads();
             }
+        for (int e = tid; e < W * W; e += NT) {
+            const int i = e / W, c = e % W;
+            a.dinv[e] = y11[i * (W + 1) + c];
         }
     }
     bulk_commit_wait_all();
-    if (rank == 0 && warp == 0 && a.dinv && lane < w)  // the inverse, identity past jmax
-        for (int i = 0; i < w; ++i)
-            a.dinv[(size_t)i * w + lane] = i < jmax ? ublk[i * (w + 1) + lane] : Cx<T>{T(i == lane), T(0)};
     cl_sync();  // every CTA's reads are done; no CTA leaves while a peer may still store into its shared memory
 #pragma unroll
-    for (int u = 0; u < MV; ++u) {
-        const int it = tid + u * CP_THREADS;
-        if (it < nitems) {
-            const int row = it / nother, cc = it % nother;
-            const int col = cc < nleft ? a.xc0 + cc : a.k + w + (cc - nleft);
-            a.A[(int64_t)mv_dst[row] * a.ld + col] = mvv[u];
-        }
-    }
+    for (int u = 0; u < MVT; ++u)
+        if (mr0 + u * mrs < nmoved)
+            *reinterpret_cast<uint4 *>(a.A + (int64_t)mv_dst[mr0 + u * mrs] * a.ld + mcol) = mvv[u];
 }
 
-// shared memory of the cluster kernel for rpc rows of width w
-template <typename T> static size_t cluster_panel_smem(int rpc, int w) {
-    return (size_t)rpc * CP_ROW_BYTES + sizeof(Cx<T>) * ((CP_SLOTS * CP_CTAS + 2 * CP_WARPS) * (size_t)w + w * (w + 1)) +
-           sizeof(PivKey) * CP_SLOTS * CP_CTAS;
-}
-
-// Launches the cluster kernel for a sub-panel; false when the rows do not fit
-// the cluster's shared memory or no cluster of CP_CTAS can be scheduled.
+// Launches the cluster kernel for a sub-panel of W columns; false when the rows
+// do not fit the cluster's shared memory or the cluster cannot be scheduled.
 template <typename T>
 static bool cluster_panel(beat_b200_ctx *c, Cx<T> *A, int64_t ld, int n, int k, int w, int *ipiv, Cx<T> *dinv,
                           int xc0 = 0, int xc1 = 0) {
+    using S = CpShape<T>;
     const int m = n - k;
-    const int rpc = (m + CP_CTAS - 1) / CP_CTAS;
+    const int C = m <= CP_ONE_CTA ? 1 : CP_CTAS;
+    const int rpc = (m + C - 1) / C;
+    // one row per thread on four warps (one per scheduler), then two, then two
+    // on eight warps, then the remaining rows in shared memory
+    const int threads = rpc <= CP_THREADS ? CP_THREADS / 2 : CP_THREADS;
+    const int rpt = rpc <= threads ? 1 : 2;
+    const int extra = std::max(0, rpc - rpt * threads);
     constexpr size_t cap = 220 * 1024;
-    if (w * sizeof(Cx<T>) > 256 || (w * sizeof(Cx<T>)) % 16 != 0 || rpc > CP_RMAX * CP_THREADS || n >= (1 << 30))
-        return false;
-    const size_t smem = cluster_panel_smem<T>(rpc, w);
+    if (w != S::W || n >= (1 << 30)) return false;
+    const size_t smem = S::smem(rpc, C, extra);
     if (smem > cap) return false;
-    static std::atomic<bool> attr_done[2] = {false, false};  // sweep lanes call this from several threads
-    const int ti = sizeof(T) == 8;
-    if (!attr_done[ti]) {
-        BB_CUDA(cudaFuncSetAttribute(cluster_panel_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        BB_CUDA(cudaFuncSetAttribute(cluster_panel_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
-        attr_done[ti] = true;
+    using Kernel = void (*)(ClusterPanelArgs<T>);
+    const Kernel kernels[3] = {cluster_panel_kernel<T, 1, false>, cluster_panel_kernel<T, 2, false>,
+                               cluster_panel_kernel<T, 2, true>};
+    static std::atomic<bool> attr_done{false};  // sweep lanes call this from several threads
+    if (!attr_done) {
+        for (Kernel f : kernels) {
+            BB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            BB_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+        }
+        attr_done = true;
     }
     ClusterPanelArgs<T> a;
     a.A = A;
     a.ld = ld;
     a.n = n;
     a.k = k;
-    a.w = w;
     a.rpc = rpc;
     a.ipiv = ipiv;
     a.status = c->status.as<int>();
@@ -1485,7 +1686,7 @@ static bool cluster_panel(beat_b200_ctx *c, Cx<T> *A, int64_t ld, int n, int k, 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(CP_CTAS);
     cfg.blockDim = dim3(CP_THREADS);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = cap;  // the largest request any sub-panel makes
     cfg.stream = c->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1496,15 +1697,17 @@ static bool cluster_panel(beat_b200_ctx *c, Cx<T> *A, int64_t ld, int n, int k, 
     cfg.numAttrs = 1;
     if (!c->cluster_checked) {
         int nclusters = 0;
-        cfg.dynamicSmemBytes = cap;  // the largest request any sub-panel makes
-        cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, (void *)cluster_panel_kernel<T>, &cfg);
-        cfg.dynamicSmemBytes = smem;
+        cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, kernels[2], &cfg);
         c->cluster_ok = (e == cudaSuccess && nclusters >= 1);
         cudaGetLastError();
         c->cluster_checked = true;
     }
     if (!c->cluster_ok) return false;
-    BB_CUDA(cudaLaunchKernelEx(&cfg, cluster_panel_kernel<T>, a));
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    attr[0].val.clusterDim.x = C;
+    BB_CUDA(cudaLaunchKernelEx(&cfg, kernels[extra > 0 ? 2 : rpt - 1], a));
     return true;
 }
 
@@ -1643,10 +1846,10 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
         for (int ks = k; ks < pe; ks += W) {
             const int m = n - ks;
             Cx<T> *dinv_s = blocked ? dinv + (size_t)(ks / W) * W * W : nullptr;
-            // the cluster kernel also swaps the panel's other columns when they fit its
-            // registers: moved rows (<= 2 W) x other columns (< nb) per CTA_THREADS x CpMove::V
-            const bool own_swaps = pe - k > W && 2 * W * (pe - k - W) <= CpMove<T>::V * CP_THREADS &&
-                                   2 * W <= CP_MAXMOVED;
+            // the cluster kernel also swaps the panel's other columns when they fit its registers
+            constexpr int CHUNK = 16 / sizeof(Cx<T>);
+            const int right = std::max(0, pe - ks - W), others = ks - k + right;
+            const bool own_swaps = others > 0 && others <= CpShape<T>::MVC * CHUNK && right % CHUNK == 0;
             const bool on_cluster =
                 cluster_panel<T>(c, A, ld, n, ks, W, ipiv, dinv_s, own_swaps ? k : 0, own_swaps ? pe : 0);
             if (!on_cluster) {
@@ -1674,7 +1877,7 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
                                                     s0));
             }
             // this sub-panel's interchanges on the rest of the panel (unless the cluster kernel did them)
-            if (pe - k > W && !(on_cluster && own_swaps)) {
+            if (others > 0 && !(on_cluster && own_swaps)) {
                 if (W <= LS_MAX)
                     laswp_panel_kernel<T><<<(pe - k + LC - 1) / LC, 256, laswp_panel_smem<T>(W), s0>>>(
                         A, ld, n, ks, W, ipiv, k, pe, ks, ks + W, nullptr);
