@@ -144,6 +144,7 @@ struct Workspace {
     DevBuf q;             // F x R FP64 Neumann data (column-major)
     DevBuf small_solve;   // block-substitution claim counter and per-block flags
     DevBuf dinv;          // FP64 inverses of the 64 x 64 diagonal blocks of L and U
+    DevBuf dinv_adj;      // the same for the solves with U^H and L^H (adjoint only)
     DevBuf field;         // field sources and evaluation points (grow-only)
     DevBuf io;            // device staging of the host-buffer entry points (grow-only)
     DevBuf qeff;          // Neumann data with the admittance term, for the field (grow-only)
@@ -278,6 +279,8 @@ void lu_factor(beat_b200_ctx *c, int precision, int nb, int split_terms);
 void lu_graph_release(beat_b200_ctx *c);  // drops the captured factorisation (buffers about to change)
 void lu_solve_fp64(beat_b200_ctx *c, int R, double *x_dev);          // in place, N x R col-major
 void lu_precond_fp32(beat_b200_ctx *c, int R, const double *in, double *out);
+void lu_adjoint_prepare(beat_b200_ctx *c);  // the adjoint solves' blocks, after a factorisation
+void lu_solve_adjoint(beat_b200_ctx *c, int R, const double *in, double *out);  // out = A^-H in (stored factors)
 
 // gmres.cu: Y += alpha * M X (M complex row-major rows x K, X/Y FP64 column-major)
 template <typename T>
@@ -295,7 +298,6 @@ IrResult gmres_refine(beat_b200_ctx *c, int R, double *x_dev, const double *b_de
 void apply_admittance_lhs(beat_b200_ctx *c, int precision);  // A += B diag(a) P
 // q_eff = q - a (P p) (F x R, FP64 column-major); a copy of q when no admittance is set
 void effective_neumann(beat_b200_ctx *c, int R, const double *p_dev, const double *q_dev, double *q_eff);
-void lu_solve_adjoint(beat_b200_ctx *c, int R, const double *in, double *out);  // out = A^-H in (stored factors)
 void adjoint(beat_b200_ctx *c, double k, int M, const double *dirs_host, int R, const double *p_dev,
              const double *g_dev, double *w_dev, double *ga_dev, const beat_b200_opts &o, IrResult *ir,
              const double **z_out = nullptr);
