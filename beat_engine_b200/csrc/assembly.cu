@@ -27,12 +27,6 @@
 
 namespace bb {
 
-constexpr int TT = 64, VT = 80;  // test tile: faces, distinct vertices (context.cu)
-constexpr int TS = 16, VS = 32;  // trial tile
-constexpr int REG_S = 3 * TS;    // slot-face indices of a trial tile
-constexpr int REG_INC = VS + 1 + REG_S;  // Tiling::inc_stride() of the trial tiles
-constexpr int REG_THREADS = 256;
-
 // rule tables: index 0 -> 1-point, 1 -> 3-point, 2 -> 6-point (order 4)
 __constant__ double c_rw64[3][6];
 __constant__ double c_rb64[3][6][3];
@@ -78,18 +72,7 @@ void upload_rule_tables(const std::vector<double> &pts, const std::vector<double
     BB_CUDA(cudaMemcpyToSymbol(c_rb32x2, b32x2, sizeof(b32x2)));
 }
 
-__device__ __forceinline__ void sincos_t(double x, double *s, double *c) { sincos_cw(x, s, c); }
-// FP32 phase: reduced to [-pi, pi] by a two-part 2 pi (6.2831854820251465 is
-// 2 pi rounded to float, -1.7484555e-7 the remainder), then the hardware
-// approximation, whose absolute error on [-pi, pi] (about 2^-21.4) is below
-// the rounding error of the FP32 phase k r itself.
-__device__ __forceinline__ void sincos_t(float x, float *s, float *c) {
-    const float n = rintf(x * 0.15915493667125702f);
-    float r = fmaf(-n, 6.2831854820251465f, x);
-    r = fmaf(-n, -1.7484555314695172e-07f, r);
-    __sincosf(r, s, c);
-}
-// The same phase given in revolutions, t = x / (2 pi): t - rint(t) is exact,
+// FP32 phase given in revolutions, t = x / (2 pi): t - rint(t) is exact,
 // so the reduction to [-1/2, 1/2] is one rounding and one subtraction.  The
 // multiply back to radians adds at most about 2^-22 absolute on [-pi, pi],
 // below the hardware approximation's own error there (about 2^-21.4); for
@@ -97,7 +80,15 @@ __device__ __forceinline__ void sincos_t(float x, float *s, float *c) {
 __device__ __forceinline__ void sincos_rev(float t, float *s, float *c) {
     __sincosf((t - rintf(t)) * 6.2831854820251465f, s, c);
 }
-__device__ __forceinline__ double rsqrt_t(double x) { return rsqrt(x); }
+// 1 / sqrt(x), x a positive normal number: the hardware approximation y (error
+// about 2^-22), then one step of the series (1 - e)^(-1/2) = 1 + e/2 + 3/8 e^2 +
+// ... with e = 1 - x y^2, whose next term 5/16 e^3 is below 2^-60
+__device__ __forceinline__ double rsqrt_t(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
 __device__ __forceinline__ float rsqrt_t(float x) { return rsqrtf(x); }
 
 __device__ __forceinline__ void red_add(double *p, double v) { atomicAdd(p, v); }
@@ -238,12 +229,11 @@ template <typename T> struct RegArgs {
     const T *normal;    // F x 3
     const T *curl;      // F x 9
     const T *area;      // F
-    const T *plane = nullptr;  // F: plane offset . normal (FP32 symmetric kernel)
+    const T *plane = nullptr;  // F: plane offset . normal (FP32; the FP64 kernel forms its own)
     const int *gvert;   // F x 3
     const int *face_id; // F
     const int *t_fstart, *t_vstart, *t_verts, *t_local;
-    const int *s_fstart, *s_vstart, *s_verts;
-    const int *t_inc = nullptr, *s_inc = nullptr;  // per-tile vertex incidences (Tiling::incidence)
+    const int *t_inc = nullptr;  // per-tile vertex incidences (Tiling::incidence)
     Cx<T> *A;
     Cx<T> *B;
     int64_t ld;         // row stride of A (complex entries)
@@ -260,277 +250,89 @@ template <typename T> struct RegArgs {
     int N = 0, R = 0;
 };
 
-// Element-pair kernel.  grid = (trial tiles, test tiles), 256 threads.
-template <typename T, int Q>
-__global__ void __launch_bounds__(REG_THREADS, sizeof(T) == 4 ? 3 : 2) regular_pairs_kernel(RegArgs<T> g) {
-    constexpr int RI = Q == 1 ? 0 : Q == 3 ? 1 : 2;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    // test vertex x trial vertex *slot* (s = b * TS + trial face): lanes that
-    // share a test vertex never add to one word together (see the symmetric
-    // kernel below); folded onto the trial tile's vertices at the flush
-    Cx<T> *sC = reinterpret_cast<Cx<T> *>(smem_raw);  // VT x REG_S
-    Cx<T> *sB = sC + VT * REG_S;                      // VT x TS
-    T *tq = reinterpret_cast<T *>(sB + VT * TS);      // TT x Q x 3
-    T *tn = tq + TT * Q * 3;                          // TT x 3
-    T *tc = tn + TT * 3;                              // TT x 9
-    T *ta = tc + TT * 9;                              // TT
-    T *sq = ta + TT;                                  // (Q*3) x TS (trial, transposed)
-    T *sn = sq + TS * Q * 3;                          // 3 x TS
-    T *sc = sn + TS * 3;                              // 9 x TS
-    T *sa = sc + TS * 9;                              // TS
-    T *tpl = sa + TS;                                 // TT: plane offset x . n of each test face
-    T *spl = tpl + TT;                                // TS: plane offset y . n of each trial face
-    int *tgv = reinterpret_cast<int *>(spl + TS);     // TT x 3
-    int *tlv = tgv + TT * 3;                          // TT x 3
-    int *sgv = tlv + TT * 3;                          // 3 x TS
-    int *inc_start = sgv + TS * 3;                    // VS + 1: trial vertex -> its slot-face indices
-    int *inc_list = inc_start + VS + 1;               // REG_S
-
-    const int tid = threadIdx.x;
-    const int t0 = g.t_fstart[blockIdx.y], nt = g.t_fstart[blockIdx.y + 1] - t0;
-    const int s0 = g.s_fstart[blockIdx.x], ns = g.s_fstart[blockIdx.x + 1] - s0;
-    const int tv0 = g.t_vstart[blockIdx.y], nvt = g.t_vstart[blockIdx.y + 1] - tv0;
-    const int sv0 = g.s_vstart[blockIdx.x], nvs = g.s_vstart[blockIdx.x + 1] - sv0;
-
-    for (int i = tid; i < VT * REG_S; i += REG_THREADS) sC[i] = Cx<T>{T(0), T(0)};
-    for (int i = tid; i < VT * TS; i += REG_THREADS) sB[i] = Cx<T>{T(0), T(0)};
-    // the tile arrays: every copy in flight at once, one wait
-    for (int i = tid; i < nt * Q * 3; i += REG_THREADS) cp_async_el(&tq[i], &g.qpts[(size_t)t0 * Q * 3 + i]);
-    for (int i = tid; i < nt * 3; i += REG_THREADS) {
-        cp_async_el(&tn[i], &g.normal[(size_t)t0 * 3 + i]);
-        cp_async_el(&tgv[i], &g.gvert[(size_t)t0 * 3 + i]);
-        cp_async_el(&tlv[i], &g.t_local[(size_t)t0 * 3 + i]);
-    }
-    for (int i = tid; i < nt * 9; i += REG_THREADS) cp_async_el(&tc[i], &g.curl[(size_t)t0 * 9 + i]);
-    for (int i = tid; i < nt; i += REG_THREADS) cp_async_el(&ta[i], &g.area[t0 + i]);
-    for (int i = tid; i < ns * Q * 3; i += REG_THREADS) {
-        int s = i / (Q * 3), j = i % (Q * 3);
-        cp_async_el(&sq[j * TS + s], &g.qpts[(size_t)s0 * Q * 3 + i]);
-    }
-    for (int i = tid; i < ns * 3; i += REG_THREADS) {
-        int s = i / 3, j = i % 3;
-        cp_async_el(&sn[j * TS + s], &g.normal[(size_t)s0 * 3 + i]);
-        cp_async_el(&sgv[j * TS + s], &g.gvert[(size_t)s0 * 3 + i]);
-    }
-    for (int i = tid; i < ns * 9; i += REG_THREADS) {
-        int s = i / 9, j = i % 9;
-        cp_async_el(&sc[j * TS + s], &g.curl[(size_t)s0 * 9 + i]);
-    }
-    for (int i = tid; i < ns; i += REG_THREADS) cp_async_el(&sa[i], &g.area[s0 + i]);
-    for (int i = tid; i < REG_INC; i += REG_THREADS)
-        cp_async_el(&inc_start[i], &g.s_inc[(size_t)blockIdx.x * REG_INC + i]);
-    cp_async_wait_all();
-    __syncthreads();
-    // every point y of a flat face has the same y . n
-    for (int i = tid; i < nt; i += REG_THREADS)
-        tpl[i] = tq[i * Q * 3] * tn[3 * i] + tq[i * Q * 3 + 1] * tn[3 * i + 1] + tq[i * Q * 3 + 2] * tn[3 * i + 2];
-    if (tid < ns) {  // one thread per trial face: its image reflection, then its plane offset
-        if (g.image) {
-            // an image pass reflects the trial tile (signs xs, curls also by det)
-            for (int j = 0; j < Q * 3; ++j) sq[j * TS + tid] *= g.xs[j % 3];
-            for (int j = 0; j < 3; ++j) sn[j * TS + tid] *= g.xs[j];
-            for (int j = 0; j < 9; ++j) sc[j * TS + tid] *= g.xdet * g.xs[j % 3];
-        }
-        spl[tid] = sq[tid] * sn[tid] + sq[TS + tid] * sn[TS + tid] + sq[2 * TS + tid] * sn[2 * TS + tid];
-    }
-    __syncthreads();
-
-    const T k = g.k, eta = g.eta;
-    const T inv4pi = T(0.07957747154594767);  // 1 / (4 pi)
-    const int npairs = nt * TS;
-    for (int p = tid; p < npairs; p += REG_THREADS) {
-        const int tl = p / TS, sl = p % TS;
-        if (sl >= ns) continue;
-        const int ga = tgv[3 * tl], gb = tgv[3 * tl + 1], gc = tgv[3 * tl + 2];
-        const int ha = sgv[sl], hb = sgv[TS + sl], hc = sgv[2 * TS + sl];
-        if (!g.image && (ga == ha || ga == hb || ga == hc || gb == ha || gb == hb || gb == hc || gc == ha ||
-                         gc == hb || gc == hc))
-            continue;  // touching pair: the Duffy kernel integrates it
-        const T ntx = tn[3 * tl], nty = tn[3 * tl + 1], ntz = tn[3 * tl + 2];
-        const T nsx = sn[sl], nsy = sn[TS + sl], nsz = sn[2 * TS + sl];
-        const T k2n = eta * g.k2 * (ntx * nsx + nty * nsy + ntz * nsz);
-        // with r = y - x:  r . n_s = ds - x . n_s  and  -r . n_t = dt - y . n_t
-        const T ds = spl[sl], dt = tpl[tl];
-        T L[9][2], Rv[3][2], cr = T(0), ci = T(0);
-#pragma unroll
-        for (int i = 0; i < 9; ++i) L[i][0] = L[i][1] = T(0);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) Rv[i][0] = Rv[i][1] = T(0);
-#pragma unroll 1
-        for (int qt = 0; qt < Q; ++qt) {
-            const T x0 = tq[(tl * Q + qt) * 3], x1 = tq[(tl * Q + qt) * 3 + 1], x2 = tq[(tl * Q + qt) * 3 + 2];
-            const T wt = RuleRef<T>::w(RI, qt) * inv4pi;
-            const T xns = ds - (x0 * nsx + x1 * nsy + x2 * nsz);
-            T S0r = 0, S0i = 0, S1r = 0, S1i = 0, S2r = 0, S2i = 0, Gr = 0, Gi = 0, Wr = 0, Wi = 0;
-#pragma unroll
-            for (int qs = 0; qs < Q; ++qs) {
-                const T y0 = sq[(qs * 3) * TS + sl], y1 = sq[(qs * 3 + 1) * TS + sl], y2 = sq[(qs * 3 + 2) * TS + sl];
-                const T rx = y0 - x0, ry = y1 - x1, rz = y2 - x2;
-                const T r2 = rx * rx + ry * ry + rz * rz;
-                const T ir = rsqrt_t(r2);
-                T sn_, cs_;
-                sincos_t(k * (r2 * ir), &sn_, &cs_);
-                const T scl = ir * (wt * RuleRef<T>::w(RI, qs));
-                const T gr = cs_ * scl, gi = sn_ * scl;           // weighted green
-                const T gsr = -gr * ir - gi * k;                  // weighted d green / d r
-                const T gsi = gr * k - gi * ir;
-                const T dns = xns * ir, dnt = (dt - (y0 * ntx + y1 * nty + y2 * ntz)) * ir;
-                const T lr = k2n * gi - gsr * dns;                // -grad*dn_s - i k2n g
-                const T li = -(gsi * dns + k2n * gr);
-                Gr += gr;
-                Gi += gi;
-                Wr += dnt * gsr;
-                Wi += dnt * gsi;
-                const T b0 = RuleRef<T>::b(RI, qs, 0), b1 = RuleRef<T>::b(RI, qs, 1), b2 = RuleRef<T>::b(RI, qs, 2);
-                S0r += b0 * lr;
-                S0i += b0 * li;
-                S1r += b1 * lr;
-                S1i += b1 * li;
-                S2r += b2 * lr;
-                S2i += b2 * li;
-            }
-            // sum over the trial points of -g - i eta grad*dn_t
-            const T Ur = -Gr + eta * Wi, Ui = -Gi - eta * Wr;
-            cr += Gr;
-            ci += Gi;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const T ba = RuleRef<T>::b(RI, qt, a);
-                L[3 * a + 0][0] += ba * S0r;
-                L[3 * a + 0][1] += ba * S0i;
-                L[3 * a + 1][0] += ba * S1r;
-                L[3 * a + 1][1] += ba * S1i;
-                L[3 * a + 2][0] += ba * S2r;
-                L[3 * a + 2][1] += ba * S2i;
-                Rv[a][0] += ba * Ur;
-                Rv[a][1] += ba * Ui;
-            }
-        }
-        // hypersingular curl term: eta * sum(g w) * curl_t . curl_s
-        const T ccr = -eta * ci, cci = eta * cr;
-        const T jac = T(4) * ta[tl] * sa[sl];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const int row = tlv[3 * tl + a];
-            int off[8];  // this vertex's 8 adds, in T words from sC
-            T val[8];
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                const T d = tc[9 * tl + 3 * a] * sc[(3 * b) * TS + sl] +
-                            tc[9 * tl + 3 * a + 1] * sc[(3 * b + 1) * TS + sl] +
-                            tc[9 * tl + 3 * a + 2] * sc[(3 * b + 2) * TS + sl];
-                const int o = 2 * (row * REG_S + b * TS + sl);
-                off[2 * b] = o;
-                val[2 * b] = (L[3 * a + b][0] + d * ccr) * jac;
-                off[2 * b + 1] = o + 1;
-                val[2 * b + 1] = (L[3 * a + b][1] + d * cci) * jac;
-            }
-            off[6] = 2 * (VT * REG_S + row * TS + sl);
-            val[6] = Rv[a][0] * jac;
-            off[7] = off[6] + 1;
-            val[7] = Rv[a][1] * jac;
-            batch_add<8>(reinterpret_cast<T *>(sC), off, val);
-        }
-    }
-    __syncthreads();
-    for (int i = tid; i < nvt * nvs; i += REG_THREADS) {
-        const int lt = i / nvs, ls = i % nvs;
-        Cx<T> v{T(0), T(0)};
-        for (int e = inc_start[ls]; e < inc_start[ls + 1]; ++e) {
-            const Cx<T> c = sC[lt * REG_S + inc_list[e]];
-            v.re += c.re;
-            v.im += c.im;
-        }
-        if (v.re != T(0) || v.im != T(0))
-            red_add_cx(&g.A[(int64_t)g.t_verts[tv0 + lt] * g.ld + g.s_verts[sv0 + ls]], v.re, v.im);
-    }
-    if (g.B) {
-        for (int i = tid; i < nvt * ns; i += REG_THREADS) {
-            const int lt = i / ns, sl = i % ns;
-            const Cx<T> v = sB[lt * TS + sl];
-            if (v.re != T(0) || v.im != T(0))
-                red_add_cx(&g.B[(int64_t)g.t_verts[tv0 + lt] * g.F + g.face_id[s0 + sl]], v.re, v.im);
-        }
-        return;
-    }
-    // matrix-free: the tile's rows of b += sB (test vertices x trial faces) q,
-    // q staged MF_RC columns at a time over the (now unused) geometry region
-    Cx<T> *qs = reinterpret_cast<Cx<T> *>(tq);  // [TS][MF_RC]
-    for (int r0 = 0; r0 < g.R; r0 += MF_RC) {
-        const int rc = min(MF_RC, g.R - r0);
-        __syncthreads();
-        for (int i = tid; i < TS * MF_RC; i += REG_THREADS) {
-            const int f = i / MF_RC, r = i % MF_RC;
-            Cx<T> v{T(0), T(0)};
-            if (f < ns && r < rc) {
-                const Cx<double> qq = g.q[(size_t)(r0 + r) * g.F + g.face_id[s0 + f]];
-                v = Cx<T>{(T)qq.re, (T)qq.im};
-            }
-            qs[i] = v;
-        }
-        __syncthreads();
-        for (int i = tid; i < nvt * rc; i += REG_THREADS) {
-            const int lt = i / rc, r = i % rc;
-            T sr = T(0), si = T(0);
-            for (int f = 0; f < ns; ++f) {
-                const Cx<T> bv = sB[lt * TS + f], qv = qs[f * MF_RC + r];
-                sr += bv.re * qv.re - bv.im * qv.im;
-                si += bv.re * qv.im + bv.im * qv.re;
-            }
-            if (sr != T(0) || si != T(0))
-                red_add_cx(&g.b[(size_t)(r0 + r) * g.N + g.t_verts[tv0 + lt]], (double)sr, (double)si);
-        }
-    }
-}
-
-template <typename T, int Q> static size_t regular_smem_bytes() {
-    return sizeof(Cx<T>) * (VT * REG_S + VT * TS) + sizeof(T) * (TT * (Q * 3 + 3 + 9 + 2) + TS * (Q * 3 + 3 + 9 + 2)) +
-           sizeof(int) * (TT * 6 + TS * 3 + REG_INC);
-}
-
 // ---------------------------------------------------------------------------
-// Symmetric element-pair kernel (FP32 form).  G(x, y) = G(y, x), so the two
-// ordered pairs (tau, sigma) and (sigma, tau) of two elements share r, the
-// phase, e^{ikr}/r and dG/dr at every point pair; only the normal
-// derivatives swap roles: with r = y - x,
+// Symmetric element-pair kernel.  G(x, y) = G(y, x), so the two ordered pairs
+// (tau, sigma) and (sigma, tau) of two elements share r, the phase, e^{ikr}/r
+// and dG/dr at every point pair; only the normal derivatives swap roles: with
+// r = y - x,
 //   order 1 (test tau at x, trial sigma at y): dn_s =  r.n_sigma / r = a,
 //                                               dn_t = -r.n_tau / r   = c,
 //   order 2 (test sigma at y, trial tau at x): dn_s = c, dn_t = a.
 // One CTA integrates an unordered pair of square tiles (I <= J; pairs of
 // elements tau < sigma inside a diagonal tile) for both orders; each order
-// has its own shared-memory accumulators, flushed like the one-order kernel.
+// has its own shared-memory accumulators, flushed once.
+//
+// Tiles: FP32 32 faces, two CTAs of 256 threads per SM (108 KB each).  FP64 16
+// faces and two CTAs of 128 threads: the accumulators are twice as wide and a
+// thread holds about 200 registers of sums, and one CTA of 32-face tiles (212
+// KB) would leave the FP64 units idle while it zeroes, loads and flushes.
+// Bound: issue (FP32), the FP64 units (FP64: about 85 FP64 instructions per
+// unordered point pair, 34 ms at F = 20,480; one ordered pair at a time took
+// 104.7 ms there, this 53.8).
 // ---------------------------------------------------------------------------
-constexpr int SYM_F = 32, SYM_V = 40;  // square tile: faces, distinct vertices (context.cu)
-// Accumulators.  A warp takes one tau and 32 sigma (one per lane), so the
-// entries a lane adds to are keyed by sigma's vertex *slot* (s = b * SYM_F +
-// sigma, the slot-face index) rather than by sigma's vertex: two lanes whose
-// faces share a vertex would otherwise add to the same word in the same
-// instruction, and shared-memory float atomics retry once per colliding lane.
-// The slot-face entries are folded onto tile J's vertices at the flush.
+// Accumulators.  A warp takes one tau and 32 sigma (FP64: two taus eight apart
+// and 16 sigma), so the entries a lane adds to are keyed by sigma's vertex
+// *slot* (s = b * F + sigma, the slot-face index) rather than by sigma's
+// vertex: two lanes whose faces share a vertex would otherwise add to the same
+// word in the same instruction, and shared-memory float atomics retry once per
+// colliding lane.  The slot-face entries are folded onto tile J's vertices at
+// the flush.
 //   C1 [vI][s]      order 1, test vertex of tau x trial slot of sigma
 //   C2 [s][vI]      order 2, test slot of sigma x trial vertex of tau
 //   B1 [vI][sigma]  order 1 right-hand side (test vertex of tau x face sigma)
 //   D2 [s][tau]     order 2 right-hand side (test slot of sigma x face tau)
 // Re / im planes; a warp's lanes step 1 or an odd stride through each, so
 // they spread over all banks.
-constexpr int SYM_S = 3 * SYM_F;                  // slot-face indices of a tile
-constexpr int SYM_C2S = SYM_V + 1, SYM_BS = SYM_F + 1;
-constexpr int SYM_C1 = 0;
-constexpr int SYM_C2 = SYM_C1 + SYM_V * SYM_S;
-constexpr int SYM_B1 = SYM_C2 + SYM_S * SYM_C2S;
-constexpr int SYM_D2 = SYM_B1 + SYM_V * SYM_BS;
-constexpr int SYM_ACC = SYM_D2 + SYM_S * SYM_BS;  // floats per plane
+template <typename T> struct SymTile {  // shapes as in context.cu
+    static constexpr int F = sizeof(T) == 4 ? 32 : 16;        // faces
+    static constexpr int V = sizeof(T) == 4 ? 40 : 32;        // distinct vertices
+    static constexpr int THREADS = sizeof(T) == 4 ? 256 : 128;
+    static constexpr int S = 3 * F;                            // slot-face indices
+    static constexpr int C2S = V + 1, BS = F + 1;
+    static constexpr int C1 = 0, C2 = C1 + V * S, B1 = C2 + S * C2S, D2 = B1 + V * BS;
+    static constexpr int ACC = D2 + S * BS;                    // entries per plane
+    static constexpr int INC = V + 1 + S;                      // Tiling::inc_stride()
+    template <int Q> static size_t smem() {
+        return sizeof(T) * (2 * ACC + 2 * F * (Q * 3 + 3 + 9 + 2)) + sizeof(int) * (3 * 3 * F + INC);
+    }
+};
 
-constexpr int SYM_INC = SYM_V + 1 + SYM_S;  // Tiling::inc_stride() of the square tiles
+// (re, im) sums: packed in FP32, two doubles in FP64
+template <typename T> struct CxSum;
+template <> struct CxSum<float> {
+    F2 v = 0;
+    __device__ __forceinline__ static F2 make(float re, float im) { return pk2(re, im); }
+    __device__ __forceinline__ static F2 scaled(float a, F2 x) { return mul2(pk2(a, a), x); }
+    __device__ __forceinline__ void add(int ri, int q, int b, F2 x) { v = fma2(rule_b2(ri, q, b), x, v); }
+    __device__ __forceinline__ void get(float &re, float &im) const { up2(v, re, im); }
+};
+template <> struct CxSum<double> {
+    Cx<double> v{0.0, 0.0};
+    __device__ __forceinline__ static Cx<double> make(double re, double im) { return Cx<double>{re, im}; }
+    __device__ __forceinline__ static Cx<double> scaled(double a, Cx<double> x) {
+        return Cx<double>{a * x.re, a * x.im};
+    }
+    __device__ __forceinline__ void add(int ri, int q, int b, Cx<double> x) {
+        v.re = fma(c_rb64[ri][q][b], x.re, v.re);
+        v.im = fma(c_rb64[ri][q][b], x.im, v.im);
+    }
+    __device__ __forceinline__ void get(double &re, double &im) const {
+        re = v.re;
+        im = v.im;
+    }
+};
+// sine and cosine of k r; kr = phase_scale(k) r is in revolutions (FP32) or radians (FP64)
+__device__ __forceinline__ float phase_scale(float k) { return k * 0.15915494309189535f; }
+__device__ __forceinline__ double phase_scale(double k) { return k; }
+__device__ __forceinline__ void sincos_kr(float kr, float *s, float *c) { sincos_rev(kr, s, c); }
+__device__ __forceinline__ void sincos_kr(double kr, double *s, double *c) { sincos_cw(kr, s, c); }
 
-template <int Q> static size_t sym_smem_bytes() {
-    return sizeof(float) * 2 * SYM_ACC + sizeof(float) * 2 * SYM_F * (Q * 3 + 3 + 9 + 2) +
-           sizeof(int) * (3 * 3 * SYM_F + SYM_INC);
-}
-
-template <int Q>
-__global__ void __launch_bounds__(REG_THREADS, 2) sym_pairs_kernel(RegArgs<float> g) {
-    using T = float;
+template <typename T, int Q>
+__global__ void __launch_bounds__(SymTile<T>::THREADS, 2) sym_pairs_kernel(RegArgs<T> g) {
+    using ST = SymTile<T>;
+    constexpr int SYM_F = ST::F, SYM_S = ST::S, SYM_C2S = ST::C2S, SYM_BS = ST::BS, SYM_ACC = ST::ACC,
+                  SYM_C1 = ST::C1, SYM_C2 = ST::C2, SYM_B1 = ST::B1, SYM_D2 = ST::D2, SYM_INC = ST::INC,
+                  SYM_V = ST::V, THREADS = ST::THREADS;
     constexpr int RI = Q == 1 ? 0 : Q == 3 ? 1 : 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *acc_re = reinterpret_cast<T *>(smem_raw), *acc_im = acc_re + SYM_ACC;
@@ -564,53 +366,63 @@ __global__ void __launch_bounds__(REG_THREADS, 2) sym_pairs_kernel(RegArgs<float
     const int tv0 = g.t_vstart[I], nvI = g.t_vstart[I + 1] - tv0;
     const int sv0 = g.t_vstart[J], nvJ = g.t_vstart[J + 1] - sv0;
 
-    static_assert((2 * SYM_ACC) % 4 == 0, "accumulators are zeroed as float4");
-    for (int i = tid; i < 2 * SYM_ACC / 4; i += REG_THREADS)
+    static_assert(2 * SYM_ACC * sizeof(T) % 16 == 0, "accumulators are zeroed as float4");
+    for (int i = tid; i < (int)(2 * SYM_ACC * sizeof(T) / 16); i += THREADS)
         reinterpret_cast<float4 *>(acc_re)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     // the tile arrays: every copy in flight at once, one wait
-    for (int i = tid; i < nI * Q * 3; i += REG_THREADS) cp_async4(&xq[i], &g.qpts[(size_t)t0 * Q * 3 + i]);
-    for (int i = tid; i < nI * 3; i += REG_THREADS) {
-        cp_async4(&xn[i], &g.normal[(size_t)t0 * 3 + i]);
-        cp_async4(&xgv[i], &g.gvert[(size_t)t0 * 3 + i]);
-        cp_async4(&xlv[i], &g.t_local[(size_t)t0 * 3 + i]);
+    for (int i = tid; i < nI * Q * 3; i += THREADS) cp_async_el(&xq[i], &g.qpts[(size_t)t0 * Q * 3 + i]);
+    for (int i = tid; i < nI * 3; i += THREADS) {
+        cp_async_el(&xn[i], &g.normal[(size_t)t0 * 3 + i]);
+        cp_async_el(&xgv[i], &g.gvert[(size_t)t0 * 3 + i]);
+        cp_async_el(&xlv[i], &g.t_local[(size_t)t0 * 3 + i]);
     }
-    for (int i = tid; i < nI * 9; i += REG_THREADS) cp_async4(&xc[i], &g.curl[(size_t)t0 * 9 + i]);
-    for (int i = tid; i < nI; i += REG_THREADS) {
-        cp_async4(&xa[i], &g.area[t0 + i]);
-        cp_async4(&xp[i], &g.plane[t0 + i]);
+    for (int i = tid; i < nI * 9; i += THREADS) cp_async_el(&xc[i], &g.curl[(size_t)t0 * 9 + i]);
+    for (int i = tid; i < nI; i += THREADS) {
+        cp_async_el(&xa[i], &g.area[t0 + i]);
+        if (sizeof(T) == 4) cp_async_el(&xp[i], &g.plane[t0 + i]);
     }
-    for (int i = tid; i < nJ * Q * 3; i += REG_THREADS) {
+    for (int i = tid; i < nJ * Q * 3; i += THREADS) {
         const int s = i / (Q * 3), j = i % (Q * 3);
-        cp_async4(&yq[j * SYM_F + s], &g.qpts[(size_t)s0 * Q * 3 + i]);
+        cp_async_el(&yq[j * SYM_F + s], &g.qpts[(size_t)s0 * Q * 3 + i]);
     }
-    for (int i = tid; i < nJ * 3; i += REG_THREADS) {
+    for (int i = tid; i < nJ * 3; i += THREADS) {
         const int s = i / 3, j = i % 3;
-        cp_async4(&yn[j * SYM_F + s], &g.normal[(size_t)s0 * 3 + i]);
-        cp_async4(&ygv[j * SYM_F + s], &g.gvert[(size_t)s0 * 3 + i]);
+        cp_async_el(&yn[j * SYM_F + s], &g.normal[(size_t)s0 * 3 + i]);
+        cp_async_el(&ygv[j * SYM_F + s], &g.gvert[(size_t)s0 * 3 + i]);
     }
-    for (int i = tid; i < nJ * 9; i += REG_THREADS) {
+    for (int i = tid; i < nJ * 9; i += THREADS) {
         const int s = i / 9, j = i % 9;
-        cp_async4(&yc[j * SYM_F + s], &g.curl[(size_t)s0 * 9 + i]);
+        cp_async_el(&yc[j * SYM_F + s], &g.curl[(size_t)s0 * 9 + i]);
     }
-    for (int i = tid; i < nJ; i += REG_THREADS) {
-        cp_async4(&ya[i], &g.area[s0 + i]);
-        cp_async4(&yp[i], &g.plane[s0 + i]);
+    for (int i = tid; i < nJ; i += THREADS) {
+        cp_async_el(&ya[i], &g.area[s0 + i]);
+        if (sizeof(T) == 4) cp_async_el(&yp[i], &g.plane[s0 + i]);
     }
-    for (int i = tid; i < SYM_INC; i += REG_THREADS) cp_async4(&inc_start[i], &g.t_inc[(size_t)J * SYM_INC + i]);
+    for (int i = tid; i < SYM_INC; i += THREADS) cp_async_el(&inc_start[i], &g.t_inc[(size_t)J * SYM_INC + i]);
     cp_async_wait_all();
     __syncthreads();
+    if (sizeof(T) == 8) {  // every point y of a flat face has the same y . n
+        for (int i = tid; i < nI + nJ; i += THREADS) {
+            if (i < nI)
+                xp[i] = xq[i * Q * 3] * xn[3 * i] + xq[i * Q * 3 + 1] * xn[3 * i + 1] + xq[i * Q * 3 + 2] * xn[3 * i + 2];
+            else
+                yp[i - nI] = yq[i - nI] * yn[i - nI] + yq[SYM_F + i - nI] * yn[SYM_F + i - nI] +
+                             yq[2 * SYM_F + i - nI] * yn[2 * SYM_F + i - nI];
+        }
+        __syncthreads();
+    }
     if (g.image) {
         // an image pass reflects tile J: pairs (tau, S sigma) and (sigma, S tau)
         // have the same distances, |x - Sy| = |Sx - y|, and swap dn_s / dn_t
-        for (int i = tid; i < nJ * Q * 3; i += REG_THREADS) {
+        for (int i = tid; i < nJ * Q * 3; i += THREADS) {
             const int s = i / (Q * 3), j = i % (Q * 3);
             yq[j * SYM_F + s] *= g.xs[j % 3];
         }
-        for (int i = tid; i < nJ * 3; i += REG_THREADS) {
+        for (int i = tid; i < nJ * 3; i += THREADS) {
             const int s = i / 3, j = i % 3;
             yn[j * SYM_F + s] *= g.xs[j];
         }
-        for (int i = tid; i < nJ * 9; i += REG_THREADS) {
+        for (int i = tid; i < nJ * 9; i += THREADS) {
             const int s = i / 9, j = i % 9;
             yc[j * SYM_F + s] *= g.xdet * g.xs[j % 3];
         }
@@ -618,10 +430,11 @@ __global__ void __launch_bounds__(REG_THREADS, 2) sym_pairs_kernel(RegArgs<float
     }
 
     const T k = g.k, eta = g.eta;
-    const T kr = k * T(0.15915494309189535);  // k / (2 pi): the phase k r in revolutions
+    const T kr = phase_scale(k);
     const T inv4pi = T(0.07957747154594767);  // 1 / (4 pi)
-    for (int p = tid; p < SYM_F * SYM_F; p += REG_THREADS) {
-        const int ti = p / SYM_F, sj = p % SYM_F;  // a warp: one tau, every sigma
+    for (int p = tid; p < SYM_F * SYM_F; p += THREADS) {
+        // a warp: one tau (two, half a tile apart), every sigma
+        const int ti = SYM_F == 32 ? p / 32 : p / 32 + (p >> 4 & 1) * 8, sj = p % SYM_F;
         // (an image pass keeps tau == sigma: the element and its own image,
         // whose two orders coincide and are taken at half weight)
         if (ti >= nI || sj >= nJ || (diag && (g.image ? sj < ti : sj <= ti))) continue;
@@ -660,7 +473,7 @@ __global__ void __launch_bounds__(REG_THREADS, 2) sym_pairs_kernel(RegArgs<float
             // Order 1's kernel value -g' (r . n_sigma) / r - i k2n g sums to
             // -xns H_b - i k2n C_b, order 2's (r . n_tau) g' / r - i k2n g to
             // P_b - i k2n C_b; each sum a packed (re, im) pair.
-            F2 C0 = 0, C1 = 0, C2 = 0, H0 = 0, H1 = 0, H2 = 0, P0 = 0, P1 = 0, P2 = 0;
+            CxSum<T> Cs[3], Hs[3], Ps[3];
 #pragma unroll
             for (int qs = 0; qs < Q; ++qs) {
                 const T rx = yq[(qs * 3) * SYM_F + sj] - x0, ry = yq[(qs * 3 + 1) * SYM_F + sj] - x1,
@@ -668,34 +481,27 @@ __global__ void __launch_bounds__(REG_THREADS, 2) sym_pairs_kernel(RegArgs<float
                 const T r2 = rx * rx + ry * ry + rz * rz;
                 const T ir = rsqrt_t(r2);
                 T sn_, cs_;
-                sincos_rev(kr * (r2 * ir), &sn_, &cs_);
+                sincos_kr(kr * (r2 * ir), &sn_, &cs_);
                 const T scl = ir * RuleRef<T>::w(RI, qs);
                 const T gr = cs_ * scl, gi = sn_ * scl;
                 const T hr = (-gr * ir - gi * k) * ir;
                 const T hi = (gr * k - gi * ir) * ir;
-                const F2 g2 = pk2(gr, gi), h2 = pk2(hr, hi);
-                const F2 b0 = rule_b2(RI, qs, 0), b1 = rule_b2(RI, qs, 1), b2 = rule_b2(RI, qs, 2);
-                C0 = fma2(b0, g2, C0);
-                C1 = fma2(b1, g2, C1);
-                C2 = fma2(b2, g2, C2);
-                H0 = fma2(b0, h2, H0);
-                H1 = fma2(b1, h2, H1);
-                H2 = fma2(b2, h2, H2);
-                const F2 p2 = mul2(pk2(ync[qs], ync[qs]), h2);
-                P0 = fma2(b0, p2, P0);
-                P1 = fma2(b1, p2, P1);
-                P2 = fma2(b2, p2, P2);
+                const auto g2 = CxSum<T>::make(gr, gi), h2 = CxSum<T>::make(hr, hi);
+#pragma unroll
+                for (int b = 0; b < 3; ++b) Cs[b].add(RI, qs, b, g2);
+#pragma unroll
+                for (int b = 0; b < 3; ++b) Hs[b].add(RI, qs, b, h2);
+                const auto p2 = CxSum<T>::scaled(ync[qs], h2);
+#pragma unroll
+                for (int b = 0; b < 3; ++b) Ps[b].add(RI, qs, b, p2);
             }
             T Cr[3], Ci[3], Hr[3], Hi[3], Pr[3], Pi[3];
-            up2(C0, Cr[0], Ci[0]);
-            up2(C1, Cr[1], Ci[1]);
-            up2(C2, Cr[2], Ci[2]);
-            up2(H0, Hr[0], Hi[0]);
-            up2(H1, Hr[1], Hi[1]);
-            up2(H2, Hr[2], Hi[2]);
-            up2(P0, Pr[0], Pi[0]);
-            up2(P1, Pr[1], Pi[1]);
-            up2(P2, Pr[2], Pi[2]);
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                Cs[b].get(Cr[b], Ci[b]);
+                Hs[b].get(Hr[b], Hi[b]);
+                Ps[b].get(Pr[b], Pi[b]);
+            }
             // order 1's right-hand-side value -G + i eta W, W = sum (r . n_tau) g' / r
             const T Gr = Cr[0] + Cr[1] + Cr[2], Gi = Ci[0] + Ci[1] + Ci[2];
             const T Wr = Pr[0] + Pr[1] + Pr[2], Wi = Pi[0] + Pi[1] + Pi[2];
@@ -744,7 +550,7 @@ __global__ void __launch_bounds__(REG_THREADS, 2) sym_pairs_kernel(RegArgs<float
         for (int a = 0; a < 3; ++a) {
             const int ra = xlv[3 * ti + a];  // vertex a of tau, tile I local
             int off[14];  // this vertex's 14 adds (re and im planes)
-            float val[14];
+            T val[14];
 #pragma unroll
             for (int b = 0; b < 3; ++b) {
                 const T d = xc[9 * ti + 3 * a] * yc[(3 * b) * SYM_F + sj] +
@@ -776,7 +582,7 @@ __global__ void __launch_bounds__(REG_THREADS, 2) sym_pairs_kernel(RegArgs<float
     }
     __syncthreads();
     // fold the slot-face entries onto tile J's vertices and flush
-    for (int i = tid; i < nvI * nvJ; i += REG_THREADS) {
+    for (int i = tid; i < nvI * nvJ; i += THREADS) {
         const int li = i / nvJ, lj = i % nvJ;
         Cx<T> v{T(0), T(0)}, u{T(0), T(0)};
         for (int e = inc_start[lj]; e < inc_start[lj + 1]; ++e) {
@@ -791,13 +597,13 @@ __global__ void __launch_bounds__(REG_THREADS, 2) sym_pairs_kernel(RegArgs<float
         if (u.re != T(0) || u.im != T(0)) red_add_cx(&g.A[(int64_t)gj_ * g.ld + gi_], u.re, u.im);
     }
     if (g.B) {
-        for (int i = tid; i < nvI * nJ; i += REG_THREADS) {
+        for (int i = tid; i < nvI * nJ; i += THREADS) {
             const int li = i / nJ, sj = i % nJ;
             const Cx<T> v{acc_re[SYM_B1 + li * SYM_BS + sj], acc_im[SYM_B1 + li * SYM_BS + sj]};
             if (v.re != T(0) || v.im != T(0))
                 red_add_cx(&g.B[(int64_t)g.t_verts[tv0 + li] * g.F + g.face_id[s0 + sj]], v.re, v.im);
         }
-        for (int i = tid; i < nvJ * nI; i += REG_THREADS) {
+        for (int i = tid; i < nvJ * nI; i += THREADS) {
             const int lj = i / nI, ti = i % nI;
             Cx<T> v{T(0), T(0)};
             for (int e = inc_start[lj]; e < inc_start[lj + 1]; ++e) {
@@ -813,11 +619,11 @@ __global__ void __launch_bounds__(REG_THREADS, 2) sym_pairs_kernel(RegArgs<float
     // matrix-free: rows of b += B1 q (tile I vertices x tile J faces) and
     // B2 q (tile J vertices x tile I faces); q of both tiles' faces staged
     // MF_RC columns at a time over the (now unused) geometry region
-    float2 *qs = reinterpret_cast<float2 *>(xq);  // [2][SYM_F][MF_RC]: tile I faces, then tile J faces
+    Cx<T> *qs = reinterpret_cast<Cx<T> *>(xq);  // [2][SYM_F][MF_RC]: tile I faces, then tile J faces
     // order 2 rows folded onto tile J's vertices, over the (read) C1 block
     constexpr int B2V = SYM_C1;  // [vJ][tau]
     __syncthreads();
-    for (int i = tid; i < nvJ * nI; i += REG_THREADS) {
+    for (int i = tid; i < nvJ * nI; i += THREADS) {
         const int lj = i / nI, ti = i % nI;
         T vr = T(0), vi = T(0);
         for (int e = inc_start[lj]; e < inc_start[lj + 1]; ++e) {
@@ -830,28 +636,28 @@ __global__ void __launch_bounds__(REG_THREADS, 2) sym_pairs_kernel(RegArgs<float
     for (int r0 = 0; r0 < g.R; r0 += MF_RC) {
         const int rc = min(MF_RC, g.R - r0);
         __syncthreads();
-        for (int i = tid; i < 2 * SYM_F * MF_RC; i += REG_THREADS) {
+        for (int i = tid; i < 2 * SYM_F * MF_RC; i += THREADS) {
             const int h = i / (SYM_F * MF_RC), f = (i / MF_RC) % SYM_F, r = i % MF_RC;
-            float2 v = make_float2(0.f, 0.f);
+            Cx<T> v{T(0), T(0)};
             if (f < (h ? nJ : nI) && r < rc) {
                 const Cx<double> qq = g.q[(size_t)(r0 + r) * g.F + g.face_id[(h ? s0 : t0) + f]];
-                v = make_float2((float)qq.re, (float)qq.im);
+                v = Cx<T>{(T)qq.re, (T)qq.im};
             }
             qs[i] = v;
         }
         __syncthreads();
-        for (int i = tid; i < (nvI + nvJ) * rc; i += REG_THREADS) {
+        for (int i = tid; i < (nvI + nvJ) * rc; i += THREADS) {
             const int row = i / rc, r = i % rc;
             const bool first = row < nvI;
             const int base = first ? SYM_B1 + row * SYM_BS : B2V + (row - nvI) * SYM_BS;
             const int nf = first ? nJ : nI;
-            const float2 *qh = qs + (first ? SYM_F * MF_RC : 0);
+            const Cx<T> *qh = qs + (first ? SYM_F * MF_RC : 0);
             T sr = T(0), si = T(0);
             for (int f = 0; f < nf; ++f) {
                 const T br = acc_re[base + f], bi = acc_im[base + f];
-                const float2 qv = qh[f * MF_RC + r];
-                sr += br * qv.x - bi * qv.y;
-                si += br * qv.y + bi * qv.x;
+                const Cx<T> qv = qh[f * MF_RC + r];
+                sr += br * qv.re - bi * qv.im;
+                si += br * qv.im + bi * qv.re;
             }
             const int gv = first ? g.t_verts[tv0 + row] : g.t_verts[sv0 + row - nvI];
             if (sr != T(0) || si != T(0)) red_add_cx(&g.b[(size_t)(r0 + r) * g.N + gv], (double)sr, (double)si);
@@ -1178,25 +984,25 @@ template <typename T> static RhsOut<T> rhs_out(beat_b200_ctx *c, int R, const Cx
     return o;
 }
 
+// the symmetric kernel over unordered pairs of square tiles
 template <typename T, int Q>
-static void launch_regular(beat_b200_ctx *c, double k, double eta, int img, int R, const Cx<double> *q) {
+static void launch_sym(beat_b200_ctx *c, double k, double eta, int img, int R, const Cx<double> *q) {
+    constexpr bool d = sizeof(T) == 8;
+    const Tiling &tiles = d ? c->trial_tiles : c->sym_tiles;
     RegArgs<T> g;
-    const bool d = sizeof(T) == 8;
     g.qpts = (const T *)(d ? c->pos_qpts64.p : c->pos_qpts32.p);
     g.normal = (const T *)(d ? c->pos_normal64.p : c->pos_normal32.p);
     g.curl = (const T *)(d ? c->pos_curl64.p : c->pos_curl32.p);
     g.area = (const T *)(d ? c->pos_area64.p : c->pos_area32.p);
+    g.plane = d ? nullptr : (const T *)c->pos_plane32.p;
     g.gvert = c->pos_gvert.as<int>();
     g.face_id = c->pos_face.as<int>();
-    g.t_fstart = c->test_tiles.face_start.as<int>();
-    g.t_vstart = c->test_tiles.vert_start.as<int>();
-    g.t_verts = c->test_tiles.verts.as<int>();
-    g.t_local = c->test_tiles.local_vert.as<int>();
-    g.s_fstart = c->trial_tiles.face_start.as<int>();
-    g.s_vstart = c->trial_tiles.vert_start.as<int>();
-    g.s_verts = c->trial_tiles.verts.as<int>();
-    g.s_inc = c->trial_tiles.incidence.as<int>();
-    BB_REQUIRE(c->trial_tiles.inc_stride() == REG_INC, BEAT_B200_STATE, "assembly: trial tile shape mismatch");
+    g.t_fstart = tiles.face_start.as<int>();
+    g.t_vstart = tiles.vert_start.as<int>();
+    g.t_verts = tiles.verts.as<int>();
+    g.t_local = tiles.local_vert.as<int>();
+    g.t_inc = tiles.incidence.as<int>();
+    BB_REQUIRE(tiles.inc_stride() == SymTile<T>::INC, BEAT_B200_STATE, "assembly: square tile shape mismatch");
     g.A = c->ws.A.as<Cx<T>>();
     g.B = c->ws.rhs_cached ? c->ws.B.as<Cx<T>>() : nullptr;
     g.q = q;
@@ -1210,60 +1016,17 @@ static void launch_regular(beat_b200_ctx *c, double k, double eta, int img, int 
     g.k2 = (T)(k * k);
     if (img >= 0) {
         g.image = 1;
-        for (int i = 0; i < 3; ++i) g.xs[i] = (T)c->img_sign[img][i];
-        g.xdet = (T)c->img_det[img];
-    }
-    const size_t smem = regular_smem_bytes<T, Q>();
-    BB_CUDA(cudaFuncSetAttribute(regular_pairs_kernel<T, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    BB_CUDA(cudaFuncSetAttribute(regular_pairs_kernel<T, Q>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared));
-    dim3 grid(c->trial_tiles.ntiles, c->test_tiles.ntiles);
-    regular_pairs_kernel<T, Q><<<grid, REG_THREADS, smem, c->stream>>>(g);
-    BB_CUDA(cudaGetLastError());
-}
-
-// FP32 form: the symmetric kernel over unordered pairs of square tiles
-template <int Q>
-static void launch_sym(beat_b200_ctx *c, double k, double eta, int img, int R, const Cx<double> *q) {
-    RegArgs<float> g;
-    g.qpts = c->pos_qpts32.as<float>();
-    g.normal = c->pos_normal32.as<float>();
-    g.curl = c->pos_curl32.as<float>();
-    g.area = c->pos_area32.as<float>();
-    g.plane = c->pos_plane32.as<float>();
-    g.gvert = c->pos_gvert.as<int>();
-    g.face_id = c->pos_face.as<int>();
-    g.t_fstart = c->sym_tiles.face_start.as<int>();
-    g.t_vstart = c->sym_tiles.vert_start.as<int>();
-    g.t_verts = c->sym_tiles.verts.as<int>();
-    g.t_local = c->sym_tiles.local_vert.as<int>();
-    g.t_inc = c->sym_tiles.incidence.as<int>();
-    BB_REQUIRE(c->sym_tiles.inc_stride() == SYM_INC, BEAT_B200_STATE, "assembly: square tile shape mismatch");
-    g.s_fstart = g.s_vstart = g.s_verts = nullptr;
-    g.A = c->ws.A.as<Cx<float>>();
-    g.B = c->ws.rhs_cached ? c->ws.B.as<Cx<float>>() : nullptr;
-    g.q = q;
-    g.b = c->ws.b.as<Cx<double>>();
-    g.N = c->V;
-    g.R = R;
-    g.ld = c->ws.ld;
-    g.F = c->F;
-    g.k = (float)k;
-    g.eta = (float)eta;
-    g.k2 = (float)(k * k);
-    if (img >= 0) {
-        g.image = 1;
         for (int i = 0; i < 3; ++i) g.xs[i] = c->img_sign[img][i];
         g.xdet = c->img_det[img];
     }
-    const size_t smem = sym_smem_bytes<Q>();
-    BB_CUDA(cudaFuncSetAttribute(sym_pairs_kernel<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    BB_CUDA(cudaFuncSetAttribute(sym_pairs_kernel<Q>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    const size_t smem = SymTile<T>::template smem<Q>();
+    BB_CUDA(cudaFuncSetAttribute(sym_pairs_kernel<T, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BB_CUDA(cudaFuncSetAttribute(sym_pairs_kernel<T, Q>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  cudaSharedmemCarveoutMaxShared));  // two CTAs per SM
-    const int64_t nt = c->sym_tiles.ntiles;
+    const int64_t nt = tiles.ntiles;
     const int64_t blocks = nt * (nt + 1) / 2;
     BB_REQUIRE(blocks < (1ll << 31), BEAT_B200_INVALID_ARG, "assembly: mesh too large for the tile-pair grid");
-    sym_pairs_kernel<Q><<<(unsigned)blocks, REG_THREADS, smem, c->stream>>>(g);
+    sym_pairs_kernel<T, Q><<<(unsigned)blocks, SymTile<T>::THREADS, smem, c->stream>>>(g);
     BB_CUDA(cudaGetLastError());
 }
 
@@ -1279,18 +1042,10 @@ template <typename T> static void assemble_t(beat_b200_ctx *c, double k, double 
         BB_CUDA(cudaMemsetAsync(w.b.p, 0, sizeof(Cx<double>) * (size_t)N * R, c->stream));
     BB_CUDA(cudaEventRecord(c->ev[8], c->stream));
     for (int img = -1; img < c->nimg; ++img) {  // the mesh itself, then one pass per symmetry image
-        if (sizeof(T) == 4) {
-            switch (c->Q) {
-                case 1: launch_sym<1>(c, k, eta, img, R, q); break;
-                case 3: launch_sym<3>(c, k, eta, img, R, q); break;
-                default: launch_sym<6>(c, k, eta, img, R, q); break;
-            }
-        } else {
-            switch (c->Q) {
-                case 1: launch_regular<T, 1>(c, k, eta, img, R, q); break;
-                case 3: launch_regular<T, 3>(c, k, eta, img, R, q); break;
-                default: launch_regular<T, 6>(c, k, eta, img, R, q); break;
-            }
+        switch (c->Q) {
+            case 1: launch_sym<T, 1>(c, k, eta, img, R, q); break;
+            case 3: launch_sym<T, 3>(c, k, eta, img, R, q); break;
+            default: launch_sym<T, 6>(c, k, eta, img, R, q); break;
         }
     }
     BB_CUDA(cudaEventRecord(c->ev[1], c->stream));

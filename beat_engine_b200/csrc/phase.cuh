@@ -13,6 +13,7 @@
 #pragma once
 
 #include <math.h>
+#include <string.h>
 
 #if defined(__CUDACC__)
 #define BB_HD __host__ __device__ __forceinline__
@@ -22,8 +23,20 @@
 
 namespace bb {
 
+BB_HD int low_word(double t) {
+#if defined(__CUDA_ARCH__)
+    return __double2loint(t);
+#else
+    long long b;
+    memcpy(&b, &t, sizeof(b));
+    return (int)b;
+#endif
+}
+
 BB_HD void sincos_cw(double x, double *s, double *c) {
-    const double n = rint(x * 0.6366197723675814);  // x * 2/pi
+    // n = x * 2/pi rounded to an integer by adding and subtracting 1.5 * 2^52,
+    // whose sum also holds n in its low bits (no conversion instructions)
+    const double big = 6755399441055744.0, t = x * 0.6366197723675814 + big, n = t - big;
     double r = fma(-n, 1.5707963267341256, x);      // pi/2, leading 33 bits
     r = fma(-n, 6.077100506303966e-11, r);          // next 33 bits
     r = fma(-n, 2.0222662487959506e-21, r);         // remainder
@@ -47,7 +60,7 @@ BB_HD void sincos_cw(double x, double *s, double *c) {
     pc = fma(pc, r2, -1.0 / 24.0);                  // 1/4!
     pc = fma(pc, r2, 0.5);                          // 1/2!
     const double cr = fma(-pc, r2, 1.0);
-    const int q = (int)(long long)n & 3;
+    const int q = low_word(t);
     const double ss = (q & 1) ? cr : sr, cc = (q & 1) ? sr : cr;
     *s = (q & 2) ? -ss : ss;
     *c = ((q + 1) & 2) ? -cc : cc;
