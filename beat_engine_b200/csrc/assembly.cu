@@ -80,15 +80,7 @@ void upload_rule_tables(const std::vector<double> &pts, const std::vector<double
 __device__ __forceinline__ void sincos_rev(float t, float *s, float *c) {
     __sincosf((t - rintf(t)) * 6.2831854820251465f, s, c);
 }
-// 1 / sqrt(x), x a positive normal number: the hardware approximation y (error
-// about 2^-22), then one step of the series (1 - e)^(-1/2) = 1 + e/2 + 3/8 e^2 +
-// ... with e = 1 - x y^2, whose next term 5/16 e^3 is below 2^-60
-__device__ __forceinline__ double rsqrt_t(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
+__device__ __forceinline__ double rsqrt_t(double x) { return rsqrt_series(x); }
 __device__ __forceinline__ float rsqrt_t(float x) { return rsqrtf(x); }
 
 __device__ __forceinline__ void red_add(double *p, double v) { atomicAdd(p, v); }

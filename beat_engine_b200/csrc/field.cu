@@ -11,9 +11,9 @@
 //     p_inf(d) = sum_src exp(-ik d.y)/(4 pi) [ (-ik)(d.n) p_src - q_src ].
 //
 // The reference launches one field kernel per excitation and output; here one
-// kernel evaluates G once per (point, source) for every column.  Points run
-// over threads, sources are staged through shared memory in chunks and the
-// source range is split over CTAs, which add their partial sums with
+// kernel evaluates G once per (point, source) for every column.  A CTA takes
+// 32 points and a part of the sources, staged through shared memory in chunks
+// that its warps share out; the CTAs add their partial sums with
 // red.global.add.  FP64 in both precision forms.
 #include <cuda_runtime.h>
 
@@ -27,9 +27,9 @@
 
 namespace bb {
 
-constexpr int FLD_RC = 16;      // right-hand sides per pass
-constexpr int FLD_CHUNK = 32;   // sources per shared-memory chunk
+constexpr int FLD_CHUNK = 32;    // sources per shared-memory chunk
 constexpr int FLD_THREADS = 128;
+constexpr int FLD_POINTS = 32;   // points per CTA
 
 struct FieldImages {
     int n;            // copies: the mesh itself, then its symmetry images
@@ -68,88 +68,216 @@ __global__ void field_sources_kernel(const double *qpts, const double *normals, 
     }
 }
 
+// Green factor (gr, gi) and double-layer factor (dr, di) of one (point,
+// source): G and G (ik - 1/r) (r.n) / r, r = y - x; FAR: E = exp(-ik d.y) / 4 pi
+// and E (-ik d.n).  Zero at r = 0.
 template <bool FAR>
+__device__ __forceinline__ void field_factors(const double (&x)[3], const double *y, const double *n, double k,
+                                              double &gr, double &gi, double &dr, double &di) {
+    const double inv4pi = 0.07957747154594767;
+    double s, c;
+    if (FAR) {
+        sincos_cw(-k * (x[0] * y[0] + x[1] * y[1] + x[2] * y[2]), &s, &c);
+        gr = c * inv4pi;
+        gi = s * inv4pi;
+        const double dn = k * (x[0] * n[0] + x[1] * n[1] + x[2] * n[2]);
+        dr = gi * dn;
+        di = -gr * dn;
+    } else {
+        const double rx = y[0] - x[0], ry = y[1] - x[1], rz = y[2] - x[2];
+        const double r2 = rx * rx + ry * ry + rz * rz;
+        // (the series wants a normal number; r = 0 contributes nothing)
+        const double ir = r2 < 2.2250738585072014e-308 ? (r2 == 0.0 ? 0.0 : rsqrt(r2)) : rsqrt_series(r2);
+        sincos_cw(k * (r2 * ir), &s, &c);
+        const double a = inv4pi * ir, proj = (rx * n[0] + ry * n[1] + rz * n[2]) * ir;
+        gr = c * a;
+        gi = s * a;
+        dr = (-gr * ir - gi * k) * proj;
+        di = (gr * k - gi * ir) * proj;
+    }
+}
+
+__device__ __forceinline__ void field_point(const double *pts, int m, int M, bool unit, double (&x)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) x[i] = m < M ? pts[3 * (size_t)m + i] : (i == 0 ? 1.0 : 0.0);
+    if (unit) {
+        const double nn = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) x[i] /= nn;
+    }
+}
+
+// Up to two right-hand sides: a lane per point, the warps take every fourth
+// source.  Bound: the FP64 units, about 45 + 8 RC instructions per (point,
+// source).
+template <bool FAR, int RC>
 __global__ void __launch_bounds__(FLD_THREADS) field_eval_kernel(const double *pts, int M, const double *ys,
                                                                  const double *ns, const double2 *ps,
                                                                  const double2 *qs, int S, int R, int r0,
                                                                  int per_cta, double k, double2 *out) {
-    __shared__ double sy[FLD_CHUNK][3], sn[FLD_CHUNK][3];
-    __shared__ double2 sp[FLD_RC][FLD_CHUNK], sq[FLD_RC][FLD_CHUNK];
-    const int m = blockIdx.x * FLD_THREADS + threadIdx.x;
+    __shared__ __align__(16) double sg[FLD_CHUNK][6];  // y, n
+    __shared__ double2 sp[FLD_CHUNK][RC], sq[FLD_CHUNK][RC];
+    __shared__ double2 part[FLD_THREADS / 32][RC][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int m = blockIdx.x * FLD_POINTS + lane;
     const int s_begin = blockIdx.y * per_cta, s_end = min(S, s_begin + per_cta);
-    const int rc = min(FLD_RC, R - r0);
-    double x0 = 0, x1 = 0, x2 = 0;
-    if (m < M) {
-        x0 = pts[3 * m];
-        x1 = pts[3 * m + 1];
-        x2 = pts[3 * m + 2];
-        if (FAR) {
-            const double nn = sqrt(x0 * x0 + x1 * x1 + x2 * x2);
-            x0 /= nn;
-            x1 /= nn;
-            x2 /= nn;
-        }
-    }
-    double ar[FLD_RC], ai[FLD_RC];
+    double x[3];
+    field_point(pts, m, M, FAR, x);
+    double ar[RC], ai[RC];
 #pragma unroll
-    for (int r = 0; r < FLD_RC; ++r) ar[r] = ai[r] = 0.0;
-    const double inv4pi = 0.07957747154594767;
+    for (int r = 0; r < RC; ++r) ar[r] = ai[r] = 0.0;
     for (int c0 = s_begin; c0 < s_end; c0 += FLD_CHUNK) {
         const int cn = min(FLD_CHUNK, s_end - c0);
         __syncthreads();
         for (int i = threadIdx.x; i < cn * 3; i += FLD_THREADS) {
-            sy[i / 3][i % 3] = ys[3 * (size_t)c0 + i];
-            sn[i / 3][i % 3] = ns[3 * (size_t)c0 + i];
+            sg[i / 3][i % 3] = ys[3 * (size_t)c0 + i];
+            sg[i / 3][3 + i % 3] = ns[3 * (size_t)c0 + i];
         }
-        for (int i = threadIdx.x; i < FLD_RC * FLD_CHUNK; i += FLD_THREADS) {
+        for (int i = threadIdx.x; i < RC * FLD_CHUNK; i += FLD_THREADS) {
             const int r = i / FLD_CHUNK, j = i % FLD_CHUNK;
-            const bool ok = r < rc && j < cn;
-            sp[r][j] = ok ? ps[(size_t)(r0 + r) * S + c0 + j] : make_double2(0, 0);
-            sq[r][j] = ok ? qs[(size_t)(r0 + r) * S + c0 + j] : make_double2(0, 0);
+            const bool ok = r0 + r < R && j < cn;
+            sp[j][r] = ok ? ps[(size_t)(r0 + r) * S + c0 + j] : make_double2(0, 0);
+            sq[j][r] = ok ? qs[(size_t)(r0 + r) * S + c0 + j] : make_double2(0, 0);
         }
         __syncthreads();
-        if (m >= M) continue;
-        for (int j = 0; j < cn; ++j) {
-            double gr, gi, dr, di;  // green and double-layer factors
-            if (!FAR) {
-                const double rx = sy[j][0] - x0, ry = sy[j][1] - x1, rz = sy[j][2] - x2;
-                const double r2 = rx * rx + ry * ry + rz * rz;
-                if (r2 == 0.0) continue;
-                const double ir = rsqrt(r2), rad = r2 * ir;
-                double sn_, cs_;
-                sincos_cw(k * rad, &sn_, &cs_);
-                gr = cs_ * inv4pi * ir;
-                gi = sn_ * inv4pi * ir;
-                const double proj = (rx * sn[j][0] + ry * sn[j][1] + rz * sn[j][2]) * ir;
-                // G (ik - 1/r) proj
-                dr = (gr * -ir - gi * k) * proj;
-                di = (gr * k + gi * -ir) * proj;
-            } else {
-                const double ph = -k * (x0 * sy[j][0] + x1 * sy[j][1] + x2 * sy[j][2]);
-                double sn_, cs_;
-                sincos_cw(ph, &sn_, &cs_);
-                gr = cs_ * inv4pi;
-                gi = sn_ * inv4pi;
-                const double dn = x0 * sn[j][0] + x1 * sn[j][1] + x2 * sn[j][2];
-                // e (-ik dn)
-                dr = gi * k * dn;
-                di = -gr * k * dn;
-            }
+#pragma unroll 2
+        for (int j = warp; j < cn; j += FLD_THREADS / 32) {
+            double gr, gi, dr, di;
+            field_factors<FAR>(x, sg[j], sg[j] + 3, k, gr, gi, dr, di);
 #pragma unroll
-            for (int r = 0; r < FLD_RC; ++r) {
-                const double2 pv = sp[r][j], qv = sq[r][j];
+            for (int r = 0; r < RC; ++r) {
+                const double2 pv = sp[j][r], qv = sq[j][r];
                 ar[r] += dr * pv.x - di * pv.y - (gr * qv.x - gi * qv.y);
                 ai[r] += dr * pv.y + di * pv.x - (gr * qv.y + gi * qv.x);
             }
         }
     }
-    if (m < M) {
 #pragma unroll
-        for (int r = 0; r < FLD_RC; ++r)
-            if (r < rc) {
-                atomicAdd(&out[(size_t)(r0 + r) * M + m].x, ar[r]);
-                atomicAdd(&out[(size_t)(r0 + r) * M + m].y, ai[r]);
+    for (int r = 0; r < RC; ++r) part[warp][r][lane] = make_double2(ar[r], ai[r]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < RC * 32; i += FLD_THREADS) {
+        const int r = i / 32, mm = blockIdx.x * FLD_POINTS + i % 32;
+        double2 v = make_double2(0, 0);
+#pragma unroll
+        for (int w = 0; w < FLD_THREADS / 32; ++w) {
+            v.x += part[w][r][i % 32].x;
+            v.y += part[w][r][i % 32].y;
+        }
+        if (mm < M && r0 + r < R) {
+            atomicAdd(&out[(size_t)(r0 + r) * M + mm].x, v.x);
+            atomicAdd(&out[(size_t)(r0 + r) * M + mm].y, v.y);
+        }
+    }
+}
+
+// Three and more right-hand sides: the sums over the sources are a real matrix
+// product, points x (4 factors per source) times (4 per source) x (2 R), on
+// the FP64 tensor cores (mma.sync.m8n8k4.f64; operand places as in the LU's
+// FP64 update).  A warp takes 8 points x 4 sources at a time: lane (g, t)
+// evaluates point g and source t once, and its factor i (dr, di, gr, gi) is its
+// A operand of the i-th product, whose K index is the source; the B operand is
+// then row i of source t,
+//     p, ip (real parts of i p), -q, -iq,   columns (re, im) of each side,
+// staged once per chunk.  So neither factors nor sums move between lanes.
+// NB: blocks of 8 real columns, 4 NB right-hand sides.  Each warp holds PG
+// groups of 8 points, so a B operand feeds PG products.
+// Bound: the FP64 units (about 45 + 32 NB FP64 instructions' worth per (point,
+// source)); a thread per point with 16 sides in registers read 32 broadcast
+// 16-byte values of shared memory per source and was held by those: field at
+// 2,000 points, 16 sides, 71,184 sources 2.9 ms, this 2.05.
+constexpr int FLD_PG = FLD_POINTS / 8;
+template <int NB> struct FieldB {
+    static constexpr int LD = NB == 1 ? 8 : 8 * NB + 8;  // row stride: 8 mod 16 doubles, two wavefronts a load
+};
+template <bool FAR, int NB>
+__global__ void __launch_bounds__(FLD_THREADS) field_mma_kernel(const double *pts, int M, const double *ys,
+                                                                const double *ns, const double2 *ps,
+                                                                const double2 *qs, int S, int R, int r0, int per_cta,
+                                                                double k, double2 *out) {
+    constexpr int RC = 4 * NB, LD = FieldB<NB>::LD, WARPS = FLD_THREADS / 32, PART = 2 * RC + 1;
+    __shared__ double sg[FLD_CHUNK][7];  // y, n; odd stride
+    union Chunk {
+        double b[4][FLD_CHUNK * LD];               // B rows of the chunk's sources
+        double part[WARPS][FLD_POINTS * PART / 2];  // (half the warps' sums at a time)
+    };
+    __shared__ Chunk ch;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int s_begin = blockIdx.y * per_cta, s_end = min(S, s_begin + per_cta);
+    double x[FLD_PG][3], c[FLD_PG][NB][2];
+#pragma unroll
+    for (int a = 0; a < FLD_PG; ++a) {
+        field_point(pts, blockIdx.x * FLD_POINTS + 8 * a + g, M, FAR, x[a]);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) c[a][b][0] = c[a][b][1] = 0.0;
+    }
+    for (int c0 = s_begin; c0 < s_end; c0 += FLD_CHUNK) {
+        const int cn = min(FLD_CHUNK, s_end - c0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < FLD_CHUNK * 3; i += FLD_THREADS) {
+            const bool ok = i < cn * 3;
+            sg[i / 3][i % 3] = ok ? ys[3 * (size_t)c0 + i] : 0.0;
+            sg[i / 3][3 + i % 3] = ok ? ns[3 * (size_t)c0 + i] : 0.0;
+        }
+        for (int i = threadIdx.x; i < RC * FLD_CHUNK; i += FLD_THREADS) {
+            const int r = i / FLD_CHUNK, j = i % FLD_CHUNK;
+            const bool ok = r0 + r < R && j < cn;
+            const double2 p = ok ? ps[(size_t)(r0 + r) * S + c0 + j] : make_double2(0, 0);
+            const double2 q = ok ? qs[(size_t)(r0 + r) * S + c0 + j] : make_double2(0, 0);
+            const int o = j * LD + 2 * r;
+            ch.b[0][o] = p.x, ch.b[0][o + 1] = p.y;
+            ch.b[1][o] = -p.y, ch.b[1][o + 1] = p.x;
+            ch.b[2][o] = -q.x, ch.b[2][o + 1] = -q.y;
+            ch.b[3][o] = q.y, ch.b[3][o + 1] = -q.x;
+        }
+        __syncthreads();
+        for (int j0 = 4 * warp; j0 < cn; j0 += 4 * WARPS) {
+            const double *sj = sg[j0 + t];
+            const double y[3] = {sj[0], sj[1], sj[2]}, n[3] = {sj[3], sj[4], sj[5]};
+            double f[FLD_PG][4];
+#pragma unroll
+            for (int a = 0; a < FLD_PG; ++a) field_factors<FAR>(x[a], y, n, k, f[a][2], f[a][3], f[a][0], f[a][1]);
+            if (j0 + 4 > cn && j0 + t >= cn) {  // past the last source
+#pragma unroll
+                for (int a = 0; a < FLD_PG; ++a)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) f[a][i] = 0.0;
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    const double bv = ch.b[i][(j0 + t) * LD + 8 * b + g];
+#pragma unroll
+                    for (int a = 0; a < FLD_PG; ++a)
+                        asm volatile(
+                            "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                            : "+d"(c[a][b][0]), "+d"(c[a][b][1])
+                            : "d"(f[a][i]), "d"(bv));
+                }
+        }
+    }
+    // the warps' sums meet in shared memory, half of the points at a time:
+    // lane (g, t) holds point 8 a + g, real columns 8 b + 2 t, 8 b + 2 t + 1
+    constexpr int HALF = FLD_PG / 2;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        __syncthreads();
+#pragma unroll
+        for (int a = 0; a < HALF; ++a)
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    ch.part[warp][(8 * a + g) * PART + 8 * b + 2 * t + e] = c[h * HALF + a][b][e];
+        __syncthreads();
+        for (int i = threadIdx.x; i < 8 * HALF * 2 * RC; i += FLD_THREADS) {
+            const int col = i / (8 * HALF), pt = i % (8 * HALF), r = r0 + col / 2;
+            const int m = blockIdx.x * FLD_POINTS + 8 * HALF * h + pt;
+            double v = 0.0;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) v += ch.part[w][pt * PART + col];
+            if (m < M && r < R) atomicAdd(reinterpret_cast<double *>(&out[(size_t)r * M + m]) + (col & 1), v);
+        }
     }
 }
 
@@ -219,6 +347,35 @@ static std::pair<dim3, int> source_split(const beat_b200_ctx *c, int M, int S, i
     return {dim3(mt, (S + per - 1) / per), per};
 }
 
+// The source range in as many parts as fill whole waves of resident CTAs best
+// (a part has at least four chunks): with 63 tiles of points and 444 CTAs
+// resident, 9 parts leave the second wave 28 % full (2.68 ms for the product
+// kernel above), 7 make one wave (2.05 ms).
+struct SourceSplit {
+    dim3 grid;
+    int per;  // sources per CTA
+};
+template <typename K> static SourceSplit resident_split(const beat_b200_ctx *c, K *kernel, int M, int S) {
+    int per_sm = 1;
+    BB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, FLD_THREADS, 0));
+    const int64_t cap = (int64_t)std::max(1, per_sm) * c->sm_count;
+    const int mt = (M + FLD_POINTS - 1) / FLD_POINTS, chunks = (S + FLD_CHUNK - 1) / FLD_CHUNK;
+    const int most = (int)std::min<int64_t>(std::max(1, chunks / 4), std::max<int64_t>(1, 4 * cap / mt));
+    int best = 1;
+    double best_use = 0;
+    for (int n = 1; n <= most; ++n) {
+        const int per = (chunks + n - 1) / n, parts = (chunks + per - 1) / per;
+        const int64_t ctas = (int64_t)mt * parts, waves = (ctas + cap - 1) / cap;
+        const double use = (double)mt * chunks / ((double)waves * cap * per);  // useful share of the waves' time
+        if (use > best_use * 1.02) {
+            best = n;
+            best_use = use;
+        }
+    }
+    const int per = (chunks + best - 1) / best * FLD_CHUNK;
+    return {dim3(mt, (S + per - 1) / per), per};
+}
+
 void farfield(beat_b200_ctx *c, double k, int M, const double *pts_host, int R, const double *p_dev,
               const double *q_dev, double *out_dev, bool far) {
     BB_REQUIRE(c->F > 0, BEAT_B200_STATE, "no mesh: call beat_b200_set_mesh first");
@@ -226,17 +383,27 @@ void farfield(beat_b200_ctx *c, double k, int M, const double *pts_host, int R, 
     if (M == 0) return;
     const StagedSources st = stage_sources(c, M, pts_host, R, p_dev, q_dev);
     BB_CUDA(cudaMemsetAsync(out_dev, 0, sizeof(double2) * (size_t)M * R, c->stream));
-    const auto [grid, per] = source_split(c, M, st.S, FLD_THREADS, FLD_CHUNK);
-    for (int r0 = 0; r0 < R; r0 += FLD_RC) {
-        if (far)
-            field_eval_kernel<true><<<grid, FLD_THREADS, 0, c->stream>>>(st.pts, M, st.ys, st.ns, st.ps, st.qs, st.S,
-                                                                         R, r0, per, k,
-                                                                         reinterpret_cast<double2 *>(out_dev));
-        else
-            field_eval_kernel<false><<<grid, FLD_THREADS, 0, c->stream>>>(st.pts, M, st.ys, st.ns, st.ps, st.qs, st.S,
-                                                                          R, r0, per, k,
-                                                                          reinterpret_cast<double2 *>(out_dev));
+    // by the columns left: one or two in registers (the products would spend 8
+    // real columns on 2 or 4: 45 + 32 against 45 + 8 instructions for one),
+    // then products of 4, 8 and 16
+    auto pass = [&](auto *kernel, int r0) {
+        const SourceSplit sp = resident_split(c, kernel, M, st.S);
+        kernel<<<sp.grid, FLD_THREADS, 0, c->stream>>>(st.pts, M, st.ys, st.ns, st.ps, st.qs, st.S, R, r0, sp.per, k,
+                                                       reinterpret_cast<double2 *>(out_dev));
         BB_CUDA(cudaGetLastError());
+    };
+    for (int r0 = 0; r0 < R; r0 += 16) {
+        const int left = R - r0;
+        if (left == 1)
+            pass(far ? field_eval_kernel<true, 1> : field_eval_kernel<false, 1>, r0);
+        else if (left == 2)
+            pass(far ? field_eval_kernel<true, 2> : field_eval_kernel<false, 2>, r0);
+        else if (left <= 4)
+            pass(far ? field_mma_kernel<true, 1> : field_mma_kernel<false, 1>, r0);
+        else if (left <= 8)
+            pass(far ? field_mma_kernel<true, 2> : field_mma_kernel<false, 2>, r0);
+        else
+            pass(far ? field_mma_kernel<true, 4> : field_mma_kernel<false, 4>, r0);
     }
     BB_CUDA(cudaStreamSynchronize(c->stream));
 }

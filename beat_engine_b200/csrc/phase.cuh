@@ -89,4 +89,16 @@ BB_HD void sincos_cw(float x, float *s, float *c) {
     *c = ((q + 1) & 2) ? -cc : cc;
 }
 
+#if defined(__CUDACC__)
+// 1 / sqrt(x), x a positive normal number: the hardware approximation y (error
+// about 2^-22), then one step of the series (1 - e)^(-1/2) = 1 + e/2 + 3/8 e^2 +
+// ... with e = 1 - x y^2, whose next term 5/16 e^3 is below 2^-60
+__device__ __forceinline__ double rsqrt_series(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+#endif
+
 }  // namespace bb
