@@ -1103,7 +1103,7 @@ template <typename T> static void assemble_t(beat_b200_ctx *c, double k, double 
             rhs_out<T>(c, R, q));
         BB_CUDA(cudaGetLastError());
     }
-    if (w.rhs_cached) {
+    if (w.rhs_cached && R > 0) {
         BB_CUDA(cudaMemsetAsync(w.b.p, 0, sizeof(Cx<double>) * (size_t)N * R, c->stream));
         tall_gemm<T>(c->stream, c->sm_count, w.B.as<Cx<T>>(), F, N, F, reinterpret_cast<const double *>(q),
                      w.b.as<double>(), R, 1.0);

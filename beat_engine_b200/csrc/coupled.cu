@@ -76,41 +76,69 @@ __global__ void csc_projection_kernel(const Cx<T> *C, int n, int F, const int *c
     }
 }
 
-// out (n x m, column-major) = scale C D, C n x F and D F x m column-major:
-// one thread per row, CP_COLS columns of D per pass staged through shared
-// memory, C read once per pass (coalesced down the rows)
-constexpr int CP_COLS = 8, CP_KCHUNK = 64, CP_THREADS = 256;
+// out (n x m, column-major) = scale C D, C n x F and D F x m column-major.  A
+// CTA takes 32 rows, a lane each, and its warps share the F columns of C, which
+// they read coalesced down the rows, several loads in flight before a chunk of
+// D (CP_COLS columns per pass, in shared memory) is waited for; the warps' sums
+// meet in shared memory.  Bound: HBM or L2, C is read once per pass.  (One
+// thread per row over all of F kept 8 CTAs busy at n = 2,000, F = 4,000: 1.21 ms
+// a product, this 0.07.)
+constexpr int CP_COLS = 8, CP_ROWS = 32, CP_WARPS = 16, CP_THREADS = 32 * CP_WARPS;
 
 template <typename T>
 __global__ void __launch_bounds__(CP_THREADS) dense_product_kernel(const Cx<T> *C, int n, int F, const Cx<T> *D,
                                                                     int m, int j0, T scale, Cx<T> *out) {
-    __shared__ Cx<T> sd[CP_KCHUNK][CP_COLS];
-    const int row = blockIdx.x * CP_THREADS + threadIdx.x;
+    constexpr int PER = sizeof(T) == 4 ? 8 : 4, KCHUNK = PER * CP_WARPS, HALF = CP_COLS / 2;
+    __shared__ Cx<T> sd[KCHUNK][CP_COLS];
+    __shared__ Cx<T> part[CP_WARPS][CP_ROWS][HALF];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row = blockIdx.x * CP_ROWS + lane;
     const int jc = min(CP_COLS, m - j0);
     T ar[CP_COLS], ai[CP_COLS];
 #pragma unroll
     for (int j = 0; j < CP_COLS; ++j) ar[j] = ai[j] = T(0);
-    for (int f0 = 0; f0 < F; f0 += CP_KCHUNK) {
-        const int fc = min(CP_KCHUNK, F - f0);
-        __syncthreads();
-        for (int i = threadIdx.x; i < CP_KCHUNK * CP_COLS; i += CP_THREADS) {
-            const int f = i / CP_COLS, j = i % CP_COLS;
-            sd[f][j] = (f < fc && j < jc) ? D[(int64_t)(j0 + j) * F + f0 + f] : Cx<T>{T(0), T(0)};
+    for (int f0 = 0; f0 < F; f0 += KCHUNK) {
+        Cx<T> a[PER];
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int f = f0 + u * CP_WARPS + warp;
+            a[u] = (row < n && f < F) ? C[(int64_t)f * n + row] : Cx<T>{T(0), T(0)};
         }
         __syncthreads();
-        if (row >= n) continue;
-        for (int f = 0; f < fc; ++f) {
-            const Cx<T> a = C[(int64_t)(f0 + f) * n + row];
+        for (int i = threadIdx.x; i < KCHUNK * CP_COLS; i += CP_THREADS) {
+            const int j = i / KCHUNK, f = i % KCHUNK;
+            sd[f][j] = (f0 + f < F && j < jc) ? D[(int64_t)(j0 + j) * F + f0 + f] : Cx<T>{T(0), T(0)};
+        }
+        __syncthreads();
 #pragma unroll
-            for (int j = 0; j < CP_COLS; ++j) {
-                const Cx<T> b = sd[f][j];
-                ar[j] += a.re * b.re - a.im * b.im;
-                ai[j] += a.re * b.im + a.im * b.re;
+        for (int u = 0; u < PER; ++u)
+            if (f0 + u * CP_WARPS + warp < F) {
+#pragma unroll
+                for (int j = 0; j < CP_COLS; ++j) {
+                    const Cx<T> b = sd[u * CP_WARPS + warp][j];
+                    ar[j] += a[u].re * b.re - a[u].im * b.im;
+                    ai[j] += a[u].re * b.im + a[u].im * b.re;
+                }
             }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < HALF; ++j) part[warp][lane][j] = Cx<T>{ar[h * HALF + j], ai[h * HALF + j]};
+        __syncthreads();
+        for (int i = threadIdx.x; i < CP_ROWS * HALF; i += CP_THREADS) {
+            const int j = i / CP_ROWS, r = i % CP_ROWS;
+            T vr = T(0), vi = T(0);
+#pragma unroll
+            for (int w = 0; w < CP_WARPS; ++w) {
+                vr += part[w][r][j].re;
+                vi += part[w][r][j].im;
+            }
+            if (blockIdx.x * CP_ROWS + r < n && h * HALF + j < jc)
+                out[(int64_t)(j0 + h * HALF + j) * n + blockIdx.x * CP_ROWS + r] = Cx<T>{scale * vr, scale * vi};
         }
     }
-    if (row < n)
-        for (int j = 0; j < jc; ++j) out[(int64_t)(j0 + j) * n + row] = Cx<T>{scale * ar[j], scale * ai[j]};
 }
 
 template <typename T>
@@ -139,8 +167,7 @@ void assemble_coupled(beat_b200_ctx *c, double k, int precision, void *d_A, void
     ensure_workspace(c, precision, 1, BEAT_B200_RHS_CACHED);
     BB_REQUIRE(c->ws.rhs_cached, BEAT_B200_OOM, "coupled assembly: the N x F operator C does not fit in memory");
     Workspace &w = c->ws;
-    BB_CUDA(cudaMemsetAsync(w.q.p, 0, (size_t)c->F * 16, c->stream));
-    assemble(c, k, 1.0 / k, precision, 1, w.q.p, nullptr, nullptr);  // alpha = i / k
+    assemble(c, k, 1.0 / k, precision, 0, w.q.p, nullptr, nullptr);  // alpha = i / k; the operators alone, no column
     w.lu_valid = 0;
     if (precision == BEAT_B200_FP64)
         export_coupled<double>(c, d_A, d_C);
@@ -168,7 +195,7 @@ static void blocks_t(beat_b200_ctx *c, const void *d_C, int ncols, const int *co
         BB_CUDA(cudaGetLastError());
         BB_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     }
-    const int rb = (n + CP_THREADS - 1) / CP_THREADS;
+    const int rb = (n + CP_ROWS - 1) / CP_ROWS;
     for (int j0 = 0; j0 < nm; j0 += CP_COLS) {
         dense_product_kernel<T><<<rb, CP_THREADS, 0, c->stream>>>(C, n, F, static_cast<const Cx<T> *>(d_motion), nm,
                                                                  j0, T(1), static_cast<Cx<T> *>(d_motion_out));

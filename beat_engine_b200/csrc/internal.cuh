@@ -270,7 +270,8 @@ void upload_rule_tables(const std::vector<double> &pts, const std::vector<double
 // context.cu: triangle_rule(T, order) of the reference (weights sum to 1/2)
 int triangle_rule(int order, std::vector<double> &pts, std::vector<double> &w);
 // assembly.cu: A (row-major N x ld) and B (N x F) in the workspace precision,
-// then b = B q (FP64, N x R column-major).  q_dev is F x R FP64 complex.
+// then b = B q (FP64, N x R column-major).  q_dev is F x R FP64 complex; R = 0
+// (cached mode) forms A and B alone.
 void assemble(beat_b200_ctx *c, double k, double eta, int precision, int R, const void *q_dev,
               float *ms_total, float *ms_singular);
 
