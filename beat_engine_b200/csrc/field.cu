@@ -338,15 +338,6 @@ static StagedSources stage_sources(beat_b200_ctx *c, int M, const double *pts_ho
     return st;
 }
 
-// CTAs over the source range so that the grid fills the GPU: (grid, sources per CTA)
-static std::pair<dim3, int> source_split(const beat_b200_ctx *c, int M, int S, int threads, int chunk) {
-    const int mt = (M + threads - 1) / threads;
-    const int want = std::max(1, (4 * c->sm_count) / mt);
-    int per = std::max(chunk, (S + want - 1) / want);
-    per = (per + chunk - 1) / chunk * chunk;
-    return {dim3(mt, (S + per - 1) / per), per};
-}
-
 // The source range in as many parts as fill whole waves of resident CTAs best
 // (a part has at least four chunks): with 63 tiles of points and 444 CTAs
 // resident, 9 parts leave the second wave 28 % full (2.68 ms for the product
@@ -427,8 +418,8 @@ void farfield(beat_b200_ctx *c, double k, int M, const double *pts_host, int R, 
 // leaf taking the fourth-order rule; a piece still too large at depth 12
 // means the point is too close to the boundary (an error, as in the
 // reference).  The reference runs that correction on host threads after the
-// device sum; here both run on the device, the correction one thread per
-// (point, near face) with an explicit subdivision stack.
+// device sum; here both run on the device, the correction one warp per (point,
+// near face) with an explicit subdivision stack, a piece per lane.
 //
 // Output layout: M x 4 x R complex, column-major, component d (0 value,
 // 1..3 d/dx, d/dy, d/dz) of column r at out[m + M (d + 4 r)].
@@ -437,7 +428,8 @@ constexpr int FG_RC = 4;          // right-hand sides per pass
 constexpr int FG_CHUNK = 32;
 constexpr int FG_THREADS = 128;
 constexpr int FG_MAX_DEPTH = 12;
-constexpr int FG_STACK = 3 * FG_MAX_DEPTH + 1;   // pending pieces of a depth-first split, at most
+constexpr int FG_STACK = 32 * (3 * FG_MAX_DEPTH + 1);  // pending pieces of a split taken 32 at a time, at most
+constexpr int FG_NEAR_WARPS = 2;                     // near pairs per CTA of the correction
 constexpr int FG_SCALE = 1 << FG_MAX_DEPTH;      // piece vertices are multiples of 1/4096 in face coordinates
 constexpr long long FG_PIECE_BUDGET = 1 << 22;   // pieces per (point, face): a bound on runaway refinement
 constexpr int FG_ERR_TOO_CLOSE = 1, FG_ERR_BUDGET = 2;
@@ -457,7 +449,7 @@ __device__ __forceinline__ void grad_source(double x0, double x1, double x2, dou
     const double rx = y0 - x0, ry = y1 - x1, rz = y2 - x2;
     const double r2 = rx * rx + ry * ry + rz * rz;
     if (r2 == 0.0) return;
-    const double ir = rsqrt(r2), rad = r2 * ir;
+    const double ir = r2 < 2.2250738585072014e-308 ? rsqrt(r2) : rsqrt_series(r2), rad = r2 * ir;
     const double u[3] = {rx * ir, ry * ir, rz * ir}, nn[3] = {n0, n1, n2};
     double sn_, cs_;
     sincos_cw(k * rad, &sn_, &cs_);
@@ -488,23 +480,21 @@ __device__ __forceinline__ void grad_source(double x0, double x1, double x2, dou
     }
 }
 
-// regular sum over the staged sources (weights and densities premultiplied)
+// regular sum over the staged sources (weights and densities premultiplied):
+// a lane per point, the CTA's warps take every fourth source, as in the field
 template <int RC>
 __global__ void __launch_bounds__(FG_THREADS) field_grad_kernel(const double *pts, int M, const double *ys,
                                                                 const double *ns, const double2 *ps,
                                                                 const double2 *qs, int S, int R, int r0, int per_cta,
                                                                 double k, double2 *out) {
-    __shared__ double sy[FG_CHUNK][3], sn[FG_CHUNK][3];
+    __shared__ double sg[FG_CHUNK][6];  // y, n
     __shared__ double2 sp[FG_CHUNK][RC], sq[FG_CHUNK][RC];
-    const int m = blockIdx.x * FG_THREADS + threadIdx.x;
+    __shared__ double part[FG_THREADS / 32][RC * 8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int m = blockIdx.x * FLD_POINTS + lane;
     const int s_begin = blockIdx.y * per_cta, s_end = min(S, s_begin + per_cta);
-    const int rc = min(RC, R - r0);
-    double x0 = 0, x1 = 0, x2 = 0;
-    if (m < M) {
-        x0 = pts[3 * m];
-        x1 = pts[3 * m + 1];
-        x2 = pts[3 * m + 2];
-    }
+    double x[3];
+    field_point(pts, m, M, false, x);
     double acc[RC][8];
 #pragma unroll
     for (int r = 0; r < RC; ++r)
@@ -514,29 +504,33 @@ __global__ void __launch_bounds__(FG_THREADS) field_grad_kernel(const double *pt
         const int cn = min(FG_CHUNK, s_end - c0);
         __syncthreads();
         for (int i = threadIdx.x; i < cn * 3; i += FG_THREADS) {
-            sy[i / 3][i % 3] = ys[3 * (size_t)c0 + i];
-            sn[i / 3][i % 3] = ns[3 * (size_t)c0 + i];
+            sg[i / 3][i % 3] = ys[3 * (size_t)c0 + i];
+            sg[i / 3][3 + i % 3] = ns[3 * (size_t)c0 + i];
         }
         for (int i = threadIdx.x; i < RC * FG_CHUNK; i += FG_THREADS) {
             const int r = i / FG_CHUNK, j = i % FG_CHUNK;
-            const bool ok = r < rc && j < cn;
+            const bool ok = r0 + r < R && j < cn;
             sp[j][r] = ok ? ps[(size_t)(r0 + r) * S + c0 + j] : make_double2(0, 0);
             sq[j][r] = ok ? qs[(size_t)(r0 + r) * S + c0 + j] : make_double2(0, 0);
         }
         __syncthreads();
-        if (m >= M) continue;
-        for (int j = 0; j < cn; ++j)
-            grad_source<RC>(x0, x1, x2, sy[j][0], sy[j][1], sy[j][2], sn[j][0], sn[j][1], sn[j][2], 1.0, k, sp[j],
-                               sq[j], acc);
+#pragma unroll 2
+        for (int j = warp; j < cn; j += FG_THREADS / 32)
+            grad_source<RC>(x[0], x[1], x[2], sg[j][0], sg[j][1], sg[j][2], sg[j][3], sg[j][4], sg[j][5], 1.0, k,
+                            sp[j], sq[j], acc);
     }
-    if (m < M) {
-        for (int r = 0; r < rc; ++r)
 #pragma unroll
-            for (int d = 0; d < 4; ++d) {
-                double2 *o = &out[(size_t)m + (size_t)M * (d + 4 * (size_t)(r0 + r))];
-                atomicAdd(&o->x, acc[r][2 * d]);
-                atomicAdd(&o->y, acc[r][2 * d + 1]);
-            }
+    for (int r = 0; r < RC; ++r)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) part[warp][8 * r + e][lane] = acc[r][e];
+    __syncthreads();
+    for (int i = threadIdx.x; i < RC * 8 * 32; i += FG_THREADS) {
+        const int e = i / 32, mm = blockIdx.x * FLD_POINTS + i % 32, r = r0 + e / 8, d = e % 8 / 2;
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < FG_THREADS / 32; ++w) v += part[w][e][i % 32];
+        if (mm < M && r < R)
+            atomicAdd(reinterpret_cast<double *>(&out[(size_t)mm + (size_t)M * (d + 4 * (size_t)r)]) + (e & 1), v);
     }
 }
 
@@ -569,144 +563,184 @@ __device__ __forceinline__ double dist_to_centroid(const double (&v)[3][3], doub
 }
 
 // (point, face copy) pairs with the face's centroid within 3 diameters of the
-// point; item = m * (F * copies) + copy * F + f, written while slots last
+// point; item = m * (F * copies) + copy * F + f, written while slots last.  A
+// thread per face copy, so that its diameter and centroid are formed once, and
+// a part of the points per blockIdx.y.
 __global__ void near_pairs_kernel(const double *pts, int M, const double *verts, const int *faces, int F,
-                                  FieldImages images, long long *items, long long cap, unsigned long long *count) {
-    const long long total = (long long)M * F * images.n;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int f = (int)(t % F);
-        const long long rest = t / F;
-        const int ix = (int)(rest % images.n), m = (int)(rest / images.n);
-        double v[3][3];
-        face_corners(verts, faces, f, images.s[ix], v);
-        const double diam = tri_diameter(v);
-        if (dist_to_centroid(v, pts[3 * m], pts[3 * m + 1], pts[3 * m + 2]) <= 3.0 * diam) {
+                                  FieldImages images, int per, long long *items, long long cap,
+                                  unsigned long long *count) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= F * images.n) return;
+    double v[3][3];
+    face_corners(verts, faces, e % F, images.s[e / F], v);
+    const double reach = 3.0 * tri_diameter(v), bound = 1.000001 * reach * reach;
+    const double cx = (v[0][0] + v[1][0] + v[2][0]) / 3.0, cy = (v[0][1] + v[1][1] + v[2][1]) / 3.0,
+                 cz = (v[0][2] + v[1][2] + v[2][2]) / 3.0;
+    const int m1 = min(M, ((int)blockIdx.y + 1) * per);
+    for (int m = blockIdx.y * per; m < m1; ++m) {
+        const double dx = pts[3 * m] - cx, dy = pts[3 * m + 1] - cy, dz = pts[3 * m + 2] - cz;
+        const double d2 = dx * dx + dy * dy + dz * dz;
+        if (d2 <= bound && sqrt(d2) <= reach) {
             const unsigned long long slot = atomicAdd(count, 1ull);
-            if ((long long)slot < cap) items[slot] = t;
+            if ((long long)slot < cap) items[slot] = (long long)m * F * images.n + e;
         }
     }
 }
 
-// one thread per (near pair, column group): adds adaptive - regular
+// Adds adaptive - regular for every near pair of columns [r0, r0 + RC), r0 =
+// RC blockIdx.y: a warp per pair, grid-strided over the *count listed pairs
+// (nothing is done when the list overflowed its cap).  The split's pending
+// pieces are a stack in shared memory; each round the warp takes up to 32 from
+// its top, a lane each: a leaf is integrated, another piece leaves its four
+// children.  (One thread per pair walked its pieces alone: 0.78 ms for 2,300
+// pairs, this 0.05.)
 template <int RC>
-__global__ void __launch_bounds__(FG_THREADS) near_correction_kernel(
+__global__ void __launch_bounds__(32 * FG_NEAR_WARPS) near_correction_kernel(
     const double *pts, int M, const double *verts, const int *faces, const double *normals, int F, int N,
-    FieldImages images, const long long *items, long long nitems, const double2 *p, const double2 *q, int R,
-    GradRule coarse, GradRule fine, double k, double2 *out, int *err) {
-    const long long it = blockIdx.x * (long long)FG_THREADS + threadIdx.x;
-    if (it >= nitems) return;
-    const int r0 = blockIdx.y * RC, rc = min(RC, R - r0);
-    const long long t = items[it];
-    const int f = (int)(t % F);
-    const long long rest = t / F;
-    const int ix = (int)(rest % images.n), m = (int)(rest / images.n);
-    const double *sg = images.s[ix];
-    const double x0 = pts[3 * m], x1 = pts[3 * m + 1], x2 = pts[3 * m + 2];
-    double v[3][3];
-    face_corners(verts, faces, f, sg, v);
-    const double n0 = sg[0] * normals[3 * f], n1 = sg[1] * normals[3 * f + 1], n2 = sg[2] * normals[3 * f + 2];
-    double2 pv[3][RC], qv[RC];
-#pragma unroll
-    for (int cc = 0; cc < RC; ++cc) {
-        const bool ok = cc < rc;
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-            pv[a][cc] = ok ? p[(size_t)(r0 + cc) * N + faces[3 * f + a]] : make_double2(0, 0);
-        qv[cc] = ok ? q[(size_t)(r0 + cc) * F + f] : make_double2(0, 0);
-    }
-    const double e1[3] = {v[1][0] - v[0][0], v[1][1] - v[0][1], v[1][2] - v[0][2]};
-    const double e2[3] = {v[2][0] - v[0][0], v[2][1] - v[0][1], v[2][2] - v[0][2]};
-    double acc[RC][8];  // adaptive minus regular
-#pragma unroll
-    for (int cc = 0; cc < RC; ++cc)
-#pragma unroll
-        for (int e = 0; e < 8; ++e) acc[cc][e] = 0.0;
-
-    // rule applied (scaled by sign) to the piece with corners pc, which are
-    // s[0..2] in face coordinates
-    auto integrate = [&](const double (&pc)[3][3], const double (&s)[3][2], const GradRule &rule, double sign) {
-        const double a1[3] = {pc[1][0] - pc[0][0], pc[1][1] - pc[0][1], pc[1][2] - pc[0][2]};
-        const double a2[3] = {pc[2][0] - pc[0][0], pc[2][1] - pc[0][1], pc[2][2] - pc[0][2]};
-        const double cx = a1[1] * a2[2] - a1[2] * a2[1], cy = a1[2] * a2[0] - a1[0] * a2[2],
-                     cz = a1[0] * a2[1] - a1[1] * a2[0];
-        const double jac = sqrt(cx * cx + cy * cy + cz * cz);
-        for (int j = 0; j < rule.n; ++j) {
-            const double b0 = rule.b[j][0], b1 = rule.b[j][1], b2 = rule.b[j][2];
-            const double y0 = b0 * pc[0][0] + b1 * pc[1][0] + b2 * pc[2][0];
-            const double y1 = b0 * pc[0][1] + b1 * pc[1][1] + b2 * pc[2][1];
-            const double y2 = b0 * pc[0][2] + b1 * pc[1][2] + b2 * pc[2][2];
-            // P1 basis of the face at the point
-            const double xi = b0 * s[0][0] + b1 * s[1][0] + b2 * s[2][0];
-            const double et = b0 * s[0][1] + b1 * s[1][1] + b2 * s[2][1];
-            const double l0 = 1.0 - xi - et;
-            double2 P[RC];
-#pragma unroll
-            for (int cc = 0; cc < RC; ++cc)
-                P[cc] = make_double2(l0 * pv[0][cc].x + xi * pv[1][cc].x + et * pv[2][cc].x,
-                                     l0 * pv[0][cc].y + xi * pv[1][cc].y + et * pv[2][cc].y);
-            grad_source<RC>(x0, x1, x2, y0, y1, y2, n0, n1, n2, sign * jac * rule.w[j], k, P, qv, acc);
-        }
-    };
-
-    {  // the regular rule on the whole face: what the regular sum added
-        const double s[3][2] = {{0, 0}, {1, 0}, {0, 1}};
-        integrate(v, s, coarse, -1.0);
-    }
-    // depth-first split; a piece is three corners in face coordinates
-    // (multiples of 1/4096 while depth <= 12, so exact in 16-bit integers)
+    FieldImages images, const long long *items, const unsigned long long *count, long long cap, const double2 *p,
+    const double2 *q, int R, GradRule coarse, GradRule fine, double k, double2 *out, int *err) {
+    // a piece: three corners in face coordinates, multiples of 1/4096 while
+    // depth <= 12 (so exact in 16-bit integers)
     struct Piece {
         unsigned short c[3][2];
-        unsigned char depth;
+        unsigned short depth;
     };
-    Piece stack[FG_STACK];
-    int top = 0;
-    stack[top++] = Piece{{{0, 0}, {FG_SCALE, 0}, {0, FG_SCALE}}, 0};
-    long long pieces = 0;
-    const double inv = 1.0 / FG_SCALE;
-    while (top > 0) {
-        const Piece pc = stack[--top];
-        double s[3][2], g[3][3];
+    __shared__ Piece stacks[FG_NEAR_WARPS][FG_STACK];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Piece *stack = stacks[warp];
+    const int r0 = blockIdx.y * RC, rc = min(RC, R - r0);
+    const long long nitems = (long long)*count;
+    if (nitems > cap) return;
+    for (long long it = (long long)blockIdx.x * FG_NEAR_WARPS + warp; it < nitems;
+         it += (long long)gridDim.x * FG_NEAR_WARPS) {
+        const long long t = items[it];
+        const int f = (int)(t % F);
+        const long long rest = t / F;
+        const int ix = (int)(rest % images.n), m = (int)(rest / images.n);
+        const double *sg = images.s[ix];
+        const double x0 = pts[3 * m], x1 = pts[3 * m + 1], x2 = pts[3 * m + 2];
+        double v[3][3];
+        face_corners(verts, faces, f, sg, v);
+        const double n0 = sg[0] * normals[3 * f], n1 = sg[1] * normals[3 * f + 1], n2 = sg[2] * normals[3 * f + 2];
+        double2 pv[3][RC], qv[RC];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            s[a][0] = pc.c[a][0] * inv;
-            s[a][1] = pc.c[a][1] * inv;
+        for (int cc = 0; cc < RC; ++cc) {
+            const bool ok = cc < rc;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) g[a][d] = v[0][d] + s[a][0] * e1[d] + s[a][1] * e2[d];
+            for (int a = 0; a < 3; ++a)
+                pv[a][cc] = ok ? p[(size_t)(r0 + cc) * N + faces[3 * f + a]] : make_double2(0, 0);
+            qv[cc] = ok ? q[(size_t)(r0 + cc) * F + f] : make_double2(0, 0);
         }
-        const double diam = tri_diameter(g);
-        if (diam <= 0.4 * dist_to_centroid(g, x0, x1, x2) && fabs(k) * diam <= 0.7) {
-            integrate(g, s, fine, 1.0);
-            continue;
-        }
-        if (pc.depth >= FG_MAX_DEPTH) {
-            atomicOr(err, FG_ERR_TOO_CLOSE);
-            return;
-        }
-        if (++pieces > FG_PIECE_BUDGET) {
-            atomicOr(err, FG_ERR_BUDGET);
-            return;
-        }
-        unsigned short mid[3][2];  // ab, bc, ca
+        const double e1[3] = {v[1][0] - v[0][0], v[1][1] - v[0][1], v[1][2] - v[0][2]};
+        const double e2[3] = {v[2][0] - v[0][0], v[2][1] - v[0][1], v[2][2] - v[0][2]};
+        double acc[RC][8];  // adaptive minus regular, this lane's part
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
+        for (int cc = 0; cc < RC; ++cc)
 #pragma unroll
-            for (int d = 0; d < 2; ++d)
-                mid[a][d] = (unsigned short)((pc.c[a][d] + pc.c[(a + 1) % 3][d]) / 2);
-        const unsigned char dd = pc.depth + 1;
-        // children (a, ab, ca), (ab, b, bc), (ca, bc, c), (ab, bc, ca)
-        stack[top++] = Piece{{{mid[0][0], mid[0][1]}, {mid[1][0], mid[1][1]}, {mid[2][0], mid[2][1]}}, dd};
-        stack[top++] = Piece{{{mid[2][0], mid[2][1]}, {mid[1][0], mid[1][1]}, {pc.c[2][0], pc.c[2][1]}}, dd};
-        stack[top++] = Piece{{{mid[0][0], mid[0][1]}, {pc.c[1][0], pc.c[1][1]}, {mid[1][0], mid[1][1]}}, dd};
-        stack[top++] = Piece{{{pc.c[0][0], pc.c[0][1]}, {mid[0][0], mid[0][1]}, {mid[2][0], mid[2][1]}}, dd};
+            for (int e = 0; e < 8; ++e) acc[cc][e] = 0.0;
+
+        // points [j0, j1) of the rule (scaled by sign) on the piece with
+        // corners pc, which are s[0..2] in face coordinates
+        auto integrate = [&](const double (&pc)[3][3], const double (&s)[3][2], const GradRule &rule, double sign,
+                             int j0, int j1) {
+            const double a1[3] = {pc[1][0] - pc[0][0], pc[1][1] - pc[0][1], pc[1][2] - pc[0][2]};
+            const double a2[3] = {pc[2][0] - pc[0][0], pc[2][1] - pc[0][1], pc[2][2] - pc[0][2]};
+            const double cx = a1[1] * a2[2] - a1[2] * a2[1], cy = a1[2] * a2[0] - a1[0] * a2[2],
+                         cz = a1[0] * a2[1] - a1[1] * a2[0];
+            const double jac = sqrt(cx * cx + cy * cy + cz * cz);
+            for (int j = j0; j < j1; ++j) {
+                const double b0 = rule.b[j][0], b1 = rule.b[j][1], b2 = rule.b[j][2];
+                const double y0 = b0 * pc[0][0] + b1 * pc[1][0] + b2 * pc[2][0];
+                const double y1 = b0 * pc[0][1] + b1 * pc[1][1] + b2 * pc[2][1];
+                const double y2 = b0 * pc[0][2] + b1 * pc[1][2] + b2 * pc[2][2];
+                // P1 basis of the face at the point
+                const double xi = b0 * s[0][0] + b1 * s[1][0] + b2 * s[2][0];
+                const double et = b0 * s[0][1] + b1 * s[1][1] + b2 * s[2][1];
+                const double l0 = 1.0 - xi - et;
+                double2 P[RC];
+#pragma unroll
+                for (int cc = 0; cc < RC; ++cc)
+                    P[cc] = make_double2(l0 * pv[0][cc].x + xi * pv[1][cc].x + et * pv[2][cc].x,
+                                         l0 * pv[0][cc].y + xi * pv[1][cc].y + et * pv[2][cc].y);
+                grad_source<RC>(x0, x1, x2, y0, y1, y2, n0, n1, n2, sign * jac * rule.w[j], k, P, qv, acc);
+            }
+        };
+
+        if (lane < coarse.n) {  // the regular rule on the whole face, a point per lane: what the regular sum added
+            const double s[3][2] = {{0, 0}, {1, 0}, {0, 1}};
+            integrate(v, s, coarse, -1.0, lane, lane + 1);
+        }
+        __syncwarp();
+        if (lane == 0) stack[0] = Piece{{{0, 0}, {FG_SCALE, 0}, {0, FG_SCALE}}, 0};
+        int top = 1;
+        long long pieces = 0;
+        const double inv = 1.0 / FG_SCALE;
+        bool failed = false;
+        while (top > 0) {
+            __syncwarp();
+            const int take = min(top, 32);
+            top -= take;
+            Piece pc;
+            bool split = false;
+            if (lane < take) {
+                pc = stack[top + lane];
+                double s[3][2], g[3][3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    s[a][0] = pc.c[a][0] * inv;
+                    s[a][1] = pc.c[a][1] * inv;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) g[a][d] = v[0][d] + s[a][0] * e1[d] + s[a][1] * e2[d];
+                }
+                const double diam = tri_diameter(g);
+                split = !(diam <= 0.4 * dist_to_centroid(g, x0, x1, x2) && fabs(k) * diam <= 0.7);
+                if (!split) integrate(g, s, fine, 1.0, 0, fine.n);
+            }
+            const unsigned mask = __ballot_sync(0xffffffffu, split);
+            if (__ballot_sync(0xffffffffu, split && pc.depth >= FG_MAX_DEPTH)) {
+                if (lane == 0) atomicOr(err, FG_ERR_TOO_CLOSE);
+                failed = true;
+                break;
+            }
+            pieces += __popc(mask);
+            if (pieces > FG_PIECE_BUDGET) {
+                if (lane == 0) atomicOr(err, FG_ERR_BUDGET);
+                failed = true;
+                break;
+            }
+            __syncwarp();  // the popped pieces are read: their places may be written
+            if (split) {
+                unsigned short mid[3][2];  // ab, bc, ca
+#pragma unroll
+                for (int a = 0; a < 3; ++a)
+#pragma unroll
+                    for (int d = 0; d < 2; ++d)
+                        mid[a][d] = (unsigned short)((pc.c[a][d] + pc.c[(a + 1) % 3][d]) / 2);
+                const unsigned short dd = pc.depth + 1;
+                Piece *to = stack + top + 4 * __popc(mask & ((1u << lane) - 1u));
+                // children (a, ab, ca), (ab, b, bc), (ca, bc, c), (ab, bc, ca)
+                to[0] = Piece{{{mid[0][0], mid[0][1]}, {mid[1][0], mid[1][1]}, {mid[2][0], mid[2][1]}}, dd};
+                to[1] = Piece{{{mid[2][0], mid[2][1]}, {mid[1][0], mid[1][1]}, {pc.c[2][0], pc.c[2][1]}}, dd};
+                to[2] = Piece{{{mid[0][0], mid[0][1]}, {pc.c[1][0], pc.c[1][1]}, {mid[1][0], mid[1][1]}}, dd};
+                to[3] = Piece{{{pc.c[0][0], pc.c[0][1]}, {mid[0][0], mid[0][1]}, {mid[2][0], mid[2][1]}}, dd};
+            }
+            top += 4 * __popc(mask);
+        }
+        if (failed) continue;
+#pragma unroll
+        for (int cc = 0; cc < RC; ++cc)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                double a = acc[cc][e];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+                if (lane == 0 && cc < rc)
+                    atomicAdd(reinterpret_cast<double *>(
+                                  &out[(size_t)m + (size_t)M * (e / 2 + 4 * (size_t)(r0 + cc))]) +
+                                  (e & 1),
+                              a);
+            }
     }
-    for (int cc = 0; cc < rc; ++cc)
-#pragma unroll
-        for (int d = 0; d < 4; ++d) {
-            double2 *o = &out[(size_t)m + (size_t)M * (d + 4 * (size_t)(r0 + cc))];
-            atomicAdd(&o->x, acc[cc][2 * d]);
-            atomicAdd(&o->y, acc[cc][2 * d + 1]);
-        }
 }
 
 static GradRule grad_rule(const std::vector<double> &pts, const std::vector<double> &w) {
@@ -730,24 +764,21 @@ void field_gradient(beat_b200_ctx *c, double k, int M, const double *pts_host, i
     const StagedSources st = stage_sources(c, M, pts_host, R, p_dev, q_dev);
     double2 *out = reinterpret_cast<double2 *>(out_dev);
     BB_CUDA(cudaMemsetAsync(out, 0, sizeof(double2) * 4 * (size_t)M * R, c->stream));
-    {
-        const auto [grid, per] = source_split(c, M, st.S, FG_THREADS, FG_CHUNK);
-        for (int r0 = 0; r0 < R; r0 += FG_RC) {
-            if (R == 1)
-                field_grad_kernel<1><<<grid, FG_THREADS, 0, c->stream>>>(st.pts, M, st.ys, st.ns, st.ps, st.qs, st.S,
-                                                                         R, r0, per, k, out);
-            else
-                field_grad_kernel<FG_RC><<<grid, FG_THREADS, 0, c->stream>>>(st.pts, M, st.ys, st.ns, st.ps, st.qs,
-                                                                             st.S, R, r0, per, k, out);
-            BB_CUDA(cudaGetLastError());
-        }
-    }
+    auto regular = [&](auto *kernel, int r0) {
+        const SourceSplit sp = resident_split(c, kernel, M, st.S);
+        kernel<<<sp.grid, FG_THREADS, 0, c->stream>>>(st.pts, M, st.ys, st.ns, st.ps, st.qs, st.S, R, r0, sp.per, k,
+                                                      out);
+        BB_CUDA(cudaGetLastError());
+    };
+    for (int r0 = 0; r0 < R; r0 += FG_RC) regular(R == 1 ? field_grad_kernel<1> : field_grad_kernel<FG_RC>, r0);
     FieldImages images;
     images.n = 1 + c->nimg;
     for (int i = 0; i < 3; ++i) images.s[0][i] = 1.0;
     for (int ix = 0; ix < c->nimg; ++ix)
         for (int i = 0; i < 3; ++i) images.s[1 + ix][i] = c->img_sign[ix][i];
-    // near pairs: count and list in one pass; a second pass if the list overflowed
+    // near pairs listed, then corrected, without a wait between: the correction
+    // reads the count on the device and does nothing when the list overflowed;
+    // then both run once more with room for every pair
     DevBuf &nb = c->ws.grad;  // [count u64][error int, pad][items i64 ...], grow-only
     const size_t head = 16;
     long long cap = nb.bytes > head ? (long long)((nb.bytes - head) / sizeof(long long)) : 0;
@@ -755,45 +786,42 @@ void field_gradient(beat_b200_ctx *c, double k, int M, const double *pts_host, i
         nb.alloc(head + 1024 * sizeof(long long));
         cap = 1024;
     }
-    const long long total = (long long)M * F * images.n;
-    const int blocks = (int)std::min<long long>((total + 255) / 256, 16LL * c->sm_count);
-    unsigned long long count = 0;
+    std::vector<double> p4, w4;
+    triangle_rule(4, p4, w4);
+    const GradRule coarse = grad_rule(c->rule_pts, c->rule_w), fine = grad_rule(p4, w4);
+    const int face_blocks = (int)(((int64_t)F * images.n + 255) / 256);
+    const int parts = std::min(M, std::max(1, 8 * c->sm_count / face_blocks)), per = (M + parts - 1) / parts;
+    struct {
+        unsigned long long count;
+        int err, pad;
+    } got{};
     for (int pass = 0; pass < 2; ++pass) {
         BB_CUDA(cudaMemsetAsync(nb.p, 0, head, c->stream));
-        near_pairs_kernel<<<blocks, 256, 0, c->stream>>>(
-            st.pts, M, c->d_verts.as<double>(), c->d_faces.as<int>(), F, images,
-            reinterpret_cast<long long *>(static_cast<char *>(nb.p) + head), cap,
-            static_cast<unsigned long long *>(nb.p));
+        unsigned long long *d_count = static_cast<unsigned long long *>(nb.p);
+        int *d_err = reinterpret_cast<int *>(static_cast<char *>(nb.p) + 8);
+        long long *items = reinterpret_cast<long long *>(static_cast<char *>(nb.p) + head);
+        near_pairs_kernel<<<dim3(face_blocks, (M + per - 1) / per), 256, 0, c->stream>>>(
+            st.pts, M, c->d_verts.as<double>(), c->d_faces.as<int>(), F, images, per, items, cap, d_count);
         BB_CUDA(cudaGetLastError());
-        BB_CUDA(cudaMemcpyAsync(&count, nb.p, sizeof(count), cudaMemcpyDeviceToHost, c->stream));
+        auto correct = [&](auto *kernel, int groups) {
+            kernel<<<dim3(4 * c->sm_count, groups), 32 * FG_NEAR_WARPS, 0, c->stream>>>(
+                st.pts, M, c->d_verts.as<double>(), c->d_faces.as<int>(), c->d_normals.as<double>(), F, N, images,
+                items, d_count, cap, reinterpret_cast<const double2 *>(p_dev), st.q, R, coarse, fine, k, out, d_err);
+            BB_CUDA(cudaGetLastError());
+        };
+        if (R == 1)
+            correct(near_correction_kernel<1>, 1);
+        else
+            correct(near_correction_kernel<FG_RC>, (R + FG_RC - 1) / FG_RC);
+        static_assert(sizeof(got) == head, "the list's head");
+        BB_CUDA(cudaMemcpyAsync(&got, nb.p, head, cudaMemcpyDeviceToHost, c->stream));
         BB_CUDA(cudaStreamSynchronize(c->stream));
-        if ((long long)count <= cap) break;
+        if ((long long)got.count <= cap) break;
         BB_REQUIRE(pass == 0, BEAT_B200_CUDA_ERROR, "field gradient: near-pair list overflowed twice");
-        cap = (long long)count;
+        cap = (long long)got.count;
         nb.alloc(head + (size_t)cap * sizeof(long long));
     }
-    int err = 0;
-    if (count > 0) {
-        std::vector<double> p4, w4;
-        triangle_rule(4, p4, w4);
-        const GradRule coarse = grad_rule(c->rule_pts, c->rule_w), fine = grad_rule(p4, w4);
-        int *d_err = reinterpret_cast<int *>(static_cast<char *>(nb.p) + 8);
-        const long long *items = reinterpret_cast<const long long *>(static_cast<char *>(nb.p) + head);
-        const unsigned nblk = (unsigned)((count + FG_THREADS - 1) / FG_THREADS);
-        if (R == 1)
-            near_correction_kernel<1><<<dim3(nblk, 1), FG_THREADS, 0, c->stream>>>(
-                st.pts, M, c->d_verts.as<double>(), c->d_faces.as<int>(), c->d_normals.as<double>(), F, N, images,
-                items, (long long)count, reinterpret_cast<const double2 *>(p_dev), st.q, R, coarse, fine, k, out,
-                d_err);
-        else
-            near_correction_kernel<FG_RC><<<dim3(nblk, (R + FG_RC - 1) / FG_RC), FG_THREADS, 0, c->stream>>>(
-                st.pts, M, c->d_verts.as<double>(), c->d_faces.as<int>(), c->d_normals.as<double>(), F, N, images,
-                items, (long long)count, reinterpret_cast<const double2 *>(p_dev), st.q, R, coarse, fine, k, out,
-                d_err);
-        BB_CUDA(cudaGetLastError());
-        BB_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    }
-    BB_CUDA(cudaStreamSynchronize(c->stream));
+    const int err = got.err;
     BB_REQUIRE(!(err & FG_ERR_TOO_CLOSE), BEAT_B200_INVALID_ARG,
                "field gradient: a point is too close to the boundary for reliable evaluation");
     BB_REQUIRE(!(err & FG_ERR_BUDGET), BEAT_B200_INVALID_ARG,
