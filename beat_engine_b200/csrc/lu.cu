@@ -799,112 +799,165 @@ __global__ void __launch_bounds__(256, 2) gemm_update_kernel(Cx<T> *A, int64_t l
 
 // ---------------------------------------------------------------------------
 // FP64 tensor-core (DMMA) complex GEMM for the FP64 form's updates:
-// C[r0.., c0..] -= L U on the same 64 x 64 complex output tiles as
-// gemm_update_kernel.  Eight warps as 2 x 4, each a 32 x 16 complex warp tile
-// of 8 x 8 blocks computed with mma.sync.m8n8k4.f64 (4 real products per
-// complex block: re += Lr Ur - Li Ui, im += Lr Ui + Li Ur).  L and U are
-// staged as separate real / imaginary planes, K in chunks of 16, with row
-// paddings that keep each fragment load to its two 128-byte wavefronts.
-// Fragments (PTX ISA, m8n8k4 .f64): A a0 at (lane / 4, lane % 4); B b0 at
-// (lane % 4, lane / 4); C c0, c1 at (lane / 4, 2 (lane % 4) + 0, 1).
+// C[r0.., c0..] -= L U, 8 x 8 complex blocks by mma.sync.m8n8k4.f64 (4 real
+// products per complex block: re -= Lr Ur - Li Ui, im -= Lr Ui + Li Ur, the
+// signs on the L fragments).  Fragments (PTX ISA, m8n8k4 .f64): A a0 at
+// (lane / 4, lane % 4); B b0 at (lane % 4, lane / 4); C c0, c1 at (lane / 4,
+// 2 (lane % 4) + 0, 1).
+//
+// The accumulators start as C, loaded while the first chunks of L and U are on
+// their way; K goes in chunks of 8 through a ring of DU_ST cp.async stages, one
+// barrier per chunk.  Complex entries stay interleaved (a fragment's real and
+// imaginary part are one 16-byte load); row strides of 4 mod 8 (L) and 2 mod 8
+// (U) entries keep a quarter-warp's loads on distinct banks.
+//
+// Two shapes of four warps: 64 x 64 tiles (32 x 32 complex per warp, 128
+// registers of sums, two CTAs per SM: one's barriers and ends lie beside the
+// other's products; one CTA of 128 x 64 measured 27.1 TFLOP/s, chunks of 16
+// 28.4), and 64 x 32 (16 x 32 per warp) where the larger would leave the last
+// wave of SMs mostly idle (launch_update).
+// Bound: the FP64 tensor cores (37 TFLOP/s measured with mma.sync alone).  64 x
+// 64 tiles staged through registers, two barriers per 16 columns and C read at
+// the end reached 22 TFLOP/s on the largest updates, these 29.7.
 // ---------------------------------------------------------------------------
-constexpr int DM_KC = 16, DM_LP = DM_KC + 4, DM_UP = GT + 4;
+constexpr int DU_K = 8, DU_ST = 4;
 
 __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(c[0]), "+d"(c[1])
-                 : "d"(a), "d"(b));
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+// 16 bytes, global -> shared, asynchronously; zeros when `in` is false
+__device__ __forceinline__ void cp_async16_zfill(double2 *smem, const double2 *gmem, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
+                 "l"(gmem), "r"(in ? 16 : 0)
+                 : "memory");
 }
 
-// Persistent over the output tiles (tiles_x per row of tiles, ntiles in all):
-// CTA b takes tiles b, b + gridDim.x, ... so a capped grid leaves SMs free
-// for the kernels running beside it (the LU's panel on the other stream).
-__global__ void __launch_bounds__(256, 2) dmma_update_kernel(Cx<double> *A, int64_t ld, int n, int k, int kk,
-                                                            int row0, int col0, int col_end, int tiles_x,
-                                                            int ntiles) {
-    __shared__ double sLr[GT][DM_LP], sLi[GT][DM_LP];  // L chunk: 64 rows x 16
-    __shared__ double sUr[DM_KC][DM_UP], sUi[DM_KC][DM_UP];  // U chunk: 16 x 64 columns
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wr = warp >> 2, wc = warp & 3;  // warp tile: rows 32 wr .., columns 16 wc ..
-    const int g = lane >> 2, t = lane & 3;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int r0 = row0 + (tile / tiles_x) * GT, c0 = col0 + (tile % tiles_x) * GT;
-    double cr[4][2][2], ci[4][2][2];  // [row block][column block][fragment]
+template <int BM, int BN, int WM, int WN> struct DmmaTile {
+    static constexpr int THREADS = 32 * (BM / WM) * (BN / WN);
+    static constexpr int LDA = DU_K + 4, LDB = BN + 2;  // complex entries
+    static constexpr int STAGE = BM * LDA + DU_K * LDB;
+    static constexpr size_t SMEM = sizeof(double2) * DU_ST * STAGE;
+};
+template <int BM, int BN, int WM, int WN>
+__global__ void __launch_bounds__(DmmaTile<BM, BN, WM, WN>::THREADS, BN == 64 ? 2 : 3)
+    dmma_update_kernel(Cx<double> *A_, int64_t ld, int n, int k, int kk, int row0, int col0, int col_end) {
+    using DT = DmmaTile<BM, BN, WM, WN>;
+    constexpr int THREADS = DT::THREADS, LDA = DT::LDA, LDB = DT::LDB, MI = WM / 8, NJ = WN / 8;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2 *ring = reinterpret_cast<double2 *>(smem_raw);
+    double2 *A = reinterpret_cast<double2 *>(A_);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int r0 = row0 + blockIdx.y * BM, c0 = col0 + blockIdx.x * BN;
+    const int wr = (warp / (BN / WN)) * WM, wc = (warp % (BN / WN)) * WN;
+    const int nk = (kk + DU_K - 1) / DU_K;
+    auto load = [&](int kt) {  // chunk kt of L (BM x DU_K) and U (DU_K x BN)
+        if (kt < nk) {
+            double2 *sl = ring + (kt % DU_ST) * DT::STAGE, *su = sl + BM * LDA;
+            const int kc = kt * DU_K;
+            static_assert(BM * DU_K % THREADS == 0 && BN * DU_K % THREADS == 0, "whole rounds of copies");
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) cr[i][j][0] = cr[i][j][1] = ci[i][j][0] = ci[i][j][1] = 0.0;
-    for (int kc = 0; kc < kk; kc += DM_KC) {
-        // stage the chunk: 64 x 16 of L and 16 x 64 of U, four complex entries each per thread
-#pragma unroll
-        for (int u = 0; u < GT * DM_KC / 256; ++u) {
-            const int idx = tid + u * 256;
-            const int i = idx / DM_KC, q = idx % DM_KC, r = r0 + i, kq = kc + q;
-            const Cx<double> vl = (r < n && kq < kk) ? A[(int64_t)r * ld + k + kq] : Cx<double>{0.0, 0.0};
-            sLr[i][q] = vl.re;
-            sLi[i][q] = vl.im;
-            const int q2 = idx / GT, j = idx % GT, c = c0 + j, kq2 = kc + q2;
-            const Cx<double> vu = (c < col_end && kq2 < kk) ? A[(int64_t)(k + kq2) * ld + c] : Cx<double>{0.0, 0.0};
-            sUr[q2][j] = vu.re;
-            sUi[q2][j] = vu.im;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k4 = 0; k4 < DM_KC; k4 += 4) {
-            double ar[4], ai[4], nai[4], br[2], bi[2];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                ar[i] = sLr[32 * wr + 8 * i + g][k4 + t];
-                ai[i] = sLi[32 * wr + 8 * i + g][k4 + t];
-                nai[i] = -ai[i];
+            for (int u = 0; u < BM * DU_K / THREADS; ++u) {
+                const int i = (tid + u * THREADS) / DU_K, q = tid % DU_K;
+                const bool in = r0 + i < n && kc + q < kk;
+                cp_async16_zfill(&sl[i * LDA + q], in ? &A[(int64_t)(r0 + i) * ld + k + kc + q] : A, in);
             }
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                br[j] = sUr[k4 + t][16 * wc + 8 * j + g];
-                bi[j] = sUi[k4 + t][16 * wc + 8 * j + g];
+            for (int u = 0; u < BN * DU_K / THREADS; ++u) {
+                const int q = (tid + u * THREADS) / BN, j = tid % BN;
+                const bool in = c0 + j < col_end && kc + q < kk;
+                cp_async16_zfill(&su[q * LDB + j], in ? &A[(int64_t)(k + kc + q) * ld + c0 + j] : A, in);
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    dmma884(cr[i][j], ar[i], br[j]);
-                    dmma884(cr[i][j], nai[i], bi[j]);
-                    dmma884(ci[i][j], ar[i], bi[j]);
-                    dmma884(ci[i][j], ai[i], br[j]);
-                }
         }
-        __syncthreads();
-    }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int s = 0; s < DU_ST - 1; ++s) load(s);
+    double cr[MI][NJ][2], ci[MI][NJ][2];  // [row block][column block][fragment]
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const int r = r0 + 32 * wr + 8 * i + g, c = c0 + 16 * wc + 8 * j + 2 * t + e;
-                if (r < n && c < col_end) {
-                    Cx<double> &d = A[(int64_t)r * ld + c];
-                    d.re -= cr[i][j][e];
-                    d.im -= ci[i][j][e];
+                const int r = r0 + wr + 8 * i + g, c = c0 + wc + 8 * j + 2 * t + e;
+                const double2 v = (r < n && c < col_end) ? A[(int64_t)r * ld + c] : make_double2(0.0, 0.0);
+                cr[i][j][e] = v.x;
+                ci[i][j][e] = v.y;
+            }
+    for (int kt = 0; kt < nk; ++kt) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(DU_ST - 2) : "memory");
+        __syncthreads();  // chunk kt is in; every warp is done with chunk kt - 1, whose place the next load takes
+        load(kt + DU_ST - 1);
+        const double2 *sl = ring + (kt % DU_ST) * DT::STAGE, *su = sl + BM * LDA;
+#pragma unroll
+        for (int k4 = 0; k4 < DU_K; k4 += 4) {
+            double2 a[MI], b[NJ];
+#pragma unroll
+            for (int i = 0; i < MI; ++i) a[i] = sl[(wr + 8 * i + g) * LDA + k4 + t];
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) b[j] = su[(k4 + t) * LDB + wc + 8 * j + g];
+#pragma unroll
+            for (int i = 0; i < MI; ++i) {
+                const double nr = -a[i].x, ni = -a[i].y;
+                // (2 NJ products between the two that add to one block)
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) {
+                    dmma884(cr[i][j], nr, b[j].x);
+                    dmma884(ci[i][j], nr, b[j].y);
+                }
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) {
+                    dmma884(cr[i][j], a[i].y, b[j].y);
+                    dmma884(ci[i][j], ni, b[j].x);
                 }
             }
+        }
     }
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = r0 + wr + 8 * i + g, c = c0 + wc + 8 * j + 2 * t + e;
+                if (r < n && c < col_end) A[(int64_t)r * ld + c] = make_double2(cr[i][j][e], ci[i][j][e]);
+            }
 }
 
-// the trailing / in-panel update C -= L U over rows row0.. and columns
-// [col0, col_end): tensor cores (DMMA) in FP64, SIMT in FP32.  max_ctas
-// (0: no cap) bounds the persistent DMMA grid.
+// the trailing / in-panel update C -= L U, L = A[row0.., k..k+kk), U = A[k..k+kk,
+// col0..col_end): tensor cores (DMMA) in FP64, SIMT in FP32
 template <typename T>
-static void launch_update(cudaStream_t st, dim3 grid, Cx<T> *A, int64_t ld, int n, int k, int kk, int row0, int col0,
-                          int col_end, int max_ctas = 0) {
+static void launch_update(beat_b200_ctx *c, cudaStream_t st, Cx<T> *A, int64_t ld, int n, int k, int kk, int row0,
+                          int col0, int col_end) {
+    const int rows = n - row0, cols = col_end - col0;
+    if (rows <= 0 || cols <= 0) return;
     if constexpr (sizeof(T) == 8) {
-        const int ntiles = (int)(grid.x * grid.y);
-        const int g = max_ctas > 0 ? std::min(ntiles, max_ctas) : ntiles;
-        if (g > 0)
-            dmma_update_kernel<<<g, 256, 0, st>>>(A, ld, n, k, kk, row0, col0, col_end, (int)grid.x, ntiles);
+        auto launch = [&](auto *kernel, int bm, int bn, int threads, size_t smem) {
+            kernel<<<dim3((cols + bn - 1) / bn, (rows + bm - 1) / bm), threads, smem, st>>>(A, ld, n, k, kk, row0,
+                                                                                            col0, col_end);
+        };
+        // the large tile while there are eight waves of it, so that an uneven
+        // last wave costs little; below, tiles of half the size even out the
+        // SMs (at 2,500 x 2,500 both reach 27 TFLOP/s)
+        using Big = DmmaTile<64, 64, 32, 32>;
+        using Small = DmmaTile<64, 32, 16, 32>;
+        if ((int64_t)((cols + 63) / 64) * ((rows + 63) / 64) >= 16 * c->sm_count)
+            launch(dmma_update_kernel<64, 64, 32, 32>, 64, 64, Big::THREADS, Big::SMEM);
+        else
+            launch(dmma_update_kernel<64, 32, 16, 32>, 64, 32, Small::THREADS, Small::SMEM);
     } else {
-        gemm_update_kernel<T><<<grid, 256, 0, st>>>(A, ld, n, k, kk, row0, col0, col_end);
+        gemm_update_kernel<T><<<dim3((cols + GT - 1) / GT, (rows + GT - 1) / GT), 256, 0, st>>>(A, ld, n, k, kk, row0,
+                                                                                               col0, col_end);
     }
+    BB_CUDA(cudaGetLastError());
+}
+static void update_setup() {
+    BB_CUDA(cudaFuncSetAttribute(dmma_update_kernel<64, 64, 32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)DmmaTile<64, 64, 32, 32>::SMEM));
+    BB_CUDA(cudaFuncSetAttribute(dmma_update_kernel<64, 32, 16, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)DmmaTile<64, 32, 16, 32>::SMEM));
 }
 
 // ---------------------------------------------------------------------------
@@ -1770,6 +1823,7 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
     if (wide)
         BB_CUDA(cudaFuncSetAttribute(trsm_narrow_kernel<T, WF, NCS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)trsm_narrow_smem<T, WF, NCS>(nb / W)));
+    if (sizeof(T) == 8) update_setup();
     c->barrier.alloc(sizeof(unsigned) * 4096);
     BB_CUDA(cudaFuncSetAttribute(panel_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
     // the unblocked U12 solve (used only when the blocked one does not apply)
@@ -1827,9 +1881,7 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
         } else {
             // one CTA per tile: capping this grid as the tensor-core one is capped
             // measured slower at N = 10,242 (154 against 136 ms for the FP64 LU)
-            dim3 grid((c_hi - c_lo + GT - 1) / GT, (n - k - nb + GT - 1) / GT);
-            launch_update<T>(st, grid, A, ld, n, k, nb, k + nb, c_lo, c_hi, 0);
-            BB_CUDA(cudaGetLastError());
+            launch_update<T>(c, st, A, ld, n, k, nb, k + nb, c_lo, c_hi);
         }
     };
     // Right-looking LU with a look-ahead of one panel.  For panel k (columns
@@ -1911,8 +1963,7 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
                     dim3 grid((cols + PU_COLS - 1) / PU_COLS, (n - ks - W + PU_ROWS - 1) / PU_ROWS);
                     panel_update_kernel<<<grid, 256, 0, s0>>>(A, ld, n, ks, W, ks + W, ks + W, pe);
                 } else {
-                    dim3 grid((cols + GT - 1) / GT, (n - ks - W + GT - 1) / GT);
-                    launch_update<T>(s0, grid, A, ld, n, ks, W, ks + W, ks + W, pe);
+                    launch_update<T>(c, s0, A, ld, n, ks, W, ks + W, ks + W, pe);
                 }
                 BB_CUDA(cudaGetLastError());
             }
