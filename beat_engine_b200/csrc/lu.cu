@@ -1038,9 +1038,8 @@ __global__ void __launch_bounds__(256, 2) panel_update_kernel(Cx<float> *A, int6
 // columns, 64 registers each), as pairs of columns with the real and the
 // imaginary parts packed (one FP32 instruction then updates both columns), so
 // eliminating a column touches shared memory only for the broadcast pivot row.
-// Rows past RPT per thread (EXTRA) stay in shared memory.  Rows never move:
-// each carries its logical position, and an interchange only swaps two
-// positions.
+// Rows never move: each carries its logical position, and an interchange only
+// swaps two positions.
 //
 // The loop over columns advances two at a time: the even column is the first
 // half of the thread's first pair, the odd one the second half, and the odd
@@ -1076,7 +1075,8 @@ __global__ void __launch_bounds__(256, 2) panel_update_kernel(Cx<float> *A, int6
 // on the chain than the candidate's own row.  Measured on a B200, the whole
 // factorisation, against rows kept in shared memory by 512 threads of 16 CTAs
 // whatever their number: FP32 N = 162 0.60 -> 0.41 ms, N = 1,390 4.17 -> 2.65,
-// N = 10,242 38.1 -> 32.2; FP64 N = 998 3.04 -> 2.83.
+// N = 10,242 38.1 -> 31.0 (three rows per thread past 8,192: 81 us a sub-panel,
+// 91 with the third row in shared memory); FP64 N = 998 3.04 -> 2.83.
 // ---------------------------------------------------------------------------
 constexpr int CP_CTAS = 16, CP_THREADS = 256, CP_WARPS = CP_THREADS / 32, CP_ROW_BYTES = 272, CP_SLOTS = 3;
 // rows up to which one CTA alone factors the sub-panel: at one row per thread
@@ -1265,14 +1265,14 @@ template <typename T> struct CpShape {
     // The interchange of the panel's other columns: at most 2 W moved rows, MVC
     // 16-byte chunks (or fewer) each, MVT values per thread of 128 or more
     static constexpr int MVC = sizeof(T) == 4 ? 64 : 128, MVT = 2 * W * MVC / 128;
-    // shared memory for rpc rows on C CTAs, `extra` of them not in registers
-    static size_t smem(int rpc, int C, int extra) {
+    // shared memory for rpc rows on C CTAs
+    static size_t smem(int rpc, int C) {
         return (size_t)rpc * CP_ROW_BYTES + (size_t)(RSL + KB) * (CP_SLOTS * C + 2) +
-               sizeof(Cx<T>) * 2 * W * (W + 1) + sizeof(int) * (size_t)extra;
+               sizeof(Cx<T>) * 2 * W * (W + 1);
     }
 };
 
-template <typename T, int RPT, bool EXTRA>
+template <typename T, int RPT>
 __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPanelArgs<T> a) {
     using S = CpShape<T>;
     using M = decltype(mag_bits(T(0)));
@@ -1288,7 +1288,6 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
     Cx<T> *l11 = reinterpret_cast<Cx<T> *>(stage_key + 2 * KB);    // W x (W + 1): L11 (rank 0)
     Cx<T> *y11 = l11 + W * (W + 1);                                // W x (W + 1): its inverse
     unsigned char *P = reinterpret_cast<unsigned char *>(y11 + W * (W + 1));  // rpc rows of CP_ROW_BYTES, complex
-    int *xpos = reinterpret_cast<int *>(P + (size_t)a.rpc * CP_ROW_BYTES);    // EXTRA: positions of those rows
     struct alignas(16) Key {  // a warp's best row
         M m;
         int pos, li;
@@ -1328,9 +1327,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
                 break;
             }
     }
-    // logical positions of this thread's register rows (local rows tid + r NT;
-    // -1: none) and, in xpos, of the shared-memory rows (local rows x0 + i)
-    const int x0 = RPT * NT, nx = EXTRA ? max(0, nrows - x0) : 0;
+    // logical positions of this thread's rows (local rows tid + r NT; -1: none)
     int mp[RPT];
     ColPair<T> A[RPT][NPM];
 #pragma unroll
@@ -1343,8 +1340,6 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
             A[r][q] = mp[r] >= 0 ? pair_make(row_at(i)[2 * q], row_at(i)[2 * q + 1]) : pair_make(z, z);
         }
     }
-    if (EXTRA)
-        for (int i = tid; i < nx; i += NT) xpos[i] = gr0 + x0 + i;  // read and swapped by the same thread
 
     // a thread's best row: magnitude, position, local row, the entry itself and
     // the multiplier that finishes the row
@@ -1384,10 +1379,6 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
         unsigned char *buf = stage + pb * RSL;
         if (warp == bw && cand.pos != CP_NONE) {
             if (lane == wl) {
-                if (EXTRA && cand.li >= x0) {
-                    const Cx<T> *row = row_at(cand.li);
-                    for (int q = base; q < NPM; ++q) pair_st(buf + q * PB, pair_make(row[2 * q], row[2 * q + 1]));
-                }
 #pragma unroll
                 for (int r = 0; r < RPT; ++r)
                     if (cand.li == tid + r * NT) {
@@ -1500,21 +1491,6 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
             if (act && more) best.offer(y, l[r], mp[r], tid + r * NT);
             if (act) row_at(tid + r * NT)[j] = l[r];  // read by the push of the candidate that holds it
         }
-        if (EXTRA)
-            for (int i = tid; i < nx; i += NT) {
-                int xp = xpos[i];
-                if (xp == p || xp == jr) xpos[i] = xp = xp == p ? jr : p;
-                if (xp > jr) {
-                    Cx<T> *row = row_at(x0 + i);
-                    const Cx<T> l1 = cmul(row[j], inv);
-                    row[j] = l1;
-                    if (more) {
-                        const Cx<T> y1 = cms(row[j + 1], l1, un);
-                        if (!ODD) row[j + 1] = y1;
-                        best.offer(y1, l1, xp, x0 + i);
-                    }
-                }
-            }
         const int nslot = par == CP_SLOTS - 1 ? 0 : par + 1;
         if (more && !publish(oddc, npc, j + 1, nslot, best, prow)) {
             stop = true;
@@ -1543,18 +1519,6 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
 #pragma unroll
             for (int r = 0; r < RPT; ++r) A[r][i - ODD] = pair_cms(A[r][i], lm[r], u);
         }
-        if (EXTRA)
-            for (int i = tid; i < nx; i += NT) {
-                if (xpos[i] <= jr) continue;
-                Cx<T> *row = row_at(x0 + i);
-                const Cx<T> l1 = row[j];
-#pragma unroll 4
-                for (int q = (j >> 1) + 1; q < NPM; ++q) {
-                    const ColPair<T> u = pair_ld(prow + q * PB, T(0));
-                    row[2 * q] = cms(row[2 * q], l1, pair_get<0>(u));
-                    row[2 * q + 1] = cms(row[2 * q + 1], l1, pair_get<1>(u));
-                }
-            }
         // the pivot's index; L11's row j (complex entries in the pairs before
         // j / 2, then the first half of pair j / 2)
         if (rank == 0 && warp == NW - 1) {
@@ -1581,8 +1545,6 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
 #pragma unroll
         for (int r = 0; r < RPT; ++r)
             if (mp[r] >= 0) best.offer(pair_get<0>(A[r][0]), z, mp[r], tid + r * NT);
-        if (EXTRA)
-            for (int i = tid; i < nx; i += NT) best.offer(row_at(x0 + i)[0], z, xpos[i], x0 + i);
         if (C > 1) cl_sync();  // every CTA's mbarriers are initialised before any remote store
         publish(std::integral_constant<int, 0>{}, std::integral_constant<int, NPM>{}, 0, 0, best, nullptr);
     }
@@ -1605,9 +1567,6 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
 #pragma unroll
         for (int r = 0; r < RPT; ++r)
             if (mp[r] >= a.k && mp[r] < a.n) fn(tid + r * NT, mp[r]);
-        if (EXTRA)
-            for (int i = tid; i < nx; i += NT)
-                if (xpos[i] >= a.k && xpos[i] < a.n) fn(x0 + i, xpos[i]);
     };
     each_row([&](int i, int pos) { bulk_s2g(a.A + (int64_t)pos * a.ld + a.k, sm_addr(row_at(i)), 256u); });
     // the same interchanges on the panel's other columns: every CTA reads its
@@ -1709,17 +1668,15 @@ static bool cluster_panel(beat_b200_ctx *c, Cx<T> *A, int64_t ld, int n, int k, 
     const int C = m <= CP_ONE_CTA ? 1 : CP_CTAS;
     const int rpc = (m + C - 1) / C;
     // one row per thread on four warps (one per scheduler), then two, then two
-    // on eight warps, then the remaining rows in shared memory
+    // or three on eight warps
     const int threads = rpc <= CP_THREADS ? CP_THREADS / 2 : CP_THREADS;
-    const int rpt = rpc <= threads ? 1 : 2;
-    const int extra = std::max(0, rpc - rpt * threads);
-    constexpr size_t cap = 220 * 1024;
-    if (w != S::W || n >= (1 << 30)) return false;
-    const size_t smem = S::smem(rpc, C, extra);
+    const int rpt = (rpc + threads - 1) / threads;
+    constexpr size_t cap = 226 * 1024;
+    if (w != S::W || n >= (1 << 30) || rpt > 3) return false;
+    const size_t smem = S::smem(rpc, C);
     if (smem > cap) return false;
     using Kernel = void (*)(ClusterPanelArgs<T>);
-    const Kernel kernels[3] = {cluster_panel_kernel<T, 1, false>, cluster_panel_kernel<T, 2, false>,
-                               cluster_panel_kernel<T, 2, true>};
+    const Kernel kernels[3] = {cluster_panel_kernel<T, 1>, cluster_panel_kernel<T, 2>, cluster_panel_kernel<T, 3>};
     static std::atomic<bool> attr_done{false};  // sweep lanes call this from several threads
     if (!attr_done) {
         for (Kernel f : kernels) {
@@ -1764,7 +1721,7 @@ static bool cluster_panel(beat_b200_ctx *c, Cx<T> *A, int64_t ld, int n, int k, 
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     attr[0].val.clusterDim.x = C;
-    BB_CUDA(cudaLaunchKernelEx(&cfg, kernels[extra > 0 ? 2 : rpt - 1], a));
+    BB_CUDA(cudaLaunchKernelEx(&cfg, kernels[rpt - 1], a));
     return true;
 }
 
