@@ -1053,11 +1053,12 @@ __global__ void __launch_bounds__(256, 2) panel_update_kernel(Cx<float> *A, int6
 //   2. the multiplier and column j + 1 of each row; each warp's best row's key
 //      to shared memory; a CTA barrier; every warp picks the CTA's best;
 //   3. the best row's thread writes the row as it stands before this step to
-//      the staging buffer, and its warp's lanes finish it there, a pair each;
-//      a second CTA barrier; the warps push it to every CTA (16 bytes per
-//      lane, st.async, complete_tx on the receiver's mbarrier).  With C = 1 the
-//      staging buffer is what every thread reads next: no exchange;
-//   4. every thread eliminates the rest of step j while the pushes fly.
+//      the staging buffer; its warp's lanes finish it, 16 bytes each, and push
+//      it with its key to every CTA (st.async, complete_tx on the receiver's
+//      mbarrier).  With C = 1 they leave it in the staging buffer, which every
+//      thread reads next after a second CTA barrier: no exchange;
+//   4. every thread eliminates the rest of step j, the other warps at once, the
+//      pushing warp afterwards.
 // Multipliers and retired pivot rows go to a shared-memory copy of the
 // sub-panel, which the bulk-copy engine loaded and stores at the end; rank 0
 // keeps the pivot rows' multipliers (L11) and inverts them during that store.
@@ -1075,8 +1076,7 @@ __global__ void __launch_bounds__(256, 2) panel_update_kernel(Cx<float> *A, int6
 // on the chain than the candidate's own row.  Measured on a B200, the whole
 // factorisation, against rows kept in shared memory by 512 threads of 16 CTAs
 // whatever their number: FP32 N = 162 0.60 -> 0.41 ms, N = 1,390 4.17 -> 2.65,
-// N = 10,242 38.1 -> 31.0 (three rows per thread past 8,192: 81 us a sub-panel,
-// 91 with the third row in shared memory); FP64 N = 998 3.04 -> 2.83.
+// N = 10,242 38.1 -> 31.0 (72 us a sub-panel, 45 at 1,390 rows); FP64 N = 998 3.04 -> 2.83.
 // ---------------------------------------------------------------------------
 constexpr int CP_CTAS = 16, CP_THREADS = 256, CP_WARPS = CP_THREADS / 32, CP_ROW_BYTES = 272, CP_SLOTS = 3;
 // rows up to which one CTA alone factors the sub-panel: at one row per thread
@@ -1096,8 +1096,11 @@ __device__ __forceinline__ uint32_t cl_map(uint32_t a, uint32_t rank) {
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
     return r;
 }
+__device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cl_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cl_arrive();
+    cl_wait();
 }
 __device__ __forceinline__ uint64_t global_ns() {
     uint64_t t;
@@ -1242,6 +1245,34 @@ __device__ __forceinline__ ColPair<double> pair_cms(const ColPair<double> &x, co
     return d;
 }
 
+// 16 bytes of a pair of columns, x - l u: a whole FP32 pair, or one half (0:
+// real parts, 1: imaginary parts) of an FP64 pair
+__device__ __forceinline__ uint4 finish16(uint4 x, const ColMult<float> &l, const ColPair<float> &u, int) {
+    const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(&x);
+    const ColPair<float> v = pair_cms(ColPair<float>{b.x, b.y}, l, u);
+    return make_uint4((uint32_t)v.re, (uint32_t)(v.re >> 32), (uint32_t)v.im, (uint32_t)(v.im >> 32));
+}
+__device__ __forceinline__ uint4 finish16(uint4 x, const ColMult<double> &l, const ColPair<double> &u, int half) {
+    double v[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const double xh = h ? __hiloint2double((int)x.w, (int)x.z) : __hiloint2double((int)x.y, (int)x.x);
+        v[h] = half ? fma(-l.i, u.re[h], fma(-l.r, u.im[h], xh)) : fma(l.i, u.im[h], fma(-l.r, u.re[h], xh));
+    }
+    return make_uint4((uint32_t)__double2loint(v[0]), (uint32_t)__double2hiint(v[0]), (uint32_t)__double2loint(v[1]),
+                      (uint32_t)__double2hiint(v[1]));
+}
+// 16 bytes (part 0, and in FP64 part 1) of a candidate's key: magnitude,
+// position, reciprocal of the pivot
+__device__ __forceinline__ uint4 key16(uint32_t m, int pos, Cx<float> inv, int) {
+    return make_uint4(m, (uint32_t)pos, __float_as_uint(inv.re), __float_as_uint(inv.im));
+}
+__device__ __forceinline__ uint4 key16(uint64_t m, int pos, Cx<double> inv, int part) {
+    if (part == 0) return make_uint4((uint32_t)m, (uint32_t)(m >> 32), (uint32_t)pos, 0u);
+    return make_uint4((uint32_t)__double2loint(inv.re), (uint32_t)__double2hiint(inv.re),
+                      (uint32_t)__double2loint(inv.im), (uint32_t)__double2hiint(inv.im));
+}
+
 template <typename T> struct ClusterPanelArgs {
     Cx<T> *A;
     int64_t ld;
@@ -1310,15 +1341,9 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
         s_abort[0] = s_abort[1] = 0;
     }
     __syncthreads();
+    if (C > 1) cl_arrive();
     for (int i = tid; i < nrows; i += NT)  // rows in flight all at once
         bulk_g2s(sm_addr(row_at(i)), a.A + (int64_t)(gr0 + i) * a.ld + a.k, 256u, sm_addr(&ldbar));
-    // the warp's share of the pushes: CTAs warp, warp + NW, ...; a peer's
-    // shared::cluster address is this CTA's plus a constant
-    constexpr int PUSH = 4;  // NW >= 4
-    uint32_t peer[PUSH];
-#pragma unroll
-    for (int i = 0; i < PUSH; ++i)
-        peer[i] = warp + i * NW < C ? cl_map(sm_addr(smem_raw), warp + i * NW) - sm_addr(smem_raw) : 0u;
     if (!mb_try(&ldbar, 0u)) {
         const uint64_t t0 = global_ns();
         while (!mb_try(&ldbar, 0u))
@@ -1359,11 +1384,10 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
         }
     };
     Key cand{0, CP_NONE, 0};  // the CTA's best row for the next column
-    // The CTA's candidate for column s (each thread's best in `b`) to the
-    // staging buffer, and from there to every CTA.  prow: the pivot row of step
-    // s - 1, which finishes the candidate's pairs from `first` on (nullptr: the
-    // rows are as loaded).  SH, NP: this thread's pairs, A[r][i] at pair
-    // (s >> 1) + i - SH.
+    // The CTA's candidate for column s (each thread's best in `b`) to every CTA
+    // (C = 1: to the staging buffer).  prow: the pivot row of step s - 1, which
+    // finishes the candidate's pairs (nullptr: the rows are as loaded).  SH, NP:
+    // this thread's pairs, A[r][i] at pair (s >> 1) + i - SH.
     auto publish = [&](auto shc, auto npc, int s, int slot, const Best &b, const unsigned char *prow) -> bool {
         constexpr int SH = decltype(shc)::value, NP = decltype(npc)::value;
         const int pb = s & 1, base = s >> 1;
@@ -1377,8 +1401,9 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
         }();
         cand = red[pb][bw];
         unsigned char *buf = stage + pb * RSL;
-        if (warp == bw && cand.pos != CP_NONE) {
-            if (lane == wl) {
+        if (warp == bw) {
+            const bool some = cand.pos != CP_NONE;
+            if (some && lane == wl) {
 #pragma unroll
                 for (int r = 0; r < RPT; ++r)
                     if (cand.li == tid + r * NT) {
@@ -1386,44 +1411,38 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
                         for (int i = SH; i < NP; ++i)  // (past the row's end: the slot's padding)
                             pair_st(buf + (base + i - SH) * PB, A[r][i]);
                     }
-                const T den = b.y.re * b.y.re + b.y.im * b.y.im;
-                const T rd = den > T(0) ? rcp_rn(den) : T(0);
-                M *km = reinterpret_cast<M *>(stage_key + pb * KB);
-                km[0] = cand.m;
-                reinterpret_cast<int *>(km + 1)[0] = cand.pos;
-                *reinterpret_cast<Cx<T> *>(stage_key + pb * KB + KB / 2) = Cx<T>{b.y.re * rd, -b.y.im * rd};
             }
-            if (prow) {  // a lane per pair: even s, from pair s / 2 on; odd s, after the pair that holds column s
-                const Cx<T> l{__shfl_sync(0xffffffffu, b.l.re, wl), __shfl_sync(0xffffffffu, b.l.im, wl)};
-                __syncwarp();
-                if (lane >= base + (s & 1) && lane < NPM)
-                    pair_st(buf + lane * PB, pair_cms(pair_ld(buf + lane * PB, T(0)), pair_mult(l),
-                                                      pair_ld(prow + lane * PB, T(0))));
-            }
-        }
-        __syncthreads();
-        if (C == 1) return true;
-        // to every CTA: the row's first s / 2 pairs (multipliers, complex
-        // entries) from the sub-panel's copy, the rest and the key staged
-        if (lane < 16 + KB / 16) {
+            const Cx<T> l{__shfl_sync(0xffffffffu, b.l.re, wl), __shfl_sync(0xffffffffu, b.l.im, wl)};
+            const Cx<T> y{__shfl_sync(0xffffffffu, b.y.re, wl), __shfl_sync(0xffffffffu, b.y.im, wl)};
+            const T den = y.re * y.re + y.im * y.im;
+            const T rd = den > T(0) ? rcp_rn(den) : T(0);
+            const Cx<T> inv{y.re * rd, -y.im * rd};
+            __syncwarp();
+            // lane q < 16: 16 bytes of the row, finished; of its first s / 2
+            // pairs (multipliers, complex entries) from the sub-panel's copy
+            const int q = lane * 16 / PB;  // the pair they belong to
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            uint32_t dst;
-            if (lane < 16) {
-                const unsigned char *src = lane * 16 < base * PB ? P + (size_t)cand.li * CP_ROW_BYTES : buf;
-                if (cand.pos != CP_NONE) v = reinterpret_cast<const uint4 *>(src)[lane];
-                dst = sm_addr(slot_row) + (uint32_t)(slot * C + rank) * RSL + 16u * lane;
-            } else {
-                if (cand.pos != CP_NONE)
-                    v = reinterpret_cast<const uint4 *>(stage_key + pb * KB)[lane - 16];
-                else if (lane == 16)
-                    (sizeof(M) == 4 ? v.y : v.z) = (uint32_t)CP_NONE;
-                dst = sm_addr(slot_key) + (uint32_t)(slot * C + rank) * KB + 16u * (lane - 16);
+            if (some && lane < 16) {
+                v = reinterpret_cast<const uint4 *>(q < base ? P + (size_t)cand.li * CP_ROW_BYTES : buf)[lane];
+                if (prow && q >= base + (s & 1)) v = finish16(v, pair_mult(l), pair_ld(prow + q * PB, T(0)), lane & 1);
+            } else if (lane >= 16) {
+                v = key16(some ? cand.m : M(0), cand.pos, some ? inv : Cx<T>{T(0), T(0)}, lane - 16);
             }
-            const uint32_t bar = sm_addr(&mbar[slot]);
+            if (C == 1) {
+                if (lane < 16 && q >= base) reinterpret_cast<uint4 *>(buf)[lane] = v;
+                if (lane >= 16 && lane < 16 + KB / 16) reinterpret_cast<uint4 *>(stage_key + pb * KB)[lane - 16] = v;
+            } else if (lane < 16 + KB / 16) {
+                const uint32_t dst = lane < 16 ? sm_addr(slot_row) + (uint32_t)(slot * C + rank) * RSL + 16u * lane
+                                               : sm_addr(slot_key) + (uint32_t)(slot * C + rank) * KB + 16u * (lane - 16);
+                const uint32_t to_bar = sm_addr(&mbar[slot]) - dst;  // the same distance in every CTA
 #pragma unroll
-            for (int i = 0; i < PUSH; ++i)
-                if (warp + i * NW < C) st_async16(dst + peer[i], v, bar + peer[i]);
+                for (int peer = 0; peer < CP_CTAS; ++peer) {
+                    const uint32_t d = cl_map(dst, peer);
+                    st_async16(d, v, d + to_bar);
+                }
+            }
         }
+        if (C == 1) __syncthreads();
         return true;
     };
 
@@ -1545,7 +1564,7 @@ __global__ void __launch_bounds__(CP_THREADS, 1) cluster_panel_kernel(ClusterPan
 #pragma unroll
         for (int r = 0; r < RPT; ++r)
             if (mp[r] >= 0) best.offer(pair_get<0>(A[r][0]), z, mp[r], tid + r * NT);
-        if (C > 1) cl_sync();  // every CTA's mbarriers are initialised before any remote store
+        if (C > 1) cl_wait();  // every CTA's mbarriers are initialised before any remote store
         publish(std::integral_constant<int, 0>{}, std::integral_constant<int, NPM>{}, 0, 0, best, nullptr);
     }
     auto run_phase = [&](auto npc, int j0) {
