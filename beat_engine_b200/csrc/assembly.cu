@@ -658,13 +658,24 @@ __global__ void __launch_bounds__(SymTile<T>::THREADS, 2) sym_pairs_kernel(RegAr
 }
 
 // ---------------------------------------------------------------------------
-// touching pairs: one warp per pair, FP64, Duffy points over the lanes
+// Touching pairs: one warp per pair, FP64, Duffy points over the lanes.
+//
+// With x = x0 + xi e1 + eta e2 on the test face and y = y0 + xi' f1 + eta' f2 on
+// the trial face, every basis product is a combination of 1, xi, eta times 1,
+// xi', eta'; so a point adds the kernel value times those nine monomials, and
+// the nine basis products follow once per pair.  r . n of either face needs only
+// the other face's coordinates.  The rule's points are stored coordinate by
+// coordinate (coalesced), and the 26 sums are reduced over the lanes by
+// halving: each exchange step also halves the number of sums a lane carries.
+// Bound: the FP64 units, about 100 instructions per point (1.1 ms at F =
+// 20,480); @SING@.
 // ---------------------------------------------------------------------------
 template <typename T> struct SingArgs {
     const int *test, *trial, *rule;
     const double *jac, *nn;
     const int *rule_start;
-    const double *rule_data;  // 5 per point
+    const double *rule_data;  // five arrays of npoints: xi, eta, xi', eta', weight
+    int64_t npoints;
     const double *verts;      // V x 3
     const int *faces;         // F x 3
     const double *normals;    // F x 3
@@ -676,6 +687,76 @@ template <typename T> struct SingArgs {
     double k, eta;
 };
 
+// Sums of v[0..31] over the lanes: lane l returns the total of v[l].  Step o
+// hands half of the remaining sums to the lane o away and keeps the others.
+__device__ __forceinline__ double warp_sum32(double (&v)[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            const double send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return v[0];
+}
+
+// the same kernel value's sums against 1, xi', eta', xi, ... in acc[2 (3 i + j)]
+// (i: test monomial 1, xi, eta; j: trial), acc[18 + 2 i]: right-hand-side value
+// against the test monomials, acc[24]: Green sum
+__device__ __forceinline__ void singular_point(double xi, double et, double yi, double ye, const double (&d0)[3],
+                                               const double (&e1)[3], const double (&e2)[3], const double (&f1)[3],
+                                               const double (&f2)[3], double ns0, double nse1, double nse2, double nt0,
+                                               double ntf1, double ntf2, double w, double k, double eta, double k2n,
+                                               double (&acc)[32]) {
+    double r[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        r[c] = fma(yi, f1[c], fma(ye, f2[c], fma(-xi, e1[c], fma(-et, e2[c], d0[c]))));
+    const double r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+    if (r2 == 0.0) return;
+    const double ir = rsqrt_series(r2);
+    double sn_, cs_;
+    sincos_cw(k * (r2 * ir), &sn_, &cs_);
+    const double scl = ir * w;
+    const double gr = cs_ * scl, gi = sn_ * scl;
+    const double hr = (-gr * ir - gi * k) * ir, hi = (gr * k - gi * ir) * ir;  // dG/dr / r
+    const double rns = fma(-xi, nse1, fma(-et, nse2, ns0));                    // r . n_s
+    const double rnt = fma(yi, ntf1, fma(ye, ntf2, nt0));                      // r . n_t
+    const double lr = k2n * gi - hr * rns, li = -(hi * rns + k2n * gr);
+    const double pt = eta * rnt;
+    const double rr = -gr - hi * pt, ri = hr * pt - gi;
+    const double m[4] = {xi * yi, xi * ye, et * yi, et * ye};
+    acc[0] += lr;
+    acc[1] += li;
+    acc[2] = fma(yi, lr, acc[2]);
+    acc[3] = fma(yi, li, acc[3]);
+    acc[4] = fma(ye, lr, acc[4]);
+    acc[5] = fma(ye, li, acc[5]);
+    acc[6] = fma(xi, lr, acc[6]);
+    acc[7] = fma(xi, li, acc[7]);
+    acc[8] = fma(m[0], lr, acc[8]);
+    acc[9] = fma(m[0], li, acc[9]);
+    acc[10] = fma(m[1], lr, acc[10]);
+    acc[11] = fma(m[1], li, acc[11]);
+    acc[12] = fma(et, lr, acc[12]);
+    acc[13] = fma(et, li, acc[13]);
+    acc[14] = fma(m[2], lr, acc[14]);
+    acc[15] = fma(m[2], li, acc[15]);
+    acc[16] = fma(m[3], lr, acc[16]);
+    acc[17] = fma(m[3], li, acc[17]);
+    acc[18] += rr;
+    acc[19] += ri;
+    acc[20] = fma(xi, rr, acc[20]);
+    acc[21] = fma(xi, ri, acc[21]);
+    acc[22] = fma(et, rr, acc[22]);
+    acc[23] = fma(et, ri, acc[23]);
+    acc[24] += gr;
+    acc[25] += gi;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256, 2) singular_pairs_kernel(SingArgs<T> g) {
     const int lane = threadIdx.x & 31;
@@ -683,88 +764,69 @@ __global__ void __launch_bounds__(256, 2) singular_pairs_kernel(SingArgs<T> g) {
     if (pair >= g.npairs) return;
     const int t = g.test[pair], s = g.trial[pair], r = g.rule[pair];
     const int *ft = g.faces + 3 * t, *fs = g.faces + 3 * s;
-    double tv[3][3], sv[3][3];
+    double d0[3], e1[3], e2[3], f1[3], f2[3], ns0 = 0, nse1 = 0, nse2 = 0, nt0 = 0, ntf1 = 0, ntf2 = 0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            tv[a][c] = g.verts[3 * ft[a] + c];
-            sv[a][c] = g.verts[3 * fs[a] + c];
-        }
-    const double ntx = g.normals[3 * t], nty = g.normals[3 * t + 1], ntz = g.normals[3 * t + 2];
-    const double nsx = g.normals[3 * s], nsy = g.normals[3 * s + 1], nsz = g.normals[3 * s + 2];
+    for (int c = 0; c < 3; ++c) {
+        const double x0 = g.verts[3 * ft[0] + c], y0 = g.verts[3 * fs[0] + c];
+        e1[c] = g.verts[3 * ft[1] + c] - x0;
+        e2[c] = g.verts[3 * ft[2] + c] - x0;
+        f1[c] = g.verts[3 * fs[1] + c] - y0;
+        f2[c] = g.verts[3 * fs[2] + c] - y0;
+        d0[c] = y0 - x0;
+        // y - y0 is orthogonal to n_s, x - x0 to n_t
+        const double ns = g.normals[3 * s + c], nt = g.normals[3 * t + c];
+        ns0 += d0[c] * ns;
+        nse1 += e1[c] * ns;
+        nse2 += e2[c] * ns;
+        nt0 += d0[c] * nt;
+        ntf1 += f1[c] * nt;
+        ntf2 += f2[c] * nt;
+    }
     const double k = g.k, eta = g.eta;
     const double k2n = eta * (k * k * g.nn[pair]);
-    double acc[26];
+    double acc[32];
 #pragma unroll
-    for (int i = 0; i < 26; ++i) acc[i] = 0.0;  // L[9] re/im, R[3] re/im, curl re/im
+    for (int i = 0; i < 32; ++i) acc[i] = 0.0;
     const int q1 = g.rule_start[r + 1];
-    for (int q = g.rule_start[r] + lane; q < q1; q += 32) {
-        const double *d = g.rule_data + 5 * (size_t)q;
-        const double xi = d[0], et = d[1], yi = d[2], ye = d[3], w = d[4];
-        const double bt[3] = {1.0 - xi - et, xi, et}, bs[3] = {1.0 - yi - ye, yi, ye};
-        double x[3], y[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            x[c] = bt[0] * tv[0][c] + bt[1] * tv[1][c] + bt[2] * tv[2][c];
-            y[c] = bs[0] * sv[0][c] + bs[1] * sv[1][c] + bs[2] * sv[2][c];
-        }
-        const double rx = y[0] - x[0], ry = y[1] - x[1], rz = y[2] - x[2];
-        const double r2 = rx * rx + ry * ry + rz * rz;
-        if (r2 == 0.0) continue;
-        const double ir = rsqrt(r2), rad = r2 * ir;  // one reciprocal square root, no divide
-        double sn_, cs_;
-        sincos_cw(k * rad, &sn_, &cs_);
-        const double scl = ir * (0.07957747154594767 * w);
-        const double gr = cs_ * scl, gi = sn_ * scl;
-        const double gsr = -gr * ir - gi * k, gsi = gr * k - gi * ir;
-        const double dns = (rx * nsx + ry * nsy + rz * nsz) * ir;
-        const double dnt = -(rx * ntx + ry * nty + rz * ntz) * ir;
-        const double lr = -gsr * dns + k2n * gi, li = -gsi * dns - k2n * gr;
-        const double rr = -gr + eta * (gsi * dnt), ri = -gi - eta * (gsr * dnt);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                const double bp = bt[a] * bs[b];
-                acc[2 * (3 * a + b)] += bp * lr;
-                acc[2 * (3 * a + b) + 1] += bp * li;
-            }
-            acc[18 + 2 * a] += bt[a] * rr;
-            acc[18 + 2 * a + 1] += bt[a] * ri;
-        }
-        acc[24] += gr;
-        acc[25] += gi;
-    }
-#pragma unroll
-    for (int i = 0; i < 26; ++i) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
-    }
+    const double *rd = g.rule_data;
+    const int64_t np = g.npoints;
+    for (int q = g.rule_start[r] + lane; q < q1; q += 32)
+        singular_point(rd[q], rd[np + q], rd[2 * np + q], rd[3 * np + q], d0, e1, e2, f1, f2, ns0, nse1, nse2, nt0,
+                       ntf1, ntf2, 0.07957747154594767 * rd[4 * np + q], k, eta, k2n, acc);
+    const double mine = warp_sum32(acc);  // lane i: sum i
+    // the basis products: phi_0 = 1 - phi_1 - phi_2 on either face
     const double jac = g.jac[pair];
-    const double ccr = -eta * acc[25], cci = eta * acc[24];
+    auto sum = [&](int i) { return __shfl_sync(0xffffffffu, mine, i); };
+    const double cr = sum(24), ci = sum(25);
+    const int a = lane / 3, b = lane % 3;  // lanes 0..8: entry (a, b); lanes 9..11: right-hand side a = lane - 9
+    // monomial sums M[i][j]: entry = sum_i,j ca(a, i) cb(b, j) M[i][j], c(0, .) = (1, -1, -1), c(1, .) = (0, 1, 0), ...
+    double vr = 0.0, vi = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int row = lane < 9 ? a : lane - 9;
+        const double ca = row == 0 ? (i == 0 ? 1.0 : -1.0) : (row == i ? 1.0 : 0.0);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const double cb = b == 0 ? (j == 0 ? 1.0 : -1.0) : (b == j ? 1.0 : 0.0);
+            const double mr = sum(2 * (3 * i + j)), mi = sum(2 * (3 * i + j) + 1);
+            if (lane < 9) {
+                vr = fma(ca * cb, mr, vr);
+                vi = fma(ca * cb, mi, vi);
+            }
+        }
+        const double qr = sum(18 + 2 * i), qi = sum(18 + 2 * i + 1);
+        if (lane >= 9) {
+            vr = fma(ca, qr, vr);
+            vi = fma(ca, qi, vi);
+        }
+    }
     if (lane < 9) {
-        const int a = lane / 3, b = lane % 3;
+        const double ccr = -eta * ci, cci = eta * cr;
         const double *cta = g.curls + 9 * t + 3 * a, *csb = g.curls + 9 * s + 3 * b;
         const double d = cta[0] * csb[0] + cta[1] * csb[1] + cta[2] * csb[2];
-        double vr = 0, vi = 0;
-#pragma unroll
-        for (int i = 0; i < 9; ++i)
-            if (i == lane) {
-                vr = acc[2 * i];
-                vi = acc[2 * i + 1];
-            }
         red_add_cx(&g.A[(int64_t)ft[a] * g.ld + fs[b]], (T)((vr + d * ccr) * jac), (T)((vi + d * cci) * jac));
     } else if (lane < 12) {
-        const int a = lane - 9;
-        double vr = 0, vi = 0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            if (i == a) {
-                vr = acc[18 + 2 * i];
-                vi = acc[18 + 2 * i + 1];
-            }
-        rhs_add(g.rhs, ft[a], s, (T)(vr * jac), (T)(vi * jac));
+        rhs_add(g.rhs, ft[lane - 9], s, (T)(vr * jac), (T)(vi * jac));
     }
 }
 
@@ -784,7 +846,8 @@ template <typename T> struct ImgArgs {
     const int *test, *trial, *rule, *img;
     const double *jac, *nn;
     const int *rule_start;
-    const double *rule_data;  // 5 per point
+    const double *rule_data;  // five arrays of npoints
+    int64_t npoints;
     const double *verts;
     const int *faces;
     const double *normals, *curls;
@@ -856,7 +919,9 @@ __global__ void __launch_bounds__(256, 2) image_delta_kernel(ImgArgs<T> g) {
     for (int i = 0; i < 26; ++i) acc[i] = 0.0;
     // + Duffy
     for (int q = g.rule_start[r] + lane; q < g.rule_start[r + 1]; q += 32) {
-        const double *d = g.rule_data + 5 * (size_t)q;
+        double d[5];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) d[c] = g.rule_data[c * g.npoints + q];
         const double bt[3] = {1.0 - d[0] - d[1], d[0], d[1]}, bs[3] = {1.0 - d[2] - d[3], d[2], d[3]};
         double x[3], y[3];
 #pragma unroll
@@ -1050,6 +1115,7 @@ template <typename T> static void assemble_t(beat_b200_ctx *c, double k, double 
         s.nn = c->sp_nn.as<double>();
         s.rule_start = c->rule_start.as<int>();
         s.rule_data = c->rule_data.as<double>();
+        s.npoints = c->npoints;
         s.verts = c->d_verts.as<double>();
         s.faces = c->d_faces.as<int>();
         s.normals = c->d_normals.as<double>();
@@ -1074,6 +1140,7 @@ template <typename T> static void assemble_t(beat_b200_ctx *c, double k, double 
         d.nn = c->ip_nn.as<double>();
         d.rule_start = c->rule_start.as<int>();
         d.rule_data = c->rule_data.as<double>();
+        d.npoints = c->npoints;
         d.verts = c->d_verts.as<double>();
         d.faces = c->d_faces.as<int>();
         d.normals = c->d_normals.as<double>();

@@ -687,7 +687,10 @@ void set_mesh(beat_b200_ctx *c, int V, const double *verts, int F, const int32_t
     upload(c->sp_jac, sp_j);
     upload(c->sp_nn, sp_n);
     upload(c->rule_start, rstart);
-    upload(c->rule_data, rdata);
+    c->npoints = (int64_t)rdata.size() / 5;  // coordinate by coordinate, so that a warp's points are coalesced
+    std::vector<double> rsoa(rdata.size());
+    for (size_t i = 0; i < rdata.size(); ++i) rsoa[(i % 5) * c->npoints + i / 5] = rdata[i];
+    upload(c->rule_data, rsoa);
 }
 
 // ---------------------------------------------------------------------------

@@ -224,7 +224,8 @@ struct beat_b200_ctx {
     bb::DevBuf sp_test, sp_trial, sp_rule;  // int per pair (original face ids)
     bb::DevBuf sp_jac, sp_nn;               // double per pair
     bb::DevBuf rule_start;                  // nrules + 1
-    bb::DevBuf rule_data;                   // per point: test xi, eta, trial xi, eta, weight
+    int64_t npoints = 0;                    // points of all rules
+    bb::DevBuf rule_data;                   // five arrays of npoints: test xi, eta, trial xi, eta, weight
 
     int64_t regular_pairs = 0;
     bb::DevBuf status;            // device status word(s)

@@ -101,7 +101,7 @@ __device__ __forceinline__ void reverse_point(const double (&x)[3], const double
     const double r[3] = {y[0] - x[0], y[1] - x[1], y[2] - x[2]};
     const double r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
     if (r2 == 0.0) return;
-    const double iR = rsqrt(r2), R = r2 * iR;
+    const double iR = rsqrt_series(r2), R = r2 * iR;
     const double rh[3] = {r[0] * iR, r[1] * iR, r[2] * iR};
     double sn_, cs_;
     sincos_cw(k * R, &sn_, &cs_);
@@ -482,7 +482,8 @@ struct ShapeSingArgs {
     ShapeImage xf[3];         // the images' reflections
     ShapeRule reg;            // the regular rule an image pass applied to the pair
     const int *rule_start;
-    const double *rule_data;  // per point: test xi, eta, trial xi, eta, weight
+    const double *rule_data;  // five arrays of npoints: test xi, eta, trial xi, eta, weight
+    int64_t npoints;
     const double *verts, *normals, *curls, *areas;
     const int *faces;
     const double2 *z, *p, *q;
@@ -546,7 +547,9 @@ __global__ void __launch_bounds__(256) shape_singular_kernel(ShapeSingArgs g) {
     pair_adj_zero(acc);
     const int q1 = g.rule_start[ru + 1];
     for (int qi = g.rule_start[ru] + lane; qi < q1; qi += 32) {
-        const double *d = g.rule_data + 5 * (size_t)qi;
+        double d[5];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) d[c] = g.rule_data[c * g.npoints + qi];
         const double bt[3] = {1.0 - d[0] - d[1], d[0], d[1]}, bs[3] = {1.0 - d[2] - d[3], d[2], d[3]};
         double x[3], y[3];
 #pragma unroll
@@ -873,6 +876,7 @@ void shape_gradient(beat_b200_ctx *c, double k, double eta, int M, const double 
     ShapeSingArgs s;
     s.rule_start = c->rule_start.as<int>();
     s.rule_data = c->rule_data.as<double>();
+    s.npoints = c->npoints;
     s.verts = c->d_verts.as<double>();
     s.normals = c->d_normals.as<double>();
     s.curls = c->d_curls.as<double>();
