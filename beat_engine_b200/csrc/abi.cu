@@ -103,20 +103,20 @@ void solve_core(beat_b200_ctx *c, double k, double eta, int R, const double *d_q
     ensure_workspace(c, o.precision, R, rhs_request(o));
     Workspace &w = c->ws;
     const int n = c->V;
-    float ms_asm = 0, ms_sing = 0, ms_lu = 0, ms_solve = 0, ms_ir = 0;
-    assemble(c, k, eta, o.precision, R, d_q, &ms_asm, &ms_sing);
+    // One solve is queued as far as the refinement's first residual before the
+    // host waits: the status words of the factorisation are read there (the
+    // substitutions end whatever the factors hold), the stage times at the end.
+    float ms_asm = 0, ms_sing = 0, ms_reg = 0, ms_lu = 0, ms_solve = 0, ms_ir = 0;
+    assemble(c, k, eta, o.precision, R, d_q);
     apply_admittance_lhs(c, o.precision);  // A += B diag(a) P when an admittance is set
     if (o.precision != BEAT_B200_FP64)
         BB_CUDA(cudaMemcpyAsync(w.Aop.p, w.A.p, (size_t)n * w.ld * 8, cudaMemcpyDeviceToDevice, c->stream));
     BB_CUDA(cudaEventRecord(c->ev[4], c->stream));
     lu_factor(c, o.precision, o.lu_block, o.lu_split_terms);
     BB_CUDA(cudaEventRecord(c->ev[5], c->stream));
-    const int st = read_status(c);
+    queue_status(c, 0);
     c->last_k = k;
     c->last_eta = eta;
-    BB_REQUIRE(!(st & DEV_BARRIER_TIMEOUT), BEAT_B200_TIMEOUT, "LU panel: grid barrier ran out of its wait budget");
-    BB_REQUIRE(!(st & DEV_ZERO_PIVOT), BEAT_B200_SINGULAR, "LU: exact zero pivot (singular system)");
-    w.lu_valid = 1;
     IrResult ir{0, 1, 0.0};
     if (o.precision == BEAT_B200_FP64) {
         BB_CUDA(cudaMemcpyAsync(d_x, w.b.p, (size_t)n * R * 16, cudaMemcpyDeviceToDevice, c->stream));
@@ -132,17 +132,20 @@ void solve_core(beat_b200_ctx *c, double k, double eta, int R, const double *d_q
             ir = gmres_refine(c, R, d_x, w.b.as<double>(), o.ir_restart, o.ir_max_iters, o.ir_rtol);
         BB_CUDA(cudaEventRecord(c->ev[7], c->stream));
     }
-    BB_CUDA(cudaEventSynchronize(c->ev[7]));
-    const int st2 = read_status(c);
-    BB_REQUIRE(!(st2 & DEV_BARRIER_TIMEOUT), BEAT_B200_TIMEOUT,
+    queue_status(c, 1);
+    BB_CUDA(cudaStreamSynchronize(c->stream));
+    check_factor_status(c);
+    w.lu_valid = 1;
+    BB_REQUIRE(!(c->h_status[1] & DEV_BARRIER_TIMEOUT), BEAT_B200_TIMEOUT,
                "triangular solve: a block wait ran out of its budget");
+    assembly_times(c, &ms_asm, &ms_sing, &ms_reg);
     BB_CUDA(cudaEventElapsedTime(&ms_lu, c->ev[4], c->ev[5]));
     BB_CUDA(cudaEventElapsedTime(&ms_solve, c->ev[5], c->ev[6]));
     BB_CUDA(cudaEventElapsedTime(&ms_ir, c->ev[6], c->ev[7]));
     if (diag) {
         diag->assembly_ms = ms_asm;
         diag->singular_ms = ms_sing;
-        diag->regular_ms = c->last_regular_ms;
+        diag->regular_ms = ms_reg;
         diag->lu_ms = ms_lu;
         diag->solve_ms = ms_solve;
         diag->ir_ms = ms_ir;
@@ -421,6 +424,8 @@ int32_t beat_b200_create(int32_t device, beat_b200_ctx **out) {
         BB_CUDA(cudaEventCreateWithFlags(&c->la_fork, cudaEventDisableTiming));
         BB_CUDA(cudaEventCreateWithFlags(&c->la_join, cudaEventDisableTiming));
         for (auto &e : c->ev) BB_CUDA(cudaEventCreate(&e));
+        BB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&c->h_status), beat_b200_ctx::HOST_PIN, cudaHostAllocDefault));
+        c->h_status[0] = c->h_status[1] = 0;
         c->status.alloc(256);
         BB_CUDA(cudaMemset(c->status.p, 0, 256));
         c->barrier.alloc(sizeof(unsigned) * 4096);
@@ -457,6 +462,7 @@ int32_t beat_b200_destroy(beat_b200_ctx *c) {
     }
     for (auto &e : c->ev)
         if (e) cudaEventDestroy(e);
+    if (c->h_status) cudaFreeHost(c->h_status);
     if (c->side_stream) cudaStreamSynchronize(c->side_stream);
     for (cudaEvent_t e : {c->la_fork, c->la_join})
         if (e) cudaEventDestroy(e);
@@ -617,7 +623,7 @@ int32_t beat_b200_assemble(beat_b200_ctx *c, double k, double eta, int32_t R, co
             BB_CUDA(cudaMemcpyAsync(w.q.p, q, (size_t)c->F * R * 16, cudaMemcpyHostToDevice, c->stream));
         else
             BB_CUDA(cudaMemsetAsync(w.q.p, 0, (size_t)c->F * 16, c->stream));
-        assemble(c, k, eta, precision, Rr, w.q.p, nullptr, nullptr);
+        assemble(c, k, eta, precision, Rr, w.q.p);
         w.lu_valid = 0;
         if (A_out) {
             DevBuf tmp;

@@ -1087,8 +1087,7 @@ static void launch_sym(beat_b200_ctx *c, double k, double eta, int img, int R, c
     BB_CUDA(cudaGetLastError());
 }
 
-template <typename T> static void assemble_t(beat_b200_ctx *c, double k, double eta, int R, const Cx<double> *q,
-                                             float *ms_total, float *ms_singular) {
+template <typename T> static void assemble_t(beat_b200_ctx *c, double k, double eta, int R, const Cx<double> *q) {
     Workspace &w = c->ws;
     const int N = c->V, F = c->F;
     BB_CUDA(cudaEventRecord(c->ev[0], c->stream));
@@ -1176,23 +1175,22 @@ template <typename T> static void assemble_t(beat_b200_ctx *c, double k, double 
                      w.b.as<double>(), R, 1.0);
     }
     BB_CUDA(cudaEventRecord(c->ev[3], c->stream));
-    if (ms_total || ms_singular) {
-        BB_CUDA(cudaEventSynchronize(c->ev[3]));
-        if (ms_total) BB_CUDA(cudaEventElapsedTime(ms_total, c->ev[0], c->ev[3]));
-        if (ms_singular) BB_CUDA(cudaEventElapsedTime(ms_singular, c->ev[1], c->ev[2]));
-        BB_CUDA(cudaEventElapsedTime(&c->last_regular_ms, c->ev[8], c->ev[1]));
-    }
 }
 
-void assemble(beat_b200_ctx *c, double k, double eta, int precision, int R, const void *q_dev, float *ms_total,
-              float *ms_singular) {
+void assembly_times(beat_b200_ctx *c, float *total, float *singular, float *regular) {
+    BB_CUDA(cudaEventElapsedTime(total, c->ev[0], c->ev[3]));
+    BB_CUDA(cudaEventElapsedTime(singular, c->ev[1], c->ev[2]));
+    BB_CUDA(cudaEventElapsedTime(regular, c->ev[8], c->ev[1]));
+}
+
+void assemble(beat_b200_ctx *c, double k, double eta, int precision, int R, const void *q_dev) {
     BB_REQUIRE(c->F > 0, BEAT_B200_STATE, "no mesh: call beat_b200_set_mesh first");
     BB_REQUIRE(std::isfinite(k) && k != 0.0 && std::isfinite(eta), BEAT_B200_INVALID_ARG,
                "assemble: wavenumber must be finite and nonzero");
     if (precision == BEAT_B200_FP64)
-        assemble_t<double>(c, k, eta, R, (const Cx<double> *)q_dev, ms_total, ms_singular);
+        assemble_t<double>(c, k, eta, R, (const Cx<double> *)q_dev);
     else
-        assemble_t<float>(c, k, eta, R, (const Cx<double> *)q_dev, ms_total, ms_singular);
+        assemble_t<float>(c, k, eta, R, (const Cx<double> *)q_dev);
 }
 
 }  // namespace bb

@@ -732,9 +732,14 @@ void ensure_workspace(beat_b200_ctx *c, int precision, int R, int rhs_request) {
     // the mode: free device memory plus what this context's matrix buffers hold
     const int64_t matrix_bytes = (int64_t)N * ld * (int64_t)csz * (precision == BEAT_B200_FP64 ? 1 : 2);
     const int64_t operator_bytes = (int64_t)N * F * (int64_t)csz;
-    size_t free_b = 0, total_b = 0;
-    BB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    const int64_t available = (int64_t)free_b + (int64_t)(w.A.bytes + w.Aop.bytes + w.B.bytes);
+    // (one excitation under auto and a matrix-free request never take the
+    // mapping: no need to ask the driver, a few tens of microseconds)
+    int64_t available = 0;
+    if (c->adm_set || rhs_request == BEAT_B200_RHS_CACHED || (rhs_request == BEAT_B200_RHS_AUTO && R >= 2)) {
+        size_t free_b = 0, total_b = 0;
+        BB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+        available = (int64_t)free_b + (int64_t)(w.A.bytes + w.Aop.bytes + w.B.bytes);
+    }
     bool cached;
     if (c->adm_set) {
         cached = true;  // the admittance term A += B diag(a) P needs B
@@ -800,6 +805,16 @@ int64_t device_bytes(const beat_b200_ctx *c) {
         s += (int64_t)(t->face_start.bytes + t->vert_start.bytes + t->verts.bytes + t->local_vert.bytes +
                        t->incidence.bytes);
     return s;
+}
+
+void queue_status(beat_b200_ctx *c, int slot) {
+    BB_CUDA(cudaMemcpyAsync(&c->h_status[slot], c->status.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+}
+
+void check_factor_status(const beat_b200_ctx *c) {
+    const int st = c->h_status[0];
+    BB_REQUIRE(!(st & DEV_BARRIER_TIMEOUT), BEAT_B200_TIMEOUT, "LU panel: grid barrier ran out of its wait budget");
+    BB_REQUIRE(!(st & DEV_ZERO_PIVOT), BEAT_B200_SINGULAR, "LU: exact zero pivot (singular system)");
 }
 
 int read_status(beat_b200_ctx *c) {

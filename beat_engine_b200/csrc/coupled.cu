@@ -167,7 +167,7 @@ void assemble_coupled(beat_b200_ctx *c, double k, int precision, void *d_A, void
     ensure_workspace(c, precision, 1, BEAT_B200_RHS_CACHED);
     BB_REQUIRE(c->ws.rhs_cached, BEAT_B200_OOM, "coupled assembly: the N x F operator C does not fit in memory");
     Workspace &w = c->ws;
-    assemble(c, k, 1.0 / k, precision, 0, w.q.p, nullptr, nullptr);  // alpha = i / k; the operators alone, no column
+    assemble(c, k, 1.0 / k, precision, 0, w.q.p);  // alpha = i / k; the operators alone, no column
     w.lu_valid = 0;
     if (precision == BEAT_B200_FP64)
         export_coupled<double>(c, d_A, d_C);

@@ -229,6 +229,10 @@ struct beat_b200_ctx {
 
     int64_t regular_pairs = 0;
     bb::DevBuf status;            // device status word(s)
+    // pinned host words: the status after the factorisation and at the end of a
+    // solve, then HOST_PIN - 16 bytes for the refinement's small read-backs
+    static constexpr size_t HOST_PIN = 65536;
+    int *h_status = nullptr;
     bb::DevBuf barrier;           // grid-barrier counters
     bb::Workspace ws;
 
@@ -242,7 +246,6 @@ struct beat_b200_ctx {
     cudaGraphExec_t lu_graph = nullptr;
     uint64_t lu_graph_key[12] = {};
     int lu_graph_state = 0;  // 0: none, 2: graph of lu_graph_key ready, 3: that key runs eagerly
-    float last_regular_ms = 0.f;
     bool cluster_checked = false;  // can a 16-CTA cluster of the panel kernel be scheduled?
     bool cluster_ok = false;
 
@@ -265,6 +268,10 @@ int rhs_use_operator(int mode, int excitations, int64_t matrix_bytes, int64_t op
 void release_workspace(beat_b200_ctx *c);
 int64_t device_bytes(const beat_b200_ctx *c);
 int read_status(beat_b200_ctx *c);
+// queues a copy of the status word to h_status[slot]; after a synchronisation,
+// check_factor_status raises what slot 0 (after the factorisation) reports
+void queue_status(beat_b200_ctx *c, int slot);
+void check_factor_status(const beat_b200_ctx *c);
 
 // assembly.cu: rule tables in constant memory (fixed per rule size)
 void upload_rule_tables(const std::vector<double> &pts, const std::vector<double> &w, int Q);
@@ -273,8 +280,9 @@ int triangle_rule(int order, std::vector<double> &pts, std::vector<double> &w);
 // assembly.cu: A (row-major N x ld) and B (N x F) in the workspace precision,
 // then b = B q (FP64, N x R column-major).  q_dev is F x R FP64 complex; R = 0
 // (cached mode) forms A and B alone.
-void assemble(beat_b200_ctx *c, double k, double eta, int precision, int R, const void *q_dev,
-              float *ms_total, float *ms_singular);
+void assemble(beat_b200_ctx *c, double k, double eta, int precision, int R, const void *q_dev);
+// stage times of the last assembly, once its events have completed
+void assembly_times(beat_b200_ctx *c, float *total, float *singular, float *regular);
 
 // lu.cu
 void lu_factor(beat_b200_ctx *c, int precision, int nb, int split_terms);
