@@ -349,21 +349,8 @@ struct SourceSplit {
 template <typename K> static SourceSplit resident_split(const beat_b200_ctx *c, K *kernel, int M, int S) {
     int per_sm = 1;
     BB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, FLD_THREADS, 0));
-    const int64_t cap = (int64_t)std::max(1, per_sm) * c->sm_count;
     const int mt = (M + FLD_POINTS - 1) / FLD_POINTS, chunks = (S + FLD_CHUNK - 1) / FLD_CHUNK;
-    const int most = (int)std::min<int64_t>(std::max(1, chunks / 4), std::max<int64_t>(1, 4 * cap / mt));
-    int best = 1;
-    double best_use = 0;
-    for (int n = 1; n <= most; ++n) {
-        const int per = (chunks + n - 1) / n, parts = (chunks + per - 1) / per;
-        const int64_t ctas = (int64_t)mt * parts, waves = (ctas + cap - 1) / cap;
-        const double use = (double)mt * chunks / ((double)waves * cap * per);  // useful share of the waves' time
-        if (use > best_use * 1.02) {
-            best = n;
-            best_use = use;
-        }
-    }
-    const int per = (chunks + best - 1) / best * FLD_CHUNK;
+    const int per = chunks_per_slice(mt, chunks, (int64_t)std::max(1, per_sm) * c->sm_count, 4) * FLD_CHUNK;
     return {dim3(mt, (S + per - 1) / per), per};
 }
 

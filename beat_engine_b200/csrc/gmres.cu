@@ -24,88 +24,145 @@
 namespace bb {
 
 // ---------------------------------------------------------------------------
-// Tall-skinny complex product Y += alpha M X (M rows x K complex in the
-// workspace precision, row-major; X, Y FP64 column-major with R columns).
-// One thread per row of M, all TG_RC right-hand sides of a chunk in FP64
-// registers: an M entry read from shared memory feeds 4 TG_RC DFMA, the X
-// entries are warp-broadcast loads.  The K range is cut into slices so that
-// about two CTAs per SM are resident; slices add into Y with FP64 atomics.
-// Bound: FP64 FMA issue (4 DFMA per complex multiply-add).
+// Tall-skinny complex products Y += alpha M X and Y += alpha M^H X (M row-major
+// in the workspace precision; X, Y FP64 column-major with R columns), on the
+// FP64 tensor cores: m8n8k4 blocks, four real products per complex block, an
+// FP32 M widened exactly as it is read.  Fragments (PTX ISA, m8n8k4 .f64): A
+// (lane / 4, lane % 4), B (lane % 4, lane / 4), C (lane / 4, 2 (lane % 4) + 0, 1).
+//
+// A warp owns TM_MB blocks of 8 outputs and 8 NB right-hand sides; M's
+// fragments go from memory straight to registers (four lanes read four
+// neighbours of a row, or eight lanes eight of them in the M^H case: whole
+// 32-byte sectors either way; 8- and 16-byte loads, so any ld will do), the next
+// 16 reduction indices while the present ones are multiplied.  X goes through
+// two cp.async stages; rows of 2 mod 8 entries keep a quarter-warp's loads on
+// distinct banks.  The reduction is cut into slices that fill whole waves of
+// resident CTAs; they add into Y with FP64 atomics.
+// Bound: M's bytes with up to 8 columns, the FP64 tensor cores with 16.
+// FP32 M, R = 16, one N x F and three N x N products with N = 10,242, F = 20,480:
+// 3.63 ms with one row and 16 columns of FP64 FMA per thread, 2.80 ms (24
+// TFLOP/s of the 37 measured) with this; N = 1,390, R = 4, N x N: 17.8 -> 7.5 us
+// (16 columns were computed whatever R was).
 // ---------------------------------------------------------------------------
-constexpr int TG_THREADS = 256, TG_RC = 16;
+constexpr int TM_WARPS = 8, TM_MB = 2, TM_ROWS = TM_WARPS * TM_MB * 8, TM_KC = 32, TM_G = 16;
 
-// one 8- or 16-byte element global -> shared through the asynchronous copy
-// unit, or zeros (nothing is read) when `in` is false
-template <typename E> __device__ __forceinline__ void cp_async_zfill(E *smem, const E *gmem, bool in) {
-    static_assert(sizeof(E) == 8 || sizeof(E) == 16, "8- or 16-byte elements");
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
-    const int n = in ? (int)sizeof(E) : 0;
-    if constexpr (sizeof(E) == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(gmem), "r"(n) : "memory");
-    else
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem), "r"(n) : "memory");
+__device__ __forceinline__ void tm_mma(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
 }
-template <typename T> struct TgChunk {
-    static constexpr int KC = 32;  // K entries per shared-memory chunk (c64 M)
-    static constexpr int STAGE_UNROLL = 1;  // unrolling of the chunk's copy loop (no spills at 128 registers)
-};
-template <> struct TgChunk<double> {
-    static constexpr int KC = 16;
-    static constexpr int STAGE_UNROLL = 4;
-};
 
-template <typename T>
-__global__ void __launch_bounds__(TG_THREADS, 2) tall_gemm_kernel(const Cx<T> *M, int64_t ld, int rows, int K,
-                                                                  const double2 *X, double2 *Y, int R, int r0,
-                                                                  double alpha, int kslice) {
-    constexpr int KC = TgChunk<T>::KC;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Cx<T> *sM = reinterpret_cast<Cx<T> *>(smem_raw);                                          // TG_THREADS x (KC + 1)
-    double2 *sX = reinterpret_cast<double2 *>(smem_raw + sizeof(Cx<T>) * TG_THREADS * (KC + 1));  // KC x TG_RC
-    const int row0 = blockIdx.x * TG_THREADS, row = row0 + (int)threadIdx.x;
+// no outputs, reduction length K: M is no x K (row-major, H = false) or K x no (H = true)
+template <typename T, bool H, int NB>
+__global__ void __launch_bounds__(TM_WARPS * 32, 2) tall_mma_kernel(const Cx<T> *M, int64_t ld, int no, int K,
+                                                                    const double2 *X, double2 *Y, int R, int r0,
+                                                                    double alpha, int kslice) {
+    constexpr int COLS = 8 * NB, XS = COLS + 2, STEPS = TM_G / 4;
+    __shared__ __align__(16) double2 sX[2][TM_KC * XS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = lane >> 2, q = lane & 3;
     const int kb = blockIdx.y * kslice, ke = min(K, kb + kslice);
-    const int rc = min(TG_RC, R - r0);
-    double ar[TG_RC], ai[TG_RC];
+    const int rc = min(COLS, R - r0);
+    const int o0 = blockIdx.x * TM_ROWS + warp * TM_MB * 8 + row;
+    const Cx<T> *base[TM_MB];  // outputs past the end read the last one's entries and are not stored
 #pragma unroll
-    for (int e = 0; e < TG_RC; ++e) ar[e] = ai[e] = 0.0;
-    for (int k0 = kb; k0 < ke; k0 += KC) {
-        const int kn = min(KC, ke - k0);
-        // the chunk of M and of X by asynchronous copies, all in flight at
-        // once; entries past the matrix are zero-filled
-#pragma unroll TgChunk<T>::STAGE_UNROLL
-        for (int i = threadIdx.x; i < TG_THREADS * KC; i += TG_THREADS) {
-            const int r = i / KC, k = i % KC;  // consecutive threads: consecutive k of one row
-            const bool in = row0 + r < rows && k < kn;
-            cp_async_zfill(&sM[r * (KC + 1) + k], in ? &M[(int64_t)(row0 + r) * ld + k0 + k] : M, in);
+    for (int m = 0; m < TM_MB; ++m) {
+        const int o = min(o0 + 8 * m, no - 1);
+        base[m] = H ? M + o : M + (int64_t)o * ld;
+    }
+    Cx<T> cur[STEPS][TM_MB], nxt[STEPS][TM_MB];
+    auto load = [&](Cx<T> (&a)[STEPS][TM_MB], int k0) {
+#pragma unroll
+        for (int s = 0; s < STEPS; ++s) {
+            const int k = k0 + 4 * s + q;
+#pragma unroll
+            for (int m = 0; m < TM_MB; ++m)
+                a[s][m] = k < ke ? base[m][H ? (int64_t)k * ld : (int64_t)k] : Cx<T>{T(0), T(0)};
         }
-        for (int i = threadIdx.x; i < KC * TG_RC; i += TG_THREADS) {
-            const int c = i / KC, k = i % KC;
-            const bool in = c < rc && k < kn;
-            cp_async_zfill(&sX[k * TG_RC + c], in ? &X[(size_t)(r0 + c) * K + k0 + k] : X, in);
+    };
+    auto stage = [&](int buf, int k0) {
+        for (int i = threadIdx.x; i < TM_KC * COLS; i += TM_WARPS * 32) {
+            const int c = i / TM_KC, k = i % TM_KC;
+            const bool in = c < rc && k0 + k < ke;
+            const double2 *src = in ? &X[(size_t)(r0 + c) * K + k0 + k] : X;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(&sX[buf][k * XS + c])),
+                         "l"(src), "r"(in ? 16 : 0)
+                         : "memory");
         }
-        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double re[TM_MB][NB][2] = {}, im[TM_MB][NB][2] = {};
+    stage(0, kb);
+    load(cur, kb);
+    int buf = 0;
+    for (int k0 = kb; k0 < ke; k0 += TM_KC, buf ^= 1) {
+        stage(buf ^ 1, k0 + TM_KC);  // past the slice: zeros
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
-#pragma unroll 2
-        for (int k = 0; k < KC; ++k) {
-            const Cx<T> m = sM[threadIdx.x * (KC + 1) + k];
-            const double mr = (double)m.re, mi = (double)m.im;
 #pragma unroll
-            for (int e = 0; e < TG_RC; ++e) {
-                const double2 x = sX[k * TG_RC + e];
-                ar[e] = fma(mr, x.x, fma(-mi, x.y, ar[e]));
-                ai[e] = fma(mr, x.y, fma(mi, x.x, ai[e]));
+        for (int g = 0; g < TM_KC; g += TM_G) {
+            load(nxt, k0 + g + TM_G);
+#pragma unroll
+            for (int s = 0; s < STEPS; ++s) {
+                const double2 *x = &sX[buf][(g + 4 * s + q) * XS + row];
+                double2 b[NB];
+#pragma unroll
+                for (int n = 0; n < NB; ++n) b[n] = x[8 * n];
+#pragma unroll
+                for (int m = 0; m < TM_MB; ++m) {
+                    const double ar = (double)cur[s][m].re;
+                    const double ai = H ? -(double)cur[s][m].im : (double)cur[s][m].im, ni = -ai;
+#pragma unroll
+                    for (int n = 0; n < NB; ++n) {
+                        tm_mma(re[m][n], ar, b[n].x);
+                        tm_mma(im[m][n], ar, b[n].y);
+                    }
+#pragma unroll
+                    for (int n = 0; n < NB; ++n) {
+                        tm_mma(re[m][n], ni, b[n].y);
+                        tm_mma(im[m][n], ai, b[n].x);
+                    }
+                }
             }
+#pragma unroll
+            for (int s = 0; s < STEPS; ++s)
+#pragma unroll
+                for (int m = 0; m < TM_MB; ++m) cur[s][m] = nxt[s][m];
         }
         __syncthreads();
     }
-    if (row < rows) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-        for (int e = 0; e < TG_RC; ++e)
-            if (e < rc) {
-                double2 *y = &Y[(size_t)(r0 + e) * rows + row];
-                atomicAdd(&y->x, alpha * ar[e]);
-                atomicAdd(&y->y, alpha * ai[e]);
+    for (int m = 0; m < TM_MB; ++m) {
+        const int o = o0 + 8 * m;
+        if (o >= no) continue;
+#pragma unroll
+        for (int n = 0; n < NB; ++n)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = 8 * n + 2 * q + h;
+                if (c >= rc) continue;
+                double2 *y = &Y[(size_t)(r0 + c) * no + o];
+                atomicAdd(&y->x, alpha * re[m][n][h]);
+                atomicAdd(&y->y, alpha * im[m][n][h]);
             }
+    }
+}
+
+template <typename T, bool H>
+static void tall_product(cudaStream_t st, int sm_count, const Cx<T> *M, int64_t ld, int no, int K, const double *X,
+                         double *Y, int R, double alpha) {
+    const int tiles = (no + TM_ROWS - 1) / TM_ROWS, chunks = (K + TM_KC - 1) / TM_KC;
+    for (int r0 = 0; r0 < R; r0 += 16) {
+        // 8 columns when no more are left: half the products, the same bytes of M
+        const auto kernel = R - r0 <= 8 ? tall_mma_kernel<T, H, 1> : tall_mma_kernel<T, H, 2>;
+        int per_sm = 1;
+        BB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, TM_WARPS * 32, 0));
+        const int per = chunks_per_slice(tiles, chunks, std::max(1, per_sm) * sm_count, 2);
+        const int kslice = per * TM_KC;
+        kernel<<<dim3(tiles, (K + kslice - 1) / kslice), TM_WARPS * 32, 0, st>>>(
+            M, ld, no, K, reinterpret_cast<const double2 *>(X), reinterpret_cast<double2 *>(Y), R, r0, alpha, kslice);
+        BB_CUDA(cudaGetLastError());
     }
 }
 
@@ -113,92 +170,18 @@ __global__ void __launch_bounds__(TG_THREADS, 2) tall_gemm_kernel(const Cx<T> *M
 template <typename T>
 void tall_gemm(cudaStream_t st, int sm_count, const Cx<T> *M, int64_t ld, int rows, int K, const double *X, double *Y,
                int R, double alpha) {
-    constexpr int KC = TgChunk<T>::KC;
-    const size_t smem = sizeof(Cx<T>) * TG_THREADS * (KC + 1) + sizeof(double2) * KC * TG_RC;
-    BB_CUDA(cudaFuncSetAttribute(tall_gemm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int row_tiles = (rows + TG_THREADS - 1) / TG_THREADS;
-    // K slices so that about two CTAs per SM run
-    int slices = std::max(1, (2 * sm_count + row_tiles / 2) / row_tiles);
-    int kslice = (K + slices - 1) / slices;
-    kslice = (kslice + KC - 1) / KC * KC;
-    slices = (K + kslice - 1) / kslice;
-    for (int r0 = 0; r0 < R; r0 += TG_RC)
-        tall_gemm_kernel<T><<<dim3(row_tiles, slices), TG_THREADS, smem, st>>>(
-            M, ld, rows, K, reinterpret_cast<const double2 *>(X), reinterpret_cast<double2 *>(Y), R, r0, alpha, kslice);
-    BB_CUDA(cudaGetLastError());
+    tall_product<T, false>(st, sm_count, M, ld, rows, K, X, Y, R, alpha);
 }
 template void tall_gemm<float>(cudaStream_t, int, const Cx<float> *, int64_t, int, int, const double *, double *, int,
                                double);
 template void tall_gemm<double>(cudaStream_t, int, const Cx<double> *, int64_t, int, int, const double *, double *,
                                 int, double);
 
-// ---------------------------------------------------------------------------
-// Conjugate-transposed tall product Y += alpha M^H X: M complex row-major
-// rows x cols, X FP64 column-major rows x R, Y FP64 column-major cols x R.
-// One thread per column of M (consecutive threads read consecutive entries of
-// a row), all TG_RC right-hand sides in FP64 registers, rows of X staged
-// through shared memory; row slices add into Y with FP64 atomics.  Used by
-// the adjoint (B^H, and A^H inside the adjoint refinement).
-// ---------------------------------------------------------------------------
-constexpr int TGH_KC = 32;
-
-template <typename T>
-__global__ void __launch_bounds__(TG_THREADS, 2) tall_gemm_h_kernel(const Cx<T> *M, int64_t ld, int rows, int cols,
-                                                                    const double2 *X, double2 *Y, int R, int r0,
-                                                                    double alpha, int islice) {
-    __shared__ double2 sX[TGH_KC][TG_RC];
-    const int j = blockIdx.x * TG_THREADS + (int)threadIdx.x;
-    const int ib = blockIdx.y * islice, ie = min(rows, ib + islice);
-    const int rc = min(TG_RC, R - r0);
-    double ar[TG_RC], ai[TG_RC];
-#pragma unroll
-    for (int e = 0; e < TG_RC; ++e) ar[e] = ai[e] = 0.0;
-    for (int i0 = ib; i0 < ie; i0 += TGH_KC) {
-        const int kn = min(TGH_KC, ie - i0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < TGH_KC * TG_RC; t += TG_THREADS) {
-            const int cidx = t / TGH_KC, k = t % TGH_KC;
-            sX[k][cidx] = (cidx < rc && k < kn) ? X[(size_t)(r0 + cidx) * rows + i0 + k] : make_double2(0, 0);
-        }
-        __syncthreads();
-        if (j < cols) {
-#pragma unroll 4
-            for (int k = 0; k < kn; ++k) {
-                const Cx<T> m = M[(int64_t)(i0 + k) * ld + j];
-                const double mr = (double)m.re, mi = -(double)m.im;  // conj(M[i][j])
-#pragma unroll
-                for (int e = 0; e < TG_RC; ++e) {
-                    const double2 x = sX[k][e];
-                    ar[e] = fma(mr, x.x, fma(-mi, x.y, ar[e]));
-                    ai[e] = fma(mr, x.y, fma(mi, x.x, ai[e]));
-                }
-            }
-        }
-    }
-    if (j < cols) {
-#pragma unroll
-        for (int e = 0; e < TG_RC; ++e)
-            if (e < rc) {
-                double2 *y = &Y[(size_t)(r0 + e) * cols + j];
-                atomicAdd(&y->x, alpha * ar[e]);
-                atomicAdd(&y->y, alpha * ai[e]);
-            }
-    }
-}
-
+// Y += alpha * M^H X (the adjoint: B^H, and A^H inside its refinement)
 template <typename T>
 void tall_gemm_h(cudaStream_t st, int sm_count, const Cx<T> *M, int64_t ld, int rows, int cols, const double *X,
                  double *Y, int R, double alpha) {
-    const int col_tiles = (cols + TG_THREADS - 1) / TG_THREADS;
-    int slices = std::max(1, (2 * sm_count + col_tiles / 2) / col_tiles);
-    int islice = (rows + slices - 1) / slices;
-    islice = (islice + TGH_KC - 1) / TGH_KC * TGH_KC;
-    slices = (rows + islice - 1) / islice;
-    for (int r0 = 0; r0 < R; r0 += TG_RC)
-        tall_gemm_h_kernel<T><<<dim3(col_tiles, slices), TG_THREADS, 0, st>>>(
-            M, ld, rows, cols, reinterpret_cast<const double2 *>(X), reinterpret_cast<double2 *>(Y), R, r0, alpha,
-            islice);
-    BB_CUDA(cudaGetLastError());
+    tall_product<T, true>(st, sm_count, M, ld, cols, rows, X, Y, R, alpha);
 }
 template void tall_gemm_h<float>(cudaStream_t, int, const Cx<float> *, int64_t, int, int, const double *, double *,
                                  int, double);

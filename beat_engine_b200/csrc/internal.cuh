@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -291,6 +292,25 @@ void lu_solve_fp64(beat_b200_ctx *c, int R, double *x_dev);          // in place
 void lu_precond_fp32(beat_b200_ctx *c, int R, const double *in, double *out);
 void lu_adjoint_prepare(beat_b200_ctx *c);  // the adjoint solves' blocks, after a factorisation
 void lu_solve_adjoint(beat_b200_ctx *c, int R, const double *in, double *out);  // out = A^-H in (stored factors)
+
+// Chunks of a sum per slice of a grid of `tiles` x slices CTAs, `cap` of them
+// resident at a time: the cut whose waves have the largest useful share (a
+// finer one has to gain 2 %), slices of `least` chunks and up, four waves at most.
+inline int chunks_per_slice(int tiles, int chunks, int64_t cap, int least) {
+    const int most = (int)std::min<int64_t>(std::max(1, chunks / least), std::max<int64_t>(1, 4 * cap / tiles));
+    int best = std::max(1, chunks);
+    double best_use = 0;
+    for (int n = 1; n <= most; ++n) {
+        const int per = (chunks + n - 1) / n, parts = (chunks + per - 1) / per;
+        const int64_t waves = ((int64_t)tiles * parts + cap - 1) / cap;
+        const double use = (double)tiles * chunks / ((double)waves * cap * per);
+        if (use > best_use * 1.02) {
+            best = per;
+            best_use = use;
+        }
+    }
+    return best;
+}
 
 // gmres.cu: Y += alpha * M X (M complex row-major rows x K, X/Y FP64 column-major)
 template <typename T>
