@@ -961,6 +961,105 @@ static void update_setup() {
 }
 
 // ---------------------------------------------------------------------------
+// FP64 U12 = L11^-1 A12 on the FP64 tensor cores: one warp solves 8 columns on
+// its own (no block barrier), 16 rows at a time: C fragments start as A12, minus
+// L_s,<s X_<s with L's fragments read through L1 and X from the warp's shared
+// memory, then times the diagonal block's inverse D_s (its upper half is not
+// read).  The next block's rows and this block's D are on their way meanwhile.
+// X rows of 10 entries keep a quarter-warp's fragment loads on distinct banks.
+// Bound: the warp's own chain, 1,152 products for 128 rows (16 cycles each on a
+// sub-core, 9.5 us), two warps per sub-core at 9,000 columns.
+// 128 rows x 9,120 columns: 16 columns per CTA with FP64 FMA from shared memory
+// and its barriers took 168 us, this 30.  The next panel's 128 columns, on the
+// critical path, stay with trsm_narrow_kernel, whose chain is shorter (24 us
+// against 31 here) at the price of whole SMs.
+// ---------------------------------------------------------------------------
+constexpr int TS_COLS = 8, TS_LD = 10;
+static size_t trsm_mma_smem(int nb, int warps) { return sizeof(double2) * (size_t)nb * TS_LD * warps; }
+__global__ void __launch_bounds__(128, 2) trsm_mma_kernel(Cx<double> *A_, int64_t ld, int k, int S, const Cx<double> *D_,
+                                                         int c_begin, int c_end) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double2 *A = reinterpret_cast<double2 *>(A_);
+    const double2 *D = reinterpret_cast<const double2 *>(D_);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int c0 = c_begin + (blockIdx.x * (blockDim.x >> 5) + warp) * TS_COLS;
+    if (c0 >= c_end) return;
+    double2 *X = reinterpret_cast<double2 *>(smem_raw) + (size_t)warp * S * 16 * TS_LD;
+    double2 v[2][2];
+    auto fetch = [&](int s) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = c0 + 2 * t + e;
+                v[i][e] = c < c_end ? A[(int64_t)(k + 16 * s + 8 * i + g) * ld + c] : make_double2(0.0, 0.0);
+            }
+    };
+    fetch(0);
+    for (int s = 0; s < S; ++s) {
+        double cr[2][2], ci[2][2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                cr[i][e] = v[i][e].x;
+                ci[i][e] = v[i][e].y;
+            }
+        if (s + 1 < S) fetch(s + 1);
+        double2 d[2][4];  // D_s: rows 8 i + g, columns 4 j + t, zero above the diagonal
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2 + 2 * i; ++j)
+                d[i][j] = 4 * j + t <= 8 * i + g ? __ldg(&D[(size_t)s * 256 + (8 * i + g) * 16 + 4 * j + t])
+                                                 : make_double2(0.0, 0.0);
+        const double2 *L0 = A + (int64_t)(k + 16 * s + g) * ld + k + t, *L1 = L0 + 8 * ld;
+#pragma unroll 4
+        for (int q = 0; q < 16 * s; q += 4) {
+            const double2 l0 = __ldg(L0 + q), l1 = __ldg(L1 + q), b = X[(q + t) * TS_LD + g];
+            dmma884(cr[0], -l0.x, b.x);
+            dmma884(ci[0], -l0.x, b.y);
+            dmma884(cr[1], -l1.x, b.x);
+            dmma884(ci[1], -l1.x, b.y);
+            dmma884(cr[0], l0.y, b.y);
+            dmma884(ci[0], -l0.y, b.x);
+            dmma884(cr[1], l1.y, b.y);
+            dmma884(ci[1], -l1.y, b.x);
+        }
+        double2 *Xs = X + 16 * s * TS_LD;
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) Xs[(8 * i + g) * TS_LD + 2 * t + e] = make_double2(cr[i][e], ci[i][e]);
+        __syncwarp();
+        double yr[2][2] = {}, yi[2][2] = {};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const double2 b = Xs[(4 * j + t) * TS_LD + g];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                if (j >= 2 + 2 * i) continue;
+                dmma884(yr[i], d[i][j].x, b.x);
+                dmma884(yi[i], d[i][j].x, b.y);
+                dmma884(yr[i], -d[i][j].y, b.y);
+                dmma884(yi[i], d[i][j].y, b.x);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const double2 y = make_double2(yr[i][e], yi[i][e]);
+                Xs[(8 * i + g) * TS_LD + 2 * t + e] = y;
+                const int c = c0 + 2 * t + e;
+                if (c < c_end) A[(int64_t)(k + 16 * s + 8 * i + g) * ld + c] = y;
+            }
+        __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------
 // FP32 update inside a panel, after each of its sub-panels: C[row0.., col0 ..
 // col_end) -= L U with L = A[r, k:k+kk], U = A[k:k+kk, c], kk <= 32.  The
 // update is 32, 64 or 96 columns wide, so the tiles are 128 x 32 complex: the
@@ -1799,7 +1898,11 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
     if (wide)
         BB_CUDA(cudaFuncSetAttribute(trsm_narrow_kernel<T, WF, NCS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)trsm_narrow_smem<T, WF, NCS>(nb / W)));
-    if (sizeof(T) == 8) update_setup();
+    if (sizeof(T) == 8) {
+        update_setup();
+        BB_CUDA(cudaFuncSetAttribute(trsm_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)trsm_mma_smem(nb, 4)));
+    }
     c->barrier.alloc(sizeof(unsigned) * 4096);
     BB_CUDA(cudaFuncSetAttribute(panel_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
     // the unblocked U12 solve (used only when the blocked one does not apply)
@@ -1835,6 +1938,15 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
         __half *bhi = nullptr, *blo = nullptr;
         float *bsc = nullptr;
         if (fused_stage) tc_stage_u_buffers(c, k, nb, &bhi, &blo, &bsc);
+        if constexpr (sizeof(T) == 8) {
+            if (blocked && !(crit && narrow)) {
+                constexpr int per = 4 * TS_COLS;
+                trsm_mma_kernel<<<(cols + per - 1) / per, 128, trsm_mma_smem(nb, 4), st>>>(
+                    A, ld, k, nb / W, dinv + (size_t)(k / W) * W * W, c_lo, c_hi);
+                BB_CUDA(cudaGetLastError());
+                return;
+            }
+        }
         if (crit && narrow)
             trsm_narrow_kernel<T, WF><<<(cols + NC - 1) / NC, 256, trsm_narrow_smem<T, WF>(nb / W), st>>>(
                 A, ld, k, nb / W, dinv + (size_t)(k / W) * W * W, c_lo, c_hi, bhi, blo, bsc, k + nb, split_terms);
