@@ -806,21 +806,22 @@ __global__ void __launch_bounds__(256, 2) gemm_update_kernel(Cx<T> *A, int64_t l
 // 2 (lane % 4) + 0, 1).
 //
 // The accumulators start as C, loaded while the first chunks of L and U are on
-// their way; K goes in chunks of 8 through a ring of DU_ST cp.async stages, one
-// barrier per chunk.  Complex entries stay interleaved (a fragment's real and
-// imaginary part are one 16-byte load); row strides of 4 mod 8 (L) and 2 mod 8
-// (U) entries keep a quarter-warp's loads on distinct banks.
+// their way; K goes in chunks of 8 through DU_ST cp.async stages, one barrier
+// per chunk.  Complex entries stay interleaved (a fragment's real and imaginary
+// part are one 16-byte load); row strides of 4 mod 8 (L) and 2 mod 8 (U)
+// entries keep a quarter-warp's loads on distinct banks.
 //
-// Two shapes of four warps: 64 x 64 tiles (32 x 32 complex per warp, 128
-// registers of sums, two CTAs per SM: one's barriers and ends lie beside the
-// other's products; one CTA of 128 x 64 measured 27.1 TFLOP/s, chunks of 16
-// 28.4), and 64 x 32 (16 x 32 per warp) where the larger would leave the last
-// wave of SMs mostly idle (launch_update).
-// Bound: the FP64 tensor cores (37 TFLOP/s measured with mma.sync alone).  64 x
-// 64 tiles staged through registers, two barriers per 16 columns and C read at
-// the end reached 22 TFLOP/s on the largest updates, these 29.7.
+// Tiles of 64 x 32, four warps of 32 x 16 complex (64 registers of sums), four
+// CTAs per SM: what holds the pipe back is the start and the end of each tile
+// (C's latency, the first chunk, the stores), and with 16 warps in four places
+// the others' products cover them.  m x m updates of K = 128 at m = 10,114 /
+// 5,000 / 2,500, TFLOP/s of the 37 measured with mma.sync alone: two CTAs of
+// 64 x 64 (32 x 32 per warp, 4 stages) 29.7 / 28.1 / 27.0 (two warps per
+// scheduler, the pipe 80 % busy); 64 x 48, 3 CTAs, 3 stages 31.2 / 29.1; these
+// with 3 CTAs and 4 stages 30.3 / 27.5, with 4 and 2 32.8 / 31.8 / 29.1; 32 x 32,
+// 8 CTAs 32.8 / 32.2 at twice the reads of L; 5 CTAs no more.
 // ---------------------------------------------------------------------------
-constexpr int DU_K = 8, DU_ST = 4;
+constexpr int DU_K = 8, DU_ST = 2, DU_M = 64, DU_N = 32, DU_THREADS = 128;
 
 __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -834,40 +835,34 @@ __device__ __forceinline__ void cp_async16_zfill(double2 *smem, const double2 *g
                  : "memory");
 }
 
-template <int BM, int BN, int WM, int WN> struct DmmaTile {
-    static constexpr int THREADS = 32 * (BM / WM) * (BN / WN);
-    static constexpr int LDA = DU_K + 4, LDB = BN + 2;  // complex entries
-    static constexpr int STAGE = BM * LDA + DU_K * LDB;
-    static constexpr size_t SMEM = sizeof(double2) * DU_ST * STAGE;
-};
-template <int BM, int BN, int WM, int WN>
-__global__ void __launch_bounds__(DmmaTile<BM, BN, WM, WN>::THREADS, BN == 64 ? 2 : 3)
+constexpr int DU_LDA = DU_K + 4, DU_LDB = DU_N + 2, DU_STAGE = DU_M * DU_LDA + DU_K * DU_LDB;  // complex entries
+constexpr size_t DU_SMEM = sizeof(double2) * DU_ST * DU_STAGE;
+__global__ void __launch_bounds__(DU_THREADS, 4)
     dmma_update_kernel(Cx<double> *A_, int64_t ld, int n, int k, int kk, int row0, int col0, int col_end) {
-    using DT = DmmaTile<BM, BN, WM, WN>;
-    constexpr int THREADS = DT::THREADS, LDA = DT::LDA, LDB = DT::LDB, MI = WM / 8, NJ = WN / 8;
+    constexpr int WM = 32, WN = 16, MI = WM / 8, NJ = WN / 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2 *ring = reinterpret_cast<double2 *>(smem_raw);
     double2 *A = reinterpret_cast<double2 *>(A_);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    const int r0 = row0 + blockIdx.y * BM, c0 = col0 + blockIdx.x * BN;
-    const int wr = (warp / (BN / WN)) * WM, wc = (warp % (BN / WN)) * WN;
+    const int r0 = row0 + blockIdx.y * DU_M, c0 = col0 + blockIdx.x * DU_N;
+    const int wr = (warp / (DU_N / WN)) * WM, wc = (warp % (DU_N / WN)) * WN;
     const int nk = (kk + DU_K - 1) / DU_K;
-    auto load = [&](int kt) {  // chunk kt of L (BM x DU_K) and U (DU_K x BN)
+    auto load = [&](int kt) {  // chunk kt of L (DU_M x DU_K) and U (DU_K x DU_N)
         if (kt < nk) {
-            double2 *sl = ring + (kt % DU_ST) * DT::STAGE, *su = sl + BM * LDA;
+            double2 *sl = ring + (kt % DU_ST) * DU_STAGE, *su = sl + DU_M * DU_LDA;
             const int kc = kt * DU_K;
-            static_assert(BM * DU_K % THREADS == 0 && BN * DU_K % THREADS == 0, "whole rounds of copies");
+            static_assert(DU_M * DU_K % DU_THREADS == 0 && DU_N * DU_K % DU_THREADS == 0, "whole rounds of copies");
 #pragma unroll
-            for (int u = 0; u < BM * DU_K / THREADS; ++u) {
-                const int i = (tid + u * THREADS) / DU_K, q = tid % DU_K;
+            for (int u = 0; u < DU_M * DU_K / DU_THREADS; ++u) {
+                const int i = (tid + u * DU_THREADS) / DU_K, q = tid % DU_K;
                 const bool in = r0 + i < n && kc + q < kk;
-                cp_async16_zfill(&sl[i * LDA + q], in ? &A[(int64_t)(r0 + i) * ld + k + kc + q] : A, in);
+                cp_async16_zfill(&sl[i * DU_LDA + q], in ? &A[(int64_t)(r0 + i) * ld + k + kc + q] : A, in);
             }
 #pragma unroll
-            for (int u = 0; u < BN * DU_K / THREADS; ++u) {
-                const int q = (tid + u * THREADS) / BN, j = tid % BN;
+            for (int u = 0; u < DU_N * DU_K / DU_THREADS; ++u) {
+                const int q = (tid + u * DU_THREADS) / DU_N, j = (tid + u * DU_THREADS) % DU_N;
                 const bool in = c0 + j < col_end && kc + q < kk;
-                cp_async16_zfill(&su[q * LDB + j], in ? &A[(int64_t)(k + kc + q) * ld + c0 + j] : A, in);
+                cp_async16_zfill(&su[q * DU_LDB + j], in ? &A[(int64_t)(k + kc + q) * ld + c0 + j] : A, in);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -890,14 +885,14 @@ __global__ void __launch_bounds__(DmmaTile<BM, BN, WM, WN>::THREADS, BN == 64 ? 
         asm volatile("cp.async.wait_group %0;" ::"n"(DU_ST - 2) : "memory");
         __syncthreads();  // chunk kt is in; every warp is done with chunk kt - 1, whose place the next load takes
         load(kt + DU_ST - 1);
-        const double2 *sl = ring + (kt % DU_ST) * DT::STAGE, *su = sl + BM * LDA;
+        const double2 *sl = ring + (kt % DU_ST) * DU_STAGE, *su = sl + DU_M * DU_LDA;
 #pragma unroll
         for (int k4 = 0; k4 < DU_K; k4 += 4) {
             double2 a[MI], b[NJ];
 #pragma unroll
-            for (int i = 0; i < MI; ++i) a[i] = sl[(wr + 8 * i + g) * LDA + k4 + t];
+            for (int i = 0; i < MI; ++i) a[i] = sl[(wr + 8 * i + g) * DU_LDA + k4 + t];
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) b[j] = su[(k4 + t) * LDB + wc + 8 * j + g];
+            for (int j = 0; j < NJ; ++j) b[j] = su[(k4 + t) * DU_LDB + wc + 8 * j + g];
 #pragma unroll
             for (int i = 0; i < MI; ++i) {
                 const double nr = -a[i].x, ni = -a[i].y;
@@ -934,19 +929,8 @@ static void launch_update(beat_b200_ctx *c, cudaStream_t st, Cx<T> *A, int64_t l
     const int rows = n - row0, cols = col_end - col0;
     if (rows <= 0 || cols <= 0) return;
     if constexpr (sizeof(T) == 8) {
-        auto launch = [&](auto *kernel, int bm, int bn, int threads, size_t smem) {
-            kernel<<<dim3((cols + bn - 1) / bn, (rows + bm - 1) / bm), threads, smem, st>>>(A, ld, n, k, kk, row0,
-                                                                                            col0, col_end);
-        };
-        // the large tile while there are eight waves of it, so that an uneven
-        // last wave costs little; below, tiles of half the size even out the
-        // SMs (at 2,500 x 2,500 both reach 27 TFLOP/s)
-        using Big = DmmaTile<64, 64, 32, 32>;
-        using Small = DmmaTile<64, 32, 16, 32>;
-        if ((int64_t)((cols + 63) / 64) * ((rows + 63) / 64) >= 16 * c->sm_count)
-            launch(dmma_update_kernel<64, 64, 32, 32>, 64, 64, Big::THREADS, Big::SMEM);
-        else
-            launch(dmma_update_kernel<64, 32, 16, 32>, 64, 32, Small::THREADS, Small::SMEM);
+        dmma_update_kernel<<<dim3((cols + DU_N - 1) / DU_N, (rows + DU_M - 1) / DU_M), DU_THREADS, DU_SMEM, st>>>(
+            A, ld, n, k, kk, row0, col0, col_end);
     } else {
         gemm_update_kernel<T><<<dim3((cols + GT - 1) / GT, (rows + GT - 1) / GT), 256, 0, st>>>(A, ld, n, k, kk, row0,
                                                                                                col0, col_end);
@@ -954,10 +938,7 @@ static void launch_update(beat_b200_ctx *c, cudaStream_t st, Cx<T> *A, int64_t l
     BB_CUDA(cudaGetLastError());
 }
 static void update_setup() {
-    BB_CUDA(cudaFuncSetAttribute(dmma_update_kernel<64, 64, 32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)DmmaTile<64, 64, 32, 32>::SMEM));
-    BB_CUDA(cudaFuncSetAttribute(dmma_update_kernel<64, 32, 16, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)DmmaTile<64, 32, 16, 32>::SMEM));
+    BB_CUDA(cudaFuncSetAttribute(dmma_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DU_SMEM));
 }
 
 // ---------------------------------------------------------------------------
