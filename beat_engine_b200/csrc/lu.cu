@@ -11,17 +11,17 @@
 // interchanges are then contiguous copies.
 //
 // Per panel of nb columns:
-//   1. panel_kernel: a cooperative kernel; the panel rows are split over the
-//      CTAs and held in shared memory.  Per column every CTA publishes its
-//      best candidate row and record, passes one grid-wide barrier (an
-//      arrival counter), reads all records at once, picks the same winner,
-//      swaps and eliminates locally.  Slots are double-buffered by column
-//      parity so one barrier per column suffices.
-//   2. laswp_kernel: the panel's interchanges on all other columns (and on
-//      the running row permutation).
-//   3. trsm_kernel: U12 = L11^-1 A12.
-//   4. trailing update A22 -= L21 U12: SIMT complex GEMM here (FP64 form),
-//      tcgen05 FP16-split tensor-core GEMM for the FP32 form (tc_gemm.cu).
+//   1. cluster_panel_kernel: a thread-block cluster factors each sub-panel (32
+//      FP32 or 16 FP64 columns), its rows in registers, one exchange per column
+//      (panel_kernel, a cooperative kernel with one grid-wide barrier per
+//      column, where the rows do not fit a cluster), then the rest of the
+//      panel is solved and updated.
+//   2. laswp_panel_kernel: the panel's interchanges on all other columns (and
+//      on the running row permutation).
+//   3. U12 = L11^-1 A12 (trsm_narrow_kernel, trsm_blocked_kernel; the FP64
+//      form's trailing columns trsm_mma_kernel).
+//   4. trailing update A22 -= L21 U12: FP64 tensor cores (dmma_update_kernel), or
+//      tcgen05 FP16-split products in the FP32 form (tc_gemm.cu).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -249,37 +249,6 @@ template <typename T> __global__ void __launch_bounds__(PANEL_THREADS) panel_ker
     for (int i = tid; i < nrows * nb; i += PANEL_THREADS) {
         const int r = i / nb, c = i % nb;
         a.A[(int64_t)(gr0 + r) * a.ld + a.k + c] = P[i];
-    }
-}
-
-// row interchanges of one panel on all columns outside it; the extra
-// "column" -1 applies them to the running permutation perm[]
-template <typename T>
-__global__ void laswp_kernel(Cx<T> *A, int64_t ld, int n, int k, int nb, const int *ipiv, int *perm) {
-    __shared__ int sp[256];
-    for (int j = threadIdx.x; j < nb; j += blockDim.x) sp[j] = ipiv[k + j];
-    __syncthreads();
-    const int c = (int)(blockIdx.x * blockDim.x + threadIdx.x) - 1;
-    const int jmax = min(nb, n - k);
-    if (c == -1) {
-        for (int j = 0; j < jmax; ++j) {
-            const int p = sp[j];
-            if (p > k + j && p < n) {
-                const int t = perm[k + j];
-                perm[k + j] = perm[p];
-                perm[p] = t;
-            }
-        }
-        return;
-    }
-    if (c >= n || (c >= k && c < k + nb)) return;
-    for (int j = 0; j < jmax; ++j) {
-        const int p = sp[j];
-        if (p > k + j && p < n) {  // an interchange always names a later row
-            const Cx<T> t = A[(int64_t)(k + j) * ld + c];
-            A[(int64_t)(k + j) * ld + c] = A[(int64_t)p * ld + c];
-            A[(int64_t)p * ld + c] = t;
-        }
     }
 }
 
@@ -1874,10 +1843,10 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
     if (narrow)
         BB_CUDA(cudaFuncSetAttribute(trsm_narrow_kernel<T, WF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)trsm_narrow_smem<T, WF>(nb / W)));
-    // the side stream's solve of the remaining columns: the same kernel with 16 columns per CTA
-    // (two entries per thread in FP32), two CTAs per SM
+    // the FP32 form's solve of the remaining columns on the side stream: the same kernel with 16 columns
+    // per CTA (two entries per thread), two CTAs per SM (FP64: trsm_mma_kernel)
     constexpr int NCS = NC > 16 ? NC : 16;
-    const bool wide = blocked && trsm_narrow_smem<T, WF, NCS>(nb / W) <= 110 * 1024;
+    const bool wide = sizeof(T) == 4 && blocked && trsm_narrow_smem<T, WF, NCS>(nb / W) <= 110 * 1024;
     if (wide)
         BB_CUDA(cudaFuncSetAttribute(trsm_narrow_kernel<T, WF, NCS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)trsm_narrow_smem<T, WF, NCS>(nb / W)));
