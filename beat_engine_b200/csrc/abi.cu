@@ -64,17 +64,6 @@ beat_b200_opts resolve_opts(const beat_b200_opts *o) {
     return r;
 }
 
-// Options of a single solve: the default panel is 32 columns wide up to 3,072
-// unknowns, where the pivot chain is all of the factorisation and a panel of one
-// sub-panel saves its inner updates (N = 150 to 3,408: mixed 4-6 %, FP64 2-7 %
-// faster than 128); from 4,500 on the wide panel's updates win, and in a sweep,
-// whose lanes fill the GPU, they do from about 3,000.
-beat_b200_opts resolve_solve_opts(const beat_b200_ctx *c, const beat_b200_opts *o) {
-    beat_b200_opts r = resolve_opts(o);
-    if ((!o || o->lu_block <= 0) && c->V <= 3072) r.lu_block = 32;
-    return r;
-}
-
 // the right-hand-side mode the flags request (BEAT_B200_RHS_*)
 static int rhs_request(const beat_b200_opts &o) {
     if (o.flags & BEAT_B200_FLAG_RHS_MATRIX_FREE) return BEAT_B200_RHS_MATRIX_FREE;
@@ -499,7 +488,7 @@ int32_t beat_b200_solve_device(beat_b200_ctx *c, double k, double eta, int32_t R
                                const beat_b200_opts *opts, void *d_p, beat_b200_diag *diag) {
     return guarded(c, [&] {
         BB_REQUIRE(d_q && d_p, BEAT_B200_INVALID_ARG, "null device pointer");
-        const beat_b200_opts o = resolve_solve_opts(c, opts);
+        const beat_b200_opts o = resolve_opts(opts);
         solve_core(c, k, eta, R, (const double *)d_q, o, (double *)d_p, diag);
     });
 }
@@ -509,7 +498,7 @@ int32_t beat_b200_solve(beat_b200_ctx *c, double k, double eta, int32_t R, const
     return guarded(c, [&] {
         BB_REQUIRE(q && p_out && R >= 1, BEAT_B200_INVALID_ARG, "null pointer or R < 1");
         BB_REQUIRE(c->F > 0, BEAT_B200_STATE, "no mesh: call beat_b200_set_mesh first");
-        const beat_b200_opts o = resolve_solve_opts(c, opts);
+        const beat_b200_opts o = resolve_opts(opts);
         c->ws.lu_valid = 0;  // the workspace may change below; solve_core sets it once the factors are good
         ensure_workspace(c, o.precision, R, rhs_request(o));
         Workspace &w = c->ws;

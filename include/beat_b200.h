@@ -62,7 +62,7 @@ typedef struct {
     int32_t lu_split_terms; /* split products per trailing update: 3 (FP16 high x high + high x low +
                                low x high, about FP32 accuracy) or 1 (FP16 high parts only) (3) */
     double ir_rtol;         /* relative residual target of the refinement (1e-10) */
-    int32_t lu_block;       /* LU panel width; 0 = tuned default (by size, 32 or 128) */
+    int32_t lu_block;       /* LU panel width; 0 = tuned default */
     int32_t flags;          /* BEAT_B200_FLAG_* bits, 0 by default */
     int32_t sweep_lanes;    /* solve lanes of a sweep (1..16); 0 = default: 6 in the mixed
                                form, 4 in FP64 (always capped by free device memory) */
