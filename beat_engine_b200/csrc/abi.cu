@@ -114,7 +114,7 @@ void solve_core(beat_b200_ctx *c, double k, double eta, int R, const double *d_q
     BB_CUDA(cudaEventRecord(c->ev[4], c->stream));
     lu_factor(c, o.precision, o.lu_block, o.lu_split_terms);
     BB_CUDA(cudaEventRecord(c->ev[5], c->stream));
-    queue_status(c, 0);
+    keep_status(c);
     c->last_k = k;
     c->last_eta = eta;
     IrResult ir{0, 1, 0.0};
@@ -132,11 +132,10 @@ void solve_core(beat_b200_ctx *c, double k, double eta, int R, const double *d_q
             ir = gmres_refine(c, R, d_x, w.b.as<double>(), o.ir_restart, o.ir_max_iters, o.ir_rtol);
         BB_CUDA(cudaEventRecord(c->ev[7], c->stream));
     }
-    queue_status(c, 1);
-    BB_CUDA(cudaStreamSynchronize(c->stream));
+    const int st = read_status(c);
     check_factor_status(c);
     w.lu_valid = 1;
-    BB_REQUIRE(!(c->h_status[1] & DEV_BARRIER_TIMEOUT), BEAT_B200_TIMEOUT,
+    BB_REQUIRE(!(st & DEV_BARRIER_TIMEOUT), BEAT_B200_TIMEOUT,
                "triangular solve: a block wait ran out of its budget");
     assembly_times(c, &ms_asm, &ms_sing, &ms_reg);
     BB_CUDA(cudaEventElapsedTime(&ms_lu, c->ev[4], c->ev[5]));
@@ -424,8 +423,6 @@ int32_t beat_b200_create(int32_t device, beat_b200_ctx **out) {
         BB_CUDA(cudaEventCreateWithFlags(&c->la_fork, cudaEventDisableTiming));
         BB_CUDA(cudaEventCreateWithFlags(&c->la_join, cudaEventDisableTiming));
         for (auto &e : c->ev) BB_CUDA(cudaEventCreate(&e));
-        BB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&c->h_status), beat_b200_ctx::HOST_PIN, cudaHostAllocDefault));
-        c->h_status[0] = c->h_status[1] = 0;
         c->status.alloc(256);
         BB_CUDA(cudaMemset(c->status.p, 0, 256));
         c->barrier.alloc(sizeof(unsigned) * 4096);
@@ -462,7 +459,6 @@ int32_t beat_b200_destroy(beat_b200_ctx *c) {
     }
     for (auto &e : c->ev)
         if (e) cudaEventDestroy(e);
-    if (c->h_status) cudaFreeHost(c->h_status);
     if (c->side_stream) cudaStreamSynchronize(c->side_stream);
     for (cudaEvent_t e : {c->la_fork, c->la_join})
         if (e) cudaEventDestroy(e);

@@ -807,21 +807,21 @@ int64_t device_bytes(const beat_b200_ctx *c) {
     return s;
 }
 
-void queue_status(beat_b200_ctx *c, int slot) {
-    BB_CUDA(cudaMemcpyAsync(&c->h_status[slot], c->status.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+void keep_status(beat_b200_ctx *c) {
+    int *w = c->status.as<int>();
+    BB_CUDA(cudaMemcpyAsync(w + 1, w, sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
 }
 
 void check_factor_status(const beat_b200_ctx *c) {
-    const int st = c->h_status[0];
+    const int st = c->h_status[1];
     BB_REQUIRE(!(st & DEV_BARRIER_TIMEOUT), BEAT_B200_TIMEOUT, "LU panel: grid barrier ran out of its wait budget");
     BB_REQUIRE(!(st & DEV_ZERO_PIVOT), BEAT_B200_SINGULAR, "LU: exact zero pivot (singular system)");
 }
 
 int read_status(beat_b200_ctx *c) {
-    int s = 0;
-    BB_CUDA(cudaMemcpyAsync(&s, c->status.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    BB_CUDA(cudaMemcpyAsync(c->h_status, c->status.p, sizeof(c->h_status), cudaMemcpyDeviceToHost, c->stream));
     BB_CUDA(cudaStreamSynchronize(c->stream));
-    return s;
+    return c->h_status[0];
 }
 
 }  // namespace bb

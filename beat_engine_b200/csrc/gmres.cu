@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 #include <complex>
+#include <cstring>
 #include <vector>
 
 #include "internal.cuh"
@@ -319,12 +320,11 @@ static IrResult gmres_t(beat_b200_ctx *c, int R, double *x_dev, const double *b_
     const unsigned blocks_nr = (unsigned)((vs + th - 1) / th);
 
     std::vector<double> bnorm(R), res(R, 1.0);
-    // read-backs: pinned words of the context, or a vector when they do not fit
-    const size_t pinned = (beat_b200_ctx::HOST_PIN - 16) / sizeof(double2);
-    std::vector<double2> spill((size_t)(m + 2) * R > pinned ? (size_t)(m + 2) * R : 0);
-    double2 *hbuf = spill.empty() ? reinterpret_cast<double2 *>(c->h_status + 4) : spill.data();
-    // norms of b and of the first residual: one wait
+    std::vector<double2> hbuf((size_t)(m + 2) * R);
+    // norms of b and of the first residual, and the status word after the
+    // factorisation queued before this refinement: one wait
     col_norm2_kernel<<<R, 256, 0, c->stream>>>(reinterpret_cast<const double2 *>(b_dev), n, R, dH + R);
+    if (!ADJ) BB_CUDA(cudaMemcpyAsync(dH + 2 * R, status_kept(c), sizeof(int), cudaMemcpyDeviceToDevice, c->stream));
 
     int iters = 0;
     bool converged = false;
@@ -337,10 +337,14 @@ static IrResult gmres_t(beat_b200_ctx *c, int R, double *x_dev, const double *b_
         matvec<T, ADJ>(c, A, x_dev, reinterpret_cast<double *>(W), R, -1.0, 1.0);
         col_norm2_kernel<<<R, 256, 0, c->stream>>>(W, n, R, dH);
         const bool first = iters == 0;
-        BB_CUDA(cudaMemcpyAsync(hbuf, dH, sizeof(double2) * R * (first ? 2 : 1), cudaMemcpyDeviceToHost, c->stream));
+        BB_CUDA(cudaMemcpyAsync(hbuf.data(), dH, sizeof(double2) * (first ? 2 * R + (ADJ ? 0 : 1) : R),
+                                cudaMemcpyDeviceToHost, c->stream));
         BB_CUDA(cudaStreamSynchronize(c->stream));
         if (first) {
-            if (!ADJ) check_factor_status(c);  // of the factorisation queued before this refinement
+            if (!ADJ) {
+                std::memcpy(&c->h_status[1], &hbuf[2 * R], sizeof(int));
+                check_factor_status(c);
+            }
             for (int r = 0; r < R; ++r) bnorm[r] = std::sqrt(hbuf[R + r].x);
         }
         std::vector<double> beta(R), sc(R);
@@ -373,7 +377,7 @@ static IrResult gmres_t(beat_b200_ctx *c, int R, double *x_dev, const double *b_
                 block_axpy_kernel<<<blocks_nr, th, 0, c->stream>>>(V, vs, j + 1, W, n, R, dH, dH2);
             }
             col_norm2_kernel<<<R, 256, 0, c->stream>>>(W, n, R, dH2 + (size_t)(j + 1) * R);
-            BB_CUDA(cudaMemcpyAsync(hbuf, dH2, sizeof(double2) * (size_t)(j + 2) * R, cudaMemcpyDeviceToHost,
+            BB_CUDA(cudaMemcpyAsync(hbuf.data(), dH2, sizeof(double2) * (size_t)(j + 2) * R, cudaMemcpyDeviceToHost,
                                     c->stream));
             BB_CUDA(cudaStreamSynchronize(c->stream));
             bool all_ok = true;
@@ -433,7 +437,7 @@ static IrResult gmres_t(beat_b200_ctx *c, int R, double *x_dev, const double *b_
         BB_CUDA(cudaMemcpyAsync(W, b_dev, sizeof(double2) * vs, cudaMemcpyDeviceToDevice, c->stream));
         matvec<T, ADJ>(c, A, x_dev, reinterpret_cast<double *>(W), R, -1.0, 1.0);
         col_norm2_kernel<<<R, 256, 0, c->stream>>>(W, n, R, dH);
-        BB_CUDA(cudaMemcpyAsync(hbuf, dH, sizeof(double2) * R, cudaMemcpyDeviceToHost, c->stream));
+        BB_CUDA(cudaMemcpyAsync(hbuf.data(), dH, sizeof(double2) * R, cudaMemcpyDeviceToHost, c->stream));
         BB_CUDA(cudaStreamSynchronize(c->stream));
         converged = true;
         for (int r = 0; r < R; ++r) {

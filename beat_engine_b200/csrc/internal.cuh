@@ -230,10 +230,7 @@ struct beat_b200_ctx {
 
     int64_t regular_pairs = 0;
     bb::DevBuf status;            // device status word(s)
-    // pinned host words: the status after the factorisation and at the end of a
-    // solve, then HOST_PIN - 16 bytes for the refinement's small read-backs
-    static constexpr size_t HOST_PIN = 65536;
-    int *h_status = nullptr;
+    int h_status[2] = {0, 0};     // as last read: at the end of a solve, after its factorisation
     bb::DevBuf barrier;           // grid-barrier counters
     bb::Workspace ws;
 
@@ -269,9 +266,11 @@ int rhs_use_operator(int mode, int excitations, int64_t matrix_bytes, int64_t op
 void release_workspace(beat_b200_ctx *c);
 int64_t device_bytes(const beat_b200_ctx *c);
 int read_status(beat_b200_ctx *c);
-// queues a copy of the status word to h_status[slot]; after a synchronisation,
-// check_factor_status raises what slot 0 (after the factorisation) reports
-void queue_status(beat_b200_ctx *c, int slot);
+// keeps the status word as it stands at this point of the stream (word 1, read
+// with word 0 by read_status; status_kept: its address); check_factor_status
+// raises what h_status[1] reports
+void keep_status(beat_b200_ctx *c);
+inline const int *status_kept(const beat_b200_ctx *c) { return static_cast<const int *>(c->status.p) + 1; }
 void check_factor_status(const beat_b200_ctx *c);
 
 // assembly.cu: rule tables in constant memory (fixed per rule size)
