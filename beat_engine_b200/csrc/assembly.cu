@@ -663,12 +663,16 @@ __global__ void __launch_bounds__(SymTile<T>::THREADS, 2) sym_pairs_kernel(RegAr
 // With x = x0 + xi e1 + eta e2 on the test face and y = y0 + xi' f1 + eta' f2 on
 // the trial face, every basis product is a combination of 1, xi, eta times 1,
 // xi', eta'; so a point adds the kernel value times those nine monomials, and
-// the nine basis products follow once per pair.  r . n of either face needs only
-// the other face's coordinates.  The rule's points are stored coordinate by
-// coordinate (coalesced), and the 26 sums are reduced over the lanes by
-// halving: each exchange step also halves the number of sums a lane carries.
-// Bound: the FP64 units, about 100 instructions per point (1.1 ms at F =
-// 20,480); @SING@.
+// the nine basis products follow once per pair.  r = y - x is formed from the
+// two points' own offsets, so that exchanging them in a face's pair with itself
+// only changes its sign, and r . n from r: a rounding error common to all points
+// (of n . e1, say, where r . n should vanish) would be weighted by 1 / r^3
+// (right-hand sides at F = 320: 5.0e-15 with r . n from such constants, 3.8e-16).
+// The rule's points are stored coordinate by coordinate (coalesced), and the 26
+// sums are reduced over the lanes by halving: each exchange step also halves
+// the number of sums a lane carries.
+// Bound: the FP64 units, about 105 instructions per point (1.2 ms at F =
+// 20,480, 2.22 measured; 2.23 with nine products and 26 butterfly sums a point).
 // ---------------------------------------------------------------------------
 template <typename T> struct SingArgs {
     const int *test, *trial, *rule;
@@ -708,13 +712,12 @@ __device__ __forceinline__ double warp_sum32(double (&v)[32]) {
 // against the test monomials, acc[24]: Green sum
 __device__ __forceinline__ void singular_point(double xi, double et, double yi, double ye, const double (&d0)[3],
                                                const double (&e1)[3], const double (&e2)[3], const double (&f1)[3],
-                                               const double (&f2)[3], double ns0, double nse1, double nse2, double nt0,
-                                               double ntf1, double ntf2, double w, double k, double eta, double k2n,
-                                               double (&acc)[32]) {
+                                               const double (&f2)[3], const double (&ns)[3], const double (&nt)[3],
+                                               double w, double k, double eta, double k2n, double (&acc)[32]) {
     double r[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
-        r[c] = fma(yi, f1[c], fma(ye, f2[c], fma(-xi, e1[c], fma(-et, e2[c], d0[c]))));
+        r[c] = fma(yi, f1[c], fma(ye, f2[c], d0[c])) - fma(xi, e1[c], et * e2[c]);
     const double r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
     if (r2 == 0.0) return;
     const double ir = rsqrt_series(r2);
@@ -723,8 +726,8 @@ __device__ __forceinline__ void singular_point(double xi, double et, double yi, 
     const double scl = ir * w;
     const double gr = cs_ * scl, gi = sn_ * scl;
     const double hr = (-gr * ir - gi * k) * ir, hi = (gr * k - gi * ir) * ir;  // dG/dr / r
-    const double rns = fma(-xi, nse1, fma(-et, nse2, ns0));                    // r . n_s
-    const double rnt = fma(yi, ntf1, fma(ye, ntf2, nt0));                      // r . n_t
+    const double rns = fma(r[0], ns[0], fma(r[1], ns[1], r[2] * ns[2]));
+    const double rnt = fma(r[0], nt[0], fma(r[1], nt[1], r[2] * nt[2]));
     const double lr = k2n * gi - hr * rns, li = -(hi * rns + k2n * gr);
     const double pt = eta * rnt;
     const double rr = -gr - hi * pt, ri = hr * pt - gi;
@@ -764,7 +767,7 @@ __global__ void __launch_bounds__(256, 2) singular_pairs_kernel(SingArgs<T> g) {
     if (pair >= g.npairs) return;
     const int t = g.test[pair], s = g.trial[pair], r = g.rule[pair];
     const int *ft = g.faces + 3 * t, *fs = g.faces + 3 * s;
-    double d0[3], e1[3], e2[3], f1[3], f2[3], ns0 = 0, nse1 = 0, nse2 = 0, nt0 = 0, ntf1 = 0, ntf2 = 0;
+    double d0[3], e1[3], e2[3], f1[3], f2[3], ns[3], nt[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const double x0 = g.verts[3 * ft[0] + c], y0 = g.verts[3 * fs[0] + c];
@@ -773,14 +776,8 @@ __global__ void __launch_bounds__(256, 2) singular_pairs_kernel(SingArgs<T> g) {
         f1[c] = g.verts[3 * fs[1] + c] - y0;
         f2[c] = g.verts[3 * fs[2] + c] - y0;
         d0[c] = y0 - x0;
-        // y - y0 is orthogonal to n_s, x - x0 to n_t
-        const double ns = g.normals[3 * s + c], nt = g.normals[3 * t + c];
-        ns0 += d0[c] * ns;
-        nse1 += e1[c] * ns;
-        nse2 += e2[c] * ns;
-        nt0 += d0[c] * nt;
-        ntf1 += f1[c] * nt;
-        ntf2 += f2[c] * nt;
+        ns[c] = g.normals[3 * s + c];
+        nt[c] = g.normals[3 * t + c];
     }
     const double k = g.k, eta = g.eta;
     const double k2n = eta * (k * k * g.nn[pair]);
@@ -791,8 +788,8 @@ __global__ void __launch_bounds__(256, 2) singular_pairs_kernel(SingArgs<T> g) {
     const double *rd = g.rule_data;
     const int64_t np = g.npoints;
     for (int q = g.rule_start[r] + lane; q < q1; q += 32)
-        singular_point(rd[q], rd[np + q], rd[2 * np + q], rd[3 * np + q], d0, e1, e2, f1, f2, ns0, nse1, nse2, nt0,
-                       ntf1, ntf2, 0.07957747154594767 * rd[4 * np + q], k, eta, k2n, acc);
+        singular_point(rd[q], rd[np + q], rd[2 * np + q], rd[3 * np + q], d0, e1, e2, f1, f2, ns, nt,
+                       0.07957747154594767 * rd[4 * np + q], k, eta, k2n, acc);
     const double mine = warp_sum32(acc);  // lane i: sum i
     // the basis products: phi_0 = 1 - phi_1 - phi_2 on either face
     const double jac = g.jac[pair];

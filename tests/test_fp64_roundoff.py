@@ -1,0 +1,41 @@
+"""Round-off of the FP64 form on a B200.
+
+u = 2^-53.  A stage that sums small terms apart before it adds them to what is
+large, and whose rounding errors have no common sign, stays within a few u of
+its exact result at these sizes; the bounds below are that, not the parity
+tests' 1e-11, which would hide the loss of three digits.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from beat_engine_b200 import _lib
+from beat_engine_b200 import mesh as M
+
+pytestmark = pytest.mark.gpu
+U = 2.0 ** -53
+
+
+def _complex(rng, *shape):
+    return rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+
+
+def _distance(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+@pytest.mark.parametrize("mode, bound", [("off", 10), ("x", 30)])
+def test_right_hand_side(mode, bound):
+    """Most of a right-hand side's entry comes from the touching pairs of its
+    own faces.  Twice the oracle's own error, which in long double arithmetic is
+    5 u here and 16 u with the image's pairs."""
+    mesh = M.reference_sphere(0.1, 2) if mode == "off" else M.uv_sphere_patch(0.1, 12, 12, -np.pi / 2, np.pi / 2)
+    k = 20.0
+    q = _complex(np.random.default_rng(1), mesh.num_faces, 1)
+    _, bo = (oracle.assemble(mesh, k, 1.0 / k, q) if mode == "off" else
+             oracle.assemble_sym(mesh, k, 1.0 / k, q, mode))
+    with _lib.Context(0) as c:
+        c.set_symmetry(mode)
+        c.set_mesh(mesh.vertices, mesh.faces, 4, 4)
+        _, b = c.assemble(k, 1.0 / k, q, _lib.FP64, want_matrix=False)
+    assert _distance(b, bo) <= bound * U
