@@ -769,20 +769,24 @@ __global__ void __launch_bounds__(256, 2) gemm_update_kernel(Cx<T> *A, int64_t l
 // ---------------------------------------------------------------------------
 // FP64 tensor-core (DMMA) complex GEMM for the FP64 form's updates:
 // C[r0.., c0..] -= L U, 8 x 8 complex blocks by mma.sync.m8n8k4.f64 (4 real
-// products per complex block: re -= Lr Ur - Li Ui, im -= Lr Ui + Li Ur, the
-// signs on the L fragments).  Fragments (PTX ISA, m8n8k4 .f64): A a0 at
+// products per complex block: re += Lr Ur - Li Ui, im += Lr Ui + Li Ur, the
+// sign on the L fragment).  Fragments (PTX ISA, m8n8k4 .f64): A a0 at
 // (lane / 4, lane % 4); B b0 at (lane % 4, lane / 4); C c0, c1 at (lane / 4,
 // 2 (lane % 4) + 0, 1).
 //
-// The accumulators start as C, loaded while the first chunks of L and U are on
-// their way; K goes in chunks of 8 through DU_ST cp.async stages, one barrier
-// per chunk.  Complex entries stay interleaved (a fragment's real and imaginary
+// L U is summed apart and subtracted from C once, so that an entry takes one
+// rounding at its own magnitude per panel instead of two per index: with C as
+// the accumulators' start the solutions' error at N = 998 / 2,616 / 10,242 was
+// 2.0 / 2.8 / 5.0e-15, so it is 4.4 / 4.6 / 7.9e-16 (the three kernels that
+// eliminate, together; LU at N = 10,242 104.5 -> 104.7 ms, N = 2,616 7.75 ->
+// 7.90).  K goes in chunks of 8 through DU_ST cp.async stages, one barrier per
+// chunk.  Complex entries stay interleaved (a fragment's real and imaginary
 // part are one 16-byte load); row strides of 4 mod 8 (L) and 2 mod 8 (U)
 // entries keep a quarter-warp's loads on distinct banks.
 //
 // Tiles of 64 x 32, four warps of 32 x 16 complex (64 registers of sums), four
 // CTAs per SM: what holds the pipe back is the start and the end of each tile
-// (C's latency, the first chunk, the stores), and with 16 warps in four places
+// (the first chunk, C's latency, the stores), and with 16 warps in four places
 // the others' products cover them.  m x m updates of K = 128 at m = 10,114 /
 // 5,000 / 2,500, TFLOP/s of the 37 measured with mma.sync alone: two CTAs of
 // 64 x 64 (32 x 32 per warp, 4 stages) 29.7 / 28.1 / 27.0 (two warps per
@@ -840,18 +844,7 @@ __global__ void __launch_bounds__(DU_THREADS, 4)
     };
 #pragma unroll
     for (int s = 0; s < DU_ST - 1; ++s) load(s);
-    double cr[MI][NJ][2], ci[MI][NJ][2];  // [row block][column block][fragment]
-#pragma unroll
-    for (int i = 0; i < MI; ++i)
-#pragma unroll
-        for (int j = 0; j < NJ; ++j)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int r = r0 + wr + 8 * i + g, c = c0 + wc + 8 * j + 2 * t + e;
-                const double2 v = (r < n && c < col_end) ? __ldcs(&A[(int64_t)r * ld + c]) : make_double2(0.0, 0.0);
-                cr[i][j][e] = v.x;
-                ci[i][j][e] = v.y;
-            }
+    double cr[MI][NJ][2] = {}, ci[MI][NJ][2] = {};  // [row block][column block][fragment]: L U
     for (int kt = 0; kt < nk; ++kt) {
         asm volatile("cp.async.wait_group %0;" ::"n"(DU_ST - 2) : "memory");
         __syncthreads();  // chunk kt is in; every warp is done with chunk kt - 1, whose place the next load takes
@@ -866,30 +859,40 @@ __global__ void __launch_bounds__(DU_THREADS, 4)
             for (int j = 0; j < NJ; ++j) b[j] = su[(k4 + t) * DU_LDB + wc + 8 * j + g];
 #pragma unroll
             for (int i = 0; i < MI; ++i) {
-                const double nr = -a[i].x, ni = -a[i].y;
+                const double ni = -a[i].y;
                 // (2 NJ products between the two that add to one block)
 #pragma unroll
                 for (int j = 0; j < NJ; ++j) {
-                    dmma884(cr[i][j], nr, b[j].x);
-                    dmma884(ci[i][j], nr, b[j].y);
+                    dmma884(cr[i][j], a[i].x, b[j].x);
+                    dmma884(ci[i][j], a[i].x, b[j].y);
                 }
 #pragma unroll
                 for (int j = 0; j < NJ; ++j) {
-                    dmma884(cr[i][j], a[i].y, b[j].y);
-                    dmma884(ci[i][j], ni, b[j].x);
+                    dmma884(cr[i][j], ni, b[j].y);
+                    dmma884(ci[i][j], a[i].y, b[j].x);
                 }
             }
         }
     }
 #pragma unroll
-    for (int i = 0; i < MI; ++i)
+    for (int i = 0; i < MI; ++i) {
+        double2 v[NJ][2];
 #pragma unroll
         for (int j = 0; j < NJ; ++j)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int r = r0 + wr + 8 * i + g, c = c0 + wc + 8 * j + 2 * t + e;
-                if (r < n && c < col_end) __stcs(&A[(int64_t)r * ld + c], make_double2(cr[i][j][e], ci[i][j][e]));
+                v[j][e] = (r < n && c < col_end) ? __ldcs(&A[(int64_t)r * ld + c]) : make_double2(0.0, 0.0);
             }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = r0 + wr + 8 * i + g, c = c0 + wc + 8 * j + 2 * t + e;
+                if (r < n && c < col_end)
+                    __stcs(&A[(int64_t)r * ld + c], make_double2(v[j][e].x - cr[i][j][e], v[j][e].y - ci[i][j][e]));
+            }
+    }
 }
 
 // the trailing / in-panel update C -= L U, L = A[row0.., k..k+kk), U = A[k..k+kk,
@@ -914,10 +917,11 @@ static void update_setup() {
 
 // ---------------------------------------------------------------------------
 // FP64 U12 = L11^-1 A12 on the FP64 tensor cores: one warp solves 8 columns on
-// its own (no block barrier), 16 rows at a time: C fragments start as A12, minus
-// L_s,<s X_<s with L's fragments read through L1 and X from the warp's shared
-// memory, then times the diagonal block's inverse D_s (its upper half is not
-// read).  The next block's rows and this block's D are on their way meanwhile.
+// its own (no block barrier), 16 rows at a time: A12 minus L_s,<s X_<s (summed
+// apart, as in the update) with L's fragments read through L1 and X from the
+// warp's shared memory, then times the diagonal block's inverse D_s (its upper
+// half is not read).  The next block's rows and this block's D are on their way
+// meanwhile.
 // X rows of 10 entries keep a quarter-warp's fragment loads on distinct banks.
 // Bound: the warp's own chain, 1,152 products for 128 rows (16 cycles each on a
 // sub-core, 9.5 us), two warps per sub-core at 9,000 columns.
@@ -949,14 +953,12 @@ __global__ void __launch_bounds__(128, 2) trsm_mma_kernel(Cx<double> *A_, int64_
     };
     fetch(0);
     for (int s = 0; s < S; ++s) {
-        double cr[2][2], ci[2][2];
+        double2 b0[2][2];
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                cr[i][e] = v[i][e].x;
-                ci[i][e] = v[i][e].y;
-            }
+            for (int e = 0; e < 2; ++e) b0[i][e] = v[i][e];
+        double cr[2][2] = {}, ci[2][2] = {};  // L_s,<s X_<s
         if (s + 1 < S) fetch(s + 1);
         double2 d[2][4];  // D_s: rows 8 i + g, columns 4 j + t, zero above the diagonal
 #pragma unroll
@@ -969,20 +971,21 @@ __global__ void __launch_bounds__(128, 2) trsm_mma_kernel(Cx<double> *A_, int64_
 #pragma unroll 4
         for (int q = 0; q < 16 * s; q += 4) {
             const double2 l0 = __ldg(L0 + q), l1 = __ldg(L1 + q), b = X[(q + t) * TS_LD + g];
-            dmma884(cr[0], -l0.x, b.x);
-            dmma884(ci[0], -l0.x, b.y);
-            dmma884(cr[1], -l1.x, b.x);
-            dmma884(ci[1], -l1.x, b.y);
-            dmma884(cr[0], l0.y, b.y);
-            dmma884(ci[0], -l0.y, b.x);
-            dmma884(cr[1], l1.y, b.y);
-            dmma884(ci[1], -l1.y, b.x);
+            dmma884(cr[0], l0.x, b.x);
+            dmma884(ci[0], l0.x, b.y);
+            dmma884(cr[1], l1.x, b.x);
+            dmma884(ci[1], l1.x, b.y);
+            dmma884(cr[0], -l0.y, b.y);
+            dmma884(ci[0], l0.y, b.x);
+            dmma884(cr[1], -l1.y, b.y);
+            dmma884(ci[1], l1.y, b.x);
         }
         double2 *Xs = X + 16 * s * TS_LD;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) Xs[(8 * i + g) * TS_LD + 2 * t + e] = make_double2(cr[i][e], ci[i][e]);
+            for (int e = 0; e < 2; ++e)
+                Xs[(8 * i + g) * TS_LD + 2 * t + e] = make_double2(b0[i][e].x - cr[i][e], b0[i][e].y - ci[i][e]);
         __syncwarp();
         double yr[2][2] = {}, yi[2][2] = {};
 #pragma unroll
@@ -1246,6 +1249,16 @@ __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsig
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
+__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long f2_add(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 __device__ __forceinline__ ColPair<float> pair_ld(const unsigned char *p, float) {
     const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(p);
     return ColPair<float>{v.x, v.y};
@@ -1280,18 +1293,21 @@ __device__ __forceinline__ ColMult<float> pair_mult(Cx<float> l) {
     return ColMult<float>{f2_pack(-l.re, -l.re), f2_pack(l.im, l.im), f2_pack(-l.im, -l.im)};
 }
 __device__ __forceinline__ ColMult<double> pair_mult(Cx<double> l) { return ColMult<double>{l.re, l.im}; }
-// x - l u
+// x - l u, the product apart: one rounding at the entry's magnitude.  (Two fused
+// steps on x round there twice: unrefined FP32 solutions at 82 to 2,524 unknowns
+// were 2 to 9 % less exact; LU 2.48 -> 2.50 ms at N = 1,390.)
 __device__ __forceinline__ ColPair<float> pair_cms(const ColPair<float> &x, const ColMult<float> &l,
                                                    const ColPair<float> &u) {
-    return ColPair<float>{f2_fma(l.i, u.im, f2_fma(l.nr, u.re, x.re)), f2_fma(l.ni, u.re, f2_fma(l.nr, u.im, x.im))};
+    return ColPair<float>{f2_add(x.re, f2_fma(l.i, u.im, f2_mul(l.nr, u.re))),
+                          f2_add(x.im, f2_fma(l.ni, u.re, f2_mul(l.nr, u.im)))};
 }
 __device__ __forceinline__ ColPair<double> pair_cms(const ColPair<double> &x, const ColMult<double> &l,
                                                     const ColPair<double> &u) {
     ColPair<double> d;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        d.re[h] = fma(l.i, u.im[h], fma(-l.r, u.re[h], x.re[h]));
-        d.im[h] = fma(-l.i, u.re[h], fma(-l.r, u.im[h], x.im[h]));
+        d.re[h] = x.re[h] + fma(l.i, u.im[h], -l.r * u.re[h]);
+        d.im[h] = x.im[h] + fma(-l.i, u.re[h], -l.r * u.im[h]);
     }
     return d;
 }
@@ -1308,7 +1324,7 @@ __device__ __forceinline__ uint4 finish16(uint4 x, const ColMult<double> &l, con
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const double xh = h ? __hiloint2double((int)x.w, (int)x.z) : __hiloint2double((int)x.y, (int)x.x);
-        v[h] = half ? fma(-l.i, u.re[h], fma(-l.r, u.im[h], xh)) : fma(l.i, u.im[h], fma(-l.r, u.re[h], xh));
+        v[h] = xh + (half ? fma(-l.i, u.re[h], -l.r * u.im[h]) : fma(l.i, u.im[h], -l.r * u.re[h]));
     }
     return make_uint4((uint32_t)__double2loint(v[0]), (uint32_t)__double2hiint(v[0]), (uint32_t)__double2loint(v[1]),
                       (uint32_t)__double2hiint(v[1]));
