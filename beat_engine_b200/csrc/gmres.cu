@@ -39,6 +39,13 @@ namespace bb {
 // two cp.async stages; rows of 2 mod 8 entries keep a quarter-warp's loads on
 // distinct banks.  The reduction is cut into slices that fill whole waves of
 // resident CTAs; they add into Y with FP64 atomics.
+//
+// An FP64 M's sums of TM_G indices are added to totals (a thread's own places in
+// shared memory) and begin again at zero: n terms with random signs in one chain
+// round like sqrt(n + K / 2n), and a whole slice as one chain gave B q an error
+// of 3.7 / 4.6 / 16e-16 at F = 636 / 1,184 / 9,064, this 2.3 / 2.4 / 3.5e-16 (one
+// column of registers per thread in shorter slices: 2.8 / 3.5 / 11e-16), for 5 %
+// of the product's time.  An FP32 M's own rounding hides the sum's.
 // Bound: M's bytes with up to 8 columns, the FP64 tensor cores with 16.
 // FP32 M, R = 16, one N x F and three N x N products with N = 10,242, F = 20,480:
 // 3.63 ms with one row and 16 columns of FP64 FMA per thread, 2.80 ms (24
@@ -53,13 +60,24 @@ __device__ __forceinline__ void tm_mma(double (&c)[2], double a, double b) {
         : "d"(a), "d"(b));
 }
 
+template <typename T, int NB> struct TallShape {
+    static constexpr bool APART = sizeof(T) == 8;  // groups of TM_G indices summed apart
+    static constexpr int XS = 8 * NB + 2;
+    static constexpr size_t STAGES = sizeof(double2) * 2 * TM_KC * XS;
+    static constexpr size_t SMEM = STAGES + (APART ? sizeof(double2) * 2 * TM_MB * NB * TM_WARPS * 32 : 0);
+};
+
 // no outputs, reduction length K: M is no x K (row-major, H = false) or K x no (H = true)
 template <typename T, bool H, int NB>
 __global__ void __launch_bounds__(TM_WARPS * 32, 2) tall_mma_kernel(const Cx<T> *M, int64_t ld, int no, int K,
                                                                     const double2 *X, double2 *Y, int R, int r0,
                                                                     double alpha, int kslice) {
-    constexpr int COLS = 8 * NB, XS = COLS + 2, STEPS = TM_G / 4;
-    __shared__ __align__(16) double2 sX[2][TM_KC * XS];
+    using TS = TallShape<T, NB>;
+    constexpr int COLS = 8 * NB, XS = TS::XS, STEPS = TM_G / 4, THREADS = TM_WARPS * 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    auto sX = reinterpret_cast<double2(*)[TM_KC * XS]>(smem_raw);
+    // (FP64) this thread's totals: block (m, n)'s real parts at [2 (m NB + n) THREADS], the imaginary after them
+    double2 *tot = reinterpret_cast<double2 *>(smem_raw + TS::STAGES) + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = lane >> 2, q = lane & 3;
     const int kb = blockIdx.y * kslice, ke = min(K, kb + kslice);
     const int rc = min(COLS, R - r0);
@@ -93,6 +111,14 @@ __global__ void __launch_bounds__(TM_WARPS * 32, 2) tall_mma_kernel(const Cx<T> 
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     double re[TM_MB][NB][2] = {}, im[TM_MB][NB][2] = {};
+    if constexpr (TS::APART) {
+#pragma unroll
+        for (int i = 0; i < 2 * TM_MB * NB; ++i) tot[i * THREADS] = make_double2(0.0, 0.0);
+    }
+    auto add = [&](double2 &t, double (&v)[2]) {
+        t = make_double2(t.x + v[0], t.y + v[1]);
+        v[0] = v[1] = 0.0;
+    };
     stage(0, kb);
     load(cur, kb);
     int buf = 0;
@@ -125,6 +151,15 @@ __global__ void __launch_bounds__(TM_WARPS * 32, 2) tall_mma_kernel(const Cx<T> 
                     }
                 }
             }
+            if constexpr (TS::APART) {
+#pragma unroll
+                for (int m = 0; m < TM_MB; ++m)
+#pragma unroll
+                    for (int n = 0; n < NB; ++n) {
+                        add(tot[2 * (m * NB + n) * THREADS], re[m][n]);
+                        add(tot[(2 * (m * NB + n) + 1) * THREADS], im[m][n]);
+                    }
+            }
 #pragma unroll
             for (int s = 0; s < STEPS; ++s)
 #pragma unroll
@@ -138,7 +173,12 @@ __global__ void __launch_bounds__(TM_WARPS * 32, 2) tall_mma_kernel(const Cx<T> 
         const int o = o0 + 8 * m;
         if (o >= no) continue;
 #pragma unroll
-        for (int n = 0; n < NB; ++n)
+        for (int n = 0; n < NB; ++n) {
+            if constexpr (TS::APART) {
+                const double2 a = tot[2 * (m * NB + n) * THREADS], b = tot[(2 * (m * NB + n) + 1) * THREADS];
+                re[m][n][0] = a.x, re[m][n][1] = a.y;
+                im[m][n][0] = b.x, im[m][n][1] = b.y;
+            }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int c = 8 * n + 2 * q + h;
@@ -147,6 +187,7 @@ __global__ void __launch_bounds__(TM_WARPS * 32, 2) tall_mma_kernel(const Cx<T> 
                 atomicAdd(&y->x, alpha * re[m][n][h]);
                 atomicAdd(&y->y, alpha * im[m][n][h]);
             }
+        }
     }
 }
 
@@ -157,11 +198,14 @@ static void tall_product(cudaStream_t st, int sm_count, const Cx<T> *M, int64_t 
     for (int r0 = 0; r0 < R; r0 += 16) {
         // 8 columns when no more are left: half the products, the same bytes of M
         const auto kernel = R - r0 <= 8 ? tall_mma_kernel<T, H, 1> : tall_mma_kernel<T, H, 2>;
+        const size_t smem = R - r0 <= 8 ? TallShape<T, 1>::SMEM : TallShape<T, 2>::SMEM;
+        if (smem > 48 * 1024)
+            BB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 1;
-        BB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, TM_WARPS * 32, 0));
+        BB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, TM_WARPS * 32, smem));
         const int per = chunks_per_slice(tiles, chunks, std::max(1, per_sm) * sm_count, 2);
         const int kslice = per * TM_KC;
-        kernel<<<dim3(tiles, (K + kslice - 1) / kslice), TM_WARPS * 32, 0, st>>>(
+        kernel<<<dim3(tiles, (K + kslice - 1) / kslice), TM_WARPS * 32, smem, st>>>(
             M, ld, no, K, reinterpret_cast<const double2 *>(X), reinterpret_cast<double2 *>(Y), R, r0, alpha, kslice);
         BB_CUDA(cudaGetLastError());
     }

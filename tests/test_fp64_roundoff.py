@@ -68,3 +68,21 @@ def test_solution(faces, lu_block):
         p, _ = c.solve(k, 1.0 / k, q, _lib.Context.opts(_lib.FP64, flags=_lib.FLAG_RHS_CACHED, lu_block=lu_block))
         A, b = c.assemble(k, 1.0 / k, q, _lib.FP64)
     assert _distance(p, _refined(A, b)) <= 8 * U
+
+
+@pytest.mark.parametrize("faces", [100, 300])
+@pytest.mark.parametrize("columns", [2, 9, 16])
+def test_mapping_times_columns(faces, columns):
+    """b = B q against the long double product with the device's own B (its
+    product with the identity is exact).  A chain of n terms of random signs,
+    then K / n such sums, have an error of sqrt(n + K / 2n) roundings in rms, of
+    u / sqrt(3) at most each; n = 16."""
+    mesh = M.rounded_box_enclosure(faces, seed=faces)
+    k, n = 20.0, mesh.num_faces
+    q = _complex(np.random.default_rng(columns), n, columns)
+    with _lib.Context(0) as c:
+        c.set_mesh(mesh.vertices, mesh.faces, 4, 4)
+        _, B = c.assemble(k, 1.0 / k, np.eye(n, dtype=np.complex128), _lib.FP64, want_matrix=False)
+        _, b = c.assemble(k, 1.0 / k, q, _lib.FP64, want_matrix=False)
+    ref = B.astype(np.clongdouble) @ q.astype(np.clongdouble)
+    assert _distance(b, ref) <= U / np.sqrt(3.0) * np.sqrt(16.0 + n / 32.0)
