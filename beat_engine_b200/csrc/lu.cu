@@ -36,12 +36,6 @@
 
 namespace bb {
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
 template <typename T> __device__ __forceinline__ T cabs1(Cx<T> v) { return fabs(v.re) + fabs(v.im); }
 // correctly rounded reciprocal (the same value as 1 / x)
 __device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
@@ -252,45 +246,13 @@ template <typename T> __global__ void __launch_bounds__(PANEL_THREADS) panel_ker
     }
 }
 
-// Row interchanges ipiv[k .. k+nsw) on the columns [c_lo, c_hi) outside
-// [x_lo, x_hi); with perm non-null, one extra thread applies them to the
-// running permutation.  (The look-ahead LU swaps a sub-panel's rows inside its
-// panel first and on the other columns once per panel.)
-template <typename T>
-__global__ void laswp_range_kernel(Cx<T> *A, int64_t ld, int n, int k, int nsw, const int *ipiv, int c_lo, int c_hi,
-                                   int x_lo, int x_hi, int *perm) {
-    __shared__ int sp[256];
-    for (int j = threadIdx.x; j < nsw; j += blockDim.x) sp[j] = ipiv[k + j];
-    __syncthreads();
-    const int jmax = min(nsw, n - k);
-    const int c = c_lo - 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (c == c_lo - 1) {
-        if (!perm) return;
-        for (int j = 0; j < jmax; ++j) {
-            const int p = sp[j];
-            if (p > k + j && p < n) {
-                const int t = perm[k + j];
-                perm[k + j] = perm[p];
-                perm[p] = t;
-            }
-        }
-        return;
-    }
-    if (c >= c_hi || (c >= x_lo && c < x_hi)) return;
-    for (int j = 0; j < jmax; ++j) {
-        const int p = sp[j];
-        if (p > k + j && p < n) {  // an interchange always names a later row
-            const Cx<T> t = A[(int64_t)(k + j) * ld + c];
-            A[(int64_t)(k + j) * ld + c] = A[(int64_t)p * ld + c];
-            A[(int64_t)p * ld + c] = t;
-        }
-    }
-}
-
-// The same interchanges as laswp_range_kernel (nsw <= LS_MAX), as one
-// permutation of at most 2 nsw rows: every CTA derives the moves from ipiv,
-// then loads every moved entry of its LS_COLS columns before it stores any, so
-// no column walks a chain of dependent global loads.  With swap j exchanging
+// Row interchanges ipiv[k .. k+nsw), nsw <= LS_MAX, on the columns [c_lo, c_hi)
+// outside [x_lo, x_hi) and, with perm non-null, on the running permutation (the
+// look-ahead swaps a sub-panel's rows inside its panel first and on the other
+// columns once per panel), as one permutation of at most 2 nsw rows: every CTA
+// derives the moves from ipiv, then loads every moved entry of its LS_COLS
+// columns before it stores any, so no column walks a chain of dependent global
+// loads.  With swap j exchanging
 // positions k + j and p_j >= k + j, position k + j is final after swap j; its
 // content then is what stood at p_j just before, and
 //   X_j (the content of k + j just before swap j) = X_prevX[j], or the row k + j
@@ -317,7 +279,7 @@ __global__ void __launch_bounds__(256) laswp_panel_kernel(Cx<T> *A, int64_t ld, 
     if (tid == 0) nmove = 0;
     for (int j = tid; j < jmax; j += 256) {
         const int p = ipiv[k + j];
-        sp[j] = (p > k + j && p < n) ? p : k + j;  // out-of-range entries are no interchange, as in laswp_range_kernel
+        sp[j] = (p > k + j && p < n) ? p : k + j;  // out-of-range entries are no interchange
     }
     __syncthreads();
     int prev_x = -1, last_p = -1;
@@ -380,44 +342,6 @@ __global__ void __launch_bounds__(256) laswp_panel_kernel(Cx<T> *A, int64_t ld, 
 __global__ void iota_kernel(int *perm, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) perm[i] = i;
-}
-
-// A[k:k+kb, c_begin:c_end] = L^-1 A[...] with L = A[k:k+kb, k:k+kb] unit
-// lower (nb = allocated width of the triangle); 32 columns per CTA
-constexpr int TRSM_COLS = 32;
-template <typename T>
-__global__ void __launch_bounds__(256) trsm_kernel(Cx<T> *A, int64_t ld, int n, int k, int nb, int c_begin, int c_end) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Cx<T> *L = reinterpret_cast<Cx<T> *>(smem_raw);  // nb x nb
-    Cx<T> *X = L + nb * nb;                           // nb x TRSM_COLS
-    const int c0 = c_begin + blockIdx.x * TRSM_COLS;
-    const int nc = min(TRSM_COLS, c_end - c0);
-    const int kb = min(nb, n - k);
-    batched_copy<256, 16, Cx<T>>(
-        kb * kb, [&](int i) { return A[(int64_t)(k + i / kb) * ld + k + i % kb]; },
-        [&](int i, Cx<T> v) { L[(i / kb) * nb + i % kb] = v; });
-    batched_copy<256, 8, Cx<T>>(
-        kb * TRSM_COLS,
-        [&](int i) {
-            const int c = i % TRSM_COLS;
-            return c < nc ? A[(int64_t)(k + i / TRSM_COLS) * ld + c0 + c] : Cx<T>{T(0), T(0)};
-        },
-        [&](int i, Cx<T> v) { X[i] = v; });
-    __syncthreads();
-    for (int j = 0; j < kb - 1; ++j) {
-        for (int idx = threadIdx.x; idx < (kb - 1 - j) * TRSM_COLS; idx += blockDim.x) {
-            const int i = j + 1 + idx / TRSM_COLS, c = idx % TRSM_COLS;
-            const Cx<T> l = L[i * nb + j], x = X[j * TRSM_COLS + c];
-            Cx<T> &d = X[i * TRSM_COLS + c];
-            d.re -= l.re * x.re - l.im * x.im;
-            d.im -= l.re * x.im + l.im * x.re;
-        }
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < kb * TRSM_COLS; i += blockDim.x) {
-        const int r = i / TRSM_COLS, c = i % TRSM_COLS;
-        if (c < nc) A[(int64_t)(k + r) * ld + c0 + c] = X[r * TRSM_COLS + c];
-    }
 }
 
 // Inverse of a unit lower triangular kb x kb block (kb <= W <= 32), by one
@@ -699,74 +623,6 @@ __global__ void __launch_bounds__(256) trsm_narrow_kernel(Cx<T> *A, int64_t ld, 
 }
 
 // ---------------------------------------------------------------------------
-// SIMT complex GEMM for the trailing update: C[m0.., n0..] -= L U
-// L = A[r, k:k+kk], U = A[k:k+kk, c]; 64 x 64 output tile, 256 threads,
-// 4 x 4 complex accumulators per thread.
-// ---------------------------------------------------------------------------
-constexpr int GT = 64, GKC = 16;
-template <typename T>
-__global__ void __launch_bounds__(256, 2) gemm_update_kernel(Cx<T> *A, int64_t ld, int n, int k, int kk, int row0,
-                                                          int col0, int col_end) {
-    __shared__ Cx<T> sL[GKC][GT + 1];
-    __shared__ Cx<T> sU[GKC][GT];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int r0 = row0 + blockIdx.y * GT, c0 = col0 + blockIdx.x * GT;
-    T acc[4][4][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = T(0);
-    for (int kc = 0; kc < kk; kc += GKC) {
-        {
-            constexpr int PER = GT * GKC / 256;
-            Cx<T> vl[PER], vu[PER];
-#pragma unroll
-            for (int u = 0; u < PER; ++u) {
-                const int idx = threadIdx.x + u * 256;
-                const int i = idx / GKC, q = idx % GKC, r = r0 + i, kq = kc + q;
-                vl[u] = (r < n && kq < kk) ? A[(int64_t)r * ld + k + kq] : Cx<T>{T(0), T(0)};
-                const int q2 = idx / GT, j = idx % GT, c = c0 + j, kq2 = kc + q2;
-                vu[u] = (c < col_end && kq2 < kk) ? A[(int64_t)(k + kq2) * ld + c] : Cx<T>{T(0), T(0)};
-            }
-#pragma unroll
-            for (int u = 0; u < PER; ++u) {
-                const int idx = threadIdx.x + u * 256;
-                sL[idx % GKC][idx / GKC] = vl[u];
-                sU[idx / GT][idx % GT] = vu[u];
-            }
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int q = 0; q < GKC; ++q) {
-            Cx<T> a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = sL[q][ty + 16 * i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = sU[q][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    acc[i][j][0] += a[i].re * b[j].re - a[i].im * b[j].im;
-                    acc[i][j][1] += a[i].re * b[j].im + a[i].im * b[j].re;
-                }
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int r = r0 + ty + 16 * i, c = c0 + tx + 16 * j;
-            if (r < n && c < col_end) {
-                Cx<T> &d = A[(int64_t)r * ld + c];
-                d.re -= acc[i][j][0];
-                d.im -= acc[i][j][1];
-            }
-        }
-}
-
-// ---------------------------------------------------------------------------
 // FP64 tensor-core (DMMA) complex GEMM for the FP64 form's updates:
 // C[r0.., c0..] -= L U, 8 x 8 complex blocks by mma.sync.m8n8k4.f64 (4 real
 // products per complex block: re += Lr Ur - Li Ui, im += Lr Ui + Li Ur, the
@@ -895,20 +751,14 @@ __global__ void __launch_bounds__(DU_THREADS, 4)
     }
 }
 
-// the trailing / in-panel update C -= L U, L = A[row0.., k..k+kk), U = A[k..k+kk,
-// col0..col_end): tensor cores (DMMA) in FP64, SIMT in FP32
-template <typename T>
-static void launch_update(beat_b200_ctx *c, cudaStream_t st, Cx<T> *A, int64_t ld, int n, int k, int kk, int row0,
-                          int col0, int col_end) {
+// the FP64 form's trailing / in-panel update C -= L U, L = A[row0.., k..k+kk),
+// U = A[k..k+kk, col0..col_end)
+static void launch_update(cudaStream_t st, Cx<double> *A, int64_t ld, int n, int k, int kk, int row0, int col0,
+                          int col_end) {
     const int rows = n - row0, cols = col_end - col0;
     if (rows <= 0 || cols <= 0) return;
-    if constexpr (sizeof(T) == 8) {
-        dmma_update_kernel<<<dim3((cols + DU_N - 1) / DU_N, (rows + DU_M - 1) / DU_M), DU_THREADS, DU_SMEM, st>>>(
-            A, ld, n, k, kk, row0, col0, col_end);
-    } else {
-        gemm_update_kernel<T><<<dim3((cols + GT - 1) / GT, (rows + GT - 1) / GT), 256, 0, st>>>(A, ld, n, k, kk, row0,
-                                                                                               col0, col_end);
-    }
+    dmma_update_kernel<<<dim3((cols + DU_N - 1) / DU_N, (rows + DU_M - 1) / DU_M), DU_THREADS, DU_SMEM, st>>>(
+        A, ld, n, k, kk, row0, col0, col_end);
     BB_CUDA(cudaGetLastError());
 }
 static void update_setup() {
@@ -1020,9 +870,8 @@ __global__ void __launch_bounds__(128, 2) trsm_mma_kernel(Cx<double> *A_, int64_
 // update is 32, 64 or 96 columns wide, so the tiles are 128 x 32 complex: the
 // whole K is staged at once by the asynchronous copy unit while each thread
 // prefetches its 4 x 4 outputs, then one barrier and kk rank-1 steps from
-// shared memory.  (The square 64 x 64 tiles of gemm_update_kernel left half of
-// each tile idle on the 32-column updates and staged K in two synchronised
-// chunks.)  C never overlaps L or U: rows >= row0 > k + kk, columns >= col0.
+// shared memory.  (Square 64 x 64 tiles left half of each tile idle on the
+// 32-column updates and staged K in two synchronised chunks.)  C never overlaps L or U: rows >= row0 > k + kk, columns >= col0.
 // ---------------------------------------------------------------------------
 constexpr int PU_ROWS = 128, PU_COLS = 32, PU_K = 32;
 __global__ void __launch_bounds__(256, 2) panel_update_kernel(Cx<float> *A, int64_t ld, int n, int k, int kk, int row0,
@@ -1812,9 +1661,7 @@ static bool cluster_panel(beat_b200_ctx *c, Cx<T> *A, int64_t ld, int n, int k, 
 }
 
 // FP32 form trailing update on the tensor cores (tc_gemm.cu)
-bool tc_update_supported(int nb);
 void tc_stage_l(beat_b200_ctx *c, int k, int nb, int split_terms, cudaStream_t st);
-void tc_stage_u(beat_b200_ctx *c, int k, int nb, int split_terms, int col_lo, int col_hi, cudaStream_t st);
 void tc_stage_u_buffers(beat_b200_ctx *c, int k, int nb, __half **bhi, __half **blo, float **bscale);
 void tc_update_cols(beat_b200_ctx *c, int k, int nb, int split_terms, int col_lo, int col_hi, cudaStream_t st,
                     int max_ctas);
@@ -1836,7 +1683,8 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
                "LU: system of order " + std::to_string(n) + " exceeds the shared-memory panel limit");
     // scratch: [2][G] pivot records, [2][G][nb] candidate rows, [2][nb] diagonal rows
     // and the inverses of the sub-panels' W x W diagonal blocks
-    const int W = std::min(nb, (int)(256 / sizeof(Cx<T>)));
+    constexpr int WF = 256 / sizeof(Cx<T>), W = WF;  // a sub-panel's columns: 256-byte rows
+    BB_REQUIRE(nb % 32 == 0 && nb <= LS_MAX, BEAT_B200_INVALID_ARG, "LU: panels of 32, 64, 128 or 256 columns");
     const size_t rec_bytes = sizeof(PivotRec) * 2 * (size_t)G;
     const size_t scratch = rec_bytes + sizeof(Cx<T>) * (2 * (size_t)G * nb + 2 * nb);
     const size_t dinv_off = (scratch + 255) / 256 * 256;
@@ -1846,23 +1694,19 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
     Cx<T> *pub_rows = reinterpret_cast<Cx<T> *>(recs + 2 * G);
     Cx<T> *pub_diag = pub_rows + 2 * (size_t)G * nb;
     Cx<T> *dinv = reinterpret_cast<Cx<T> *>(w.panel_scratch.as<unsigned char>() + dinv_off);
-    // blocked U12 solves need whole W-column sub-panels of 256-byte rows
-    constexpr int WF = 256 / sizeof(Cx<T>);
-    const bool blocked = W == WF && nb % W == 0;
     const size_t tb_smem = sizeof(Cx<T>) * ((size_t)nb * TB_COLS + (size_t)W * (W + 1) + (size_t)W * (nb - W + 1));
-    if (blocked)
-        BB_CUDA(cudaFuncSetAttribute(trsm_blocked_kernel<T, WF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)tb_smem));
+    BB_CUDA(cudaFuncSetAttribute(trsm_blocked_kernel<T, WF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)tb_smem));
     // the critical-path solves take the narrow kernel when its whole triangle fits
     constexpr int NC = narrow_cols<WF>();
-    const bool narrow = blocked && trsm_narrow_smem<T, WF>(nb / W) <= 227 * 1024;
+    const bool narrow = trsm_narrow_smem<T, WF>(nb / W) <= 227 * 1024;
     if (narrow)
         BB_CUDA(cudaFuncSetAttribute(trsm_narrow_kernel<T, WF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)trsm_narrow_smem<T, WF>(nb / W)));
     // the FP32 form's solve of the remaining columns on the side stream: the same kernel with 16 columns
     // per CTA (two entries per thread), two CTAs per SM (FP64: trsm_mma_kernel)
     constexpr int NCS = NC > 16 ? NC : 16;
-    const bool wide = sizeof(T) == 4 && blocked && trsm_narrow_smem<T, WF, NCS>(nb / W) <= 110 * 1024;
+    const bool wide = sizeof(T) == 4 && trsm_narrow_smem<T, WF, NCS>(nb / W) <= 110 * 1024;
     if (wide)
         BB_CUDA(cudaFuncSetAttribute(trsm_narrow_kernel<T, WF, NCS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)trsm_narrow_smem<T, WF, NCS>(nb / W)));
@@ -1873,23 +1717,15 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
     }
     c->barrier.alloc(sizeof(unsigned) * 4096);
     BB_CUDA(cudaFuncSetAttribute(panel_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap));
-    // the unblocked U12 solve (used only when the blocked one does not apply)
-    const size_t trsm_smem = sizeof(Cx<T>) * ((size_t)nb * nb + (size_t)nb * TRSM_COLS);
-    if (!blocked) {
-        BB_REQUIRE(trsm_smem <= 227 * 1024, BEAT_B200_INVALID_ARG,
-                   "LU: lu_block " + std::to_string(nb) + " is too wide for the unblocked U12 solve");
-        BB_CUDA(cudaFuncSetAttribute(trsm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)trsm_smem));
-    }
     constexpr int LC = ls_cols<T>();
     BB_CUDA(cudaFuncSetAttribute(laswp_panel_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)laswp_panel_smem<T>(std::min(nb, LS_MAX))));
+                                 (int)laswp_panel_smem<T>(nb)));
     iota_kernel<<<(n + 255) / 256, 256, 0, c->stream>>>(w.perm.as<int>(), n);
     BB_CUDA(cudaMemsetAsync(c->status.p, 0, sizeof(int), c->stream));
-    const size_t trsm_w_smem = sizeof(Cx<T>) * ((size_t)W * W + (size_t)W * TRSM_COLS);
     int *ipiv = w.ipiv.as<int>();
     int *perm = w.perm.as<int>();
     cudaStream_t s0 = c->stream, s1 = c->side_stream;
-    const bool tc = sizeof(T) == 4 && tc_update_supported(nb);
+    constexpr bool tc = sizeof(T) == 4;  // the tensor-core update (K = 2 nb, a multiple of its 64)
     // SMs the look-ahead update leaves to the panel factorisation beside it: one
     // 16-CTA cluster, and as many again for the panel's own updates and solves
     // between its sub-panels (measured at N = 10,242: mixed LU 46.4 ms with one
@@ -1897,17 +1733,16 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
     // the grid-wide panel fallback waits for its own SMs
     const int side_cap = std::max(1, G - 2 * CP_CTAS);
     // U12 = L11^-1 A12 of panel k for the columns [c_lo, c_hi), on stream st
-    // with the tensor-core update (blocked) the same launch stages U12 as the update's B operand
-    const bool fused_stage = tc && blocked;
+    // with the tensor-core update the same launch stages U12 as the update's B operand
     // (crit: the next panel's columns, on the critical path)
     auto u_solve = [&](int k, int c_lo, int c_hi, cudaStream_t st, bool crit) {
         const int cols = c_hi - c_lo;
         if (cols <= 0) return;
         __half *bhi = nullptr, *blo = nullptr;
         float *bsc = nullptr;
-        if (fused_stage) tc_stage_u_buffers(c, k, nb, &bhi, &blo, &bsc);
+        if (tc) tc_stage_u_buffers(c, k, nb, &bhi, &blo, &bsc);
         if constexpr (sizeof(T) == 8) {
-            if (blocked && !(crit && narrow)) {
+            if (!(crit && narrow)) {
                 constexpr int per = 4 * TS_COLS;
                 trsm_mma_kernel<<<(cols + per - 1) / per, 128, trsm_mma_smem(nb, 4), st>>>(
                     A, ld, k, nb / W, dinv + (size_t)(k / W) * W * W, c_lo, c_hi);
@@ -1921,24 +1756,18 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
         else if (wide)
             trsm_narrow_kernel<T, WF, NCS><<<(cols + NCS - 1) / NCS, 256, trsm_narrow_smem<T, WF, NCS>(nb / W), st>>>(
                 A, ld, k, nb / W, dinv + (size_t)(k / W) * W * W, c_lo, c_hi, bhi, blo, bsc, k + nb, split_terms);
-        else if (blocked)
+        else
             trsm_blocked_kernel<T, WF><<<(cols + TB_COLS - 1) / TB_COLS, 256, tb_smem, st>>>(
                 A, ld, k, nb / W, dinv + (size_t)(k / W) * W * W, c_lo, c_hi, bhi, blo, bsc, k + nb, split_terms);
-        else
-            trsm_kernel<T><<<(cols + TRSM_COLS - 1) / TRSM_COLS, 256, trsm_smem, st>>>(A, ld, n, k, nb, c_lo, c_hi);
         BB_CUDA(cudaGetLastError());
     };
     // A[k+nb.., c_lo..c_hi) -= L21 U12 of panel k, on stream st
     auto update = [&](int k, int c_lo, int c_hi, cudaStream_t st, int cap) {
         if (c_hi <= c_lo || k + nb >= n) return;
-        if (tc) {
-            if (!fused_stage) tc_stage_u(c, k, nb, split_terms, c_lo, c_hi, st);
+        if constexpr (tc)
             tc_update_cols(c, k, nb, split_terms, c_lo, c_hi, st, cap);
-        } else {
-            // one CTA per tile: capping this grid as the tensor-core one is capped
-            // measured slower at N = 10,242 (154 against 136 ms for the FP64 LU)
-            launch_update<T>(c, st, A, ld, n, k, nb, k + nb, c_lo, c_hi);
-        }
+        else  // one CTA per tile: a grid capped as the tensor-core one is was slower (154 against 136 ms a factorisation)
+            launch_update(st, A, ld, n, k, nb, k + nb, c_lo, c_hi);
     };
     // Right-looking LU with a look-ahead of one panel.  For panel k (columns
     // [k, pe)):
@@ -1957,7 +1786,7 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
         const int pe = std::min(k + nb, n);  // end of this panel
         for (int ks = k; ks < pe; ks += W) {
             const int m = n - ks;
-            Cx<T> *dinv_s = blocked ? dinv + (size_t)(ks / W) * W * W : nullptr;
+            Cx<T> *dinv_s = dinv + (size_t)(ks / W) * W * W;
             // the cluster kernel also swaps the panel's other columns when they fit its registers
             constexpr int CHUNK = 16 / sizeof(Cx<T>);
             const int right = std::max(0, pe - ks - W), others = ks - k + right;
@@ -1990,15 +1819,11 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
             }
             // this sub-panel's interchanges on the rest of the panel (unless the cluster kernel did them)
             if (others > 0 && !(on_cluster && own_swaps)) {
-                if (W <= LS_MAX)
-                    laswp_panel_kernel<T><<<(pe - k + LC - 1) / LC, 256, laswp_panel_smem<T>(W), s0>>>(
-                        A, ld, n, ks, W, ipiv, k, pe, ks, ks + W, nullptr);
-                else
-                    laswp_range_kernel<T><<<(pe - k + 1 + 255) / 256, 256, 0, s0>>>(A, ld, n, ks, W, ipiv, k, pe, ks,
-                                                                                    ks + W, nullptr);
+                laswp_panel_kernel<T><<<(pe - k + LC - 1) / LC, 256, laswp_panel_smem<T>(W), s0>>>(
+                    A, ld, n, ks, W, ipiv, k, pe, ks, ks + W, nullptr);
                 BB_CUDA(cudaGetLastError());
             }
-            if (blocked && !on_cluster) {
+            if (!on_cluster) {
                 diag_block_inverse_kernel<T><<<1, 32, 0, s0>>>(A, ld, n, ks, W, dinv_s);
                 BB_CUDA(cudaGetLastError());
             }
@@ -2009,17 +1834,14 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
                     trsm_narrow_kernel<T, WF><<<(cols + NC - 1) / NC, 256, trsm_narrow_smem<T, WF>(1), s0>>>(
                         A, ld, ks, 1, dinv + (size_t)(ks / W) * W * W, ks + W, pe, nullptr, nullptr, nullptr, 0,
                         split_terms);
-                else if (blocked)
+                else
                     trsm_blocked_kernel<T, WF><<<(cols + TB_COLS - 1) / TB_COLS, 256, tb_smem, s0>>>(
                         A, ld, ks, 1, dinv + (size_t)(ks / W) * W * W, ks + W, pe);
-                else
-                    trsm_kernel<T><<<(cols + TRSM_COLS - 1) / TRSM_COLS, 256, trsm_w_smem, s0>>>(
-                        A, ld, n, ks, W, ks + W, pe);
                 if constexpr (sizeof(T) == 4) {
                     dim3 grid((cols + PU_COLS - 1) / PU_COLS, (n - ks - W + PU_ROWS - 1) / PU_ROWS);
                     panel_update_kernel<<<grid, 256, 0, s0>>>(A, ld, n, ks, W, ks + W, ks + W, pe);
                 } else {
-                    launch_update<T>(c, s0, A, ld, n, ks, W, ks + W, ks + W, pe);
+                    launch_update(s0, A, ld, n, ks, W, ks + W, ks + W, pe);
                 }
                 BB_CUDA(cudaGetLastError());
             }
@@ -2029,11 +1851,8 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
             side_pending = false;
         }
         // the panel's interchanges on every column outside it, and on perm
-        if (pe - k <= LS_MAX)
-            laswp_panel_kernel<T><<<(n + LC - 1) / LC, 256, laswp_panel_smem<T>(pe - k), s0>>>(A, ld, n, k, pe - k, ipiv,
-                                                                                            0, n, k, pe, perm);
-        else
-            laswp_range_kernel<T><<<(n + 1 + 255) / 256, 256, 0, s0>>>(A, ld, n, k, pe - k, ipiv, 0, n, k, pe, perm);
+        laswp_panel_kernel<T><<<(n + LC - 1) / LC, 256, laswp_panel_smem<T>(pe - k), s0>>>(A, ld, n, k, pe - k, ipiv, 0,
+                                                                                        n, k, pe, perm);
         BB_CUDA(cudaGetLastError());
         if (pe >= n) break;
         const int ne = std::min(pe + nb, n);  // end of the next panel
@@ -2059,8 +1878,6 @@ template <typename T> static void lu_factor_t(beat_b200_ctx *c, int nb, int spli
     }
     if (side_pending) BB_CUDA(cudaStreamWaitEvent(s0, c->la_join, 0));
 }
-
-
 
 // ---------------------------------------------------------------------------
 // triangular solves with R right-hand sides (X column-major N x R, FP64)
@@ -2387,13 +2204,6 @@ __global__ void __launch_bounds__(SubstTile<SubstType<T, ADJ>, RC>::THREADS, 1)
             dst[q * XP + a] = Cx<C>{(C)v.x, (C)v.y};
         }
     };
-    // an FP64 64 x 64 block (D_b^-1 or H_b) into dst in the compute type
-    auto load_block = [&](const Cx<double> *src, Cx<C> *dst) {
-        for (int i = gt; i < SB * SB; i += 128) {
-            const Cx<double> v = src[i];
-            dst[(i / SB) * LP + i % SB] = Cx<C>{(C)v.re, (C)v.im};
-        }
-    };
     C ar[2][CT], ai[2][CT];
 #pragma unroll
     for (int h = 0; h < 2; ++h)
@@ -2431,6 +2241,7 @@ __global__ void __launch_bounds__(SubstTile<SubstType<T, ADJ>, RC>::THREADS, 1)
     // else group 0's after the D product
     Cx<C> *TH1 = NG >= 3 ? base + 2 * ST::GROUP : T0;
     Cx<C> *X0 = base + SB * LP;                // group 0's X block
+    // an FP64 64 x 64 block (D_b^-1 or H_b) into dst in the compute type
     auto load_block_all = [&](const Cx<double> *src, Cx<C> *dst) {
         for (int i = tid; i < SB * SB; i += THREADS) {
             const Cx<double> v = src[i];

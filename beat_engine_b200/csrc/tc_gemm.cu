@@ -335,8 +335,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 }
 
 // ---------------------------------------------------------------------------
-// operand staging: A_s[i][k'] = L_R rows, B_s[n][k'] = U_big columns, hi/lo
-// FP16, scaled (see the top of this file)
+// operand staging: A_s[i][k'] = L_R rows here, B_s[n][k'] = U_big columns in the
+// U12 solve (lu.cu), hi/lo FP16, scaled (see the top of this file)
 // ---------------------------------------------------------------------------
 __global__ void stage_a_kernel(const float2 *A, int64_t ld, int k, int nb, int m, __half *ahi, __half *alo,
                                int split) {
@@ -351,45 +351,6 @@ __global__ void stage_a_kernel(const float2 *A, int64_t ld, int k, int nb, int m
     split_f16(v.y * sc, hi_, li);
     reinterpret_cast<__half2 *>(ahi + (int64_t)i * 2 * nb)[kk] = __halves2half2(hr, hi_);
     if (split == 3) reinterpret_cast<__half2 *>(alo + (int64_t)i * 2 * nb)[kk] = __halves2half2(lr, li);
-}
-
-// One warp per complex column j of U12 (U12[kk][j] = A[k+kk][k+nb+j], j = j0 ..
-// j0+ncols): the column's exponent s_j from its largest |re| or |im|, then
-// rows 2j and 2j+1 of B_s get (Ur, -Ui) 2^s_j and (Ui, Ur) 2^s_j at K = 2kk,
-// and bscale[j] = 2^-(s_j + L_SHIFT).
-__global__ void stage_b_kernel(const float2 *A, int64_t ld, int k, int nb, int j0, int ncols, __half *bhi,
-                               __half *blo, float *bscale, int split) {
-    const int wi = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (wi >= ncols) return;  // whole warps
-    const int j = j0 + wi;
-    const float2 *col = A + (int64_t)k * ld + k + nb + j;
-    float mx = 0.f;
-    for (int kk = lane; kk < nb; kk += 32) {
-        const float2 u = col[(int64_t)kk * ld];
-        mx = fmaxf(mx, fmaxf(fabsf(u.x), fabsf(u.y)));
-    }
-    mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));  // non-negative: ordered as bits
-    const int sx = stage_exp(mx);
-    const float sc = pow2f(sx);
-    if (lane == 0) bscale[j] = pow2f(-sx - L_SHIFT);
-    __half2 *h0 = reinterpret_cast<__half2 *>(bhi + (int64_t)(2 * j) * 2 * nb);
-    __half2 *h1 = reinterpret_cast<__half2 *>(bhi + (int64_t)(2 * j + 1) * 2 * nb);
-    __half2 *l0 = reinterpret_cast<__half2 *>(blo + (int64_t)(2 * j) * 2 * nb);
-    __half2 *l1 = reinterpret_cast<__half2 *>(blo + (int64_t)(2 * j + 1) * 2 * nb);
-    for (int kk = lane; kk < nb; kk += 32) {
-        const float2 u = col[(int64_t)kk * ld];
-        __half er, ei, orr, oi, ler, lei, lor, loi;
-        split_f16(u.x * sc, er, ler);
-        split_f16(-u.y * sc, ei, lei);
-        split_f16(u.y * sc, orr, lor);
-        split_f16(u.x * sc, oi, loi);
-        h0[kk] = __halves2half2(er, ei);
-        h1[kk] = __halves2half2(orr, oi);
-        if (split == 3) {
-            l0[kk] = __halves2half2(ler, lei);
-            l1[kk] = __halves2half2(lor, loi);
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -481,8 +442,6 @@ static TcStage tc_stage_buffers(beat_b200_ctx *c, int k, int nb) {
     return s;
 }
 
-bool tc_update_supported(int nb) { return nb % 32 == 0; }  // K = 2 nb must be a multiple of TC_BK
-
 // Stages L21 of panel k (every row below the panel).
 void tc_stage_l(beat_b200_ctx *c, int k, int nb, int split_terms, cudaStream_t st) {
     const TcStage s = tc_stage_buffers(c, k, nb);
@@ -490,17 +449,6 @@ void tc_stage_l(beat_b200_ctx *c, int k, int nb, int split_terms, cudaStream_t s
     const int64_t na = (int64_t)s.m * nb;
     stage_a_kernel<<<(unsigned)((na + 255) / 256), 256, 0, st>>>(c->ws.A.as<float2>(), c->ws.ld, k, nb, s.m, s.ahi,
                                                                  s.alo, split_terms);
-    BB_CUDA(cudaGetLastError());
-}
-
-// Stages U12 of panel k for the columns [col_lo, col_hi) (absolute, >= k + nb),
-// which must already hold U12 = L11^-1 A12.
-void tc_stage_u(beat_b200_ctx *c, int k, int nb, int split_terms, int col_lo, int col_hi, cudaStream_t st) {
-    const TcStage s = tc_stage_buffers(c, k, nb);
-    const int nc = col_hi - col_lo;
-    if (s.m <= 0 || nc <= 0) return;
-    stage_b_kernel<<<(unsigned)(((int64_t)nc * 32 + 255) / 256), 256, 0, st>>>(
-        c->ws.A.as<float2>(), c->ws.ld, k, nb, col_lo - (k + nb), nc, s.bhi, s.blo, s.bscale, split_terms);
     BB_CUDA(cudaGetLastError());
 }
 
