@@ -16,7 +16,11 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libbeatb200.so")
 SOURCES = ["context.cu", "assembly.cu", "lu.cu", "tc_gemm.cu", "gmres.cu", "field.cu", "adjoint.cu", "coupled.cu", "shape.cu", "abi.cu",
-           "noalloc.cu"]
+           "noalloc.cu", "cluster_panel.cu"]
+HEADERS = ["internal.cuh", "phase.cuh", "lu.cuh"]
+# sources compiled several times: object name and its flags
+VARIANTS = {"cluster_panel.cu": {f"cluster_panel_{t}_{r}": [f"-DBB_T={t}", f"-DBB_ROWS={r}"]
+                                 for t in ("float", "double") for r in (1, 2, 3)}}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # per-file flags: the FP32 element-pair quadrature flushes denormals (its values
 # are nowhere near the FP32 denormal range; the FP64 paths are unaffected)
@@ -34,8 +38,7 @@ def needs_build() -> bool:
     if not os.path.exists(LIB):
         return True
     t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, s) for s in SOURCES] + [os.path.join(CSRC, "internal.cuh"), os.path.join(CSRC, "phase.cuh"),
-                                                        os.path.join(HERE, "..", "include", "beat_b200.h")]
+    deps = [os.path.join(CSRC, s) for s in SOURCES + HEADERS] + [os.path.join(HERE, "..", "include", "beat_b200.h")]
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
@@ -51,10 +54,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
     objs = []
     procs = []
     for src in SOURCES:
-        obj = os.path.join(objdir, src.replace(".cu", ".o"))
-        objs.append(obj)
-        cmd = [nvcc, *flags, *FILE_FLAGS.get(src, []), "-c", os.path.join(CSRC, src), "-o", obj]
-        procs.append((cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT)))
+        for name, extra in VARIANTS.get(src, {src.replace(".cu", ""): []}).items():
+            obj = os.path.join(objdir, name + ".o")
+            objs.append(obj)
+            cmd = [nvcc, *flags, *FILE_FLAGS.get(src, []), *extra, "-c", os.path.join(CSRC, src), "-o", obj]
+            procs.append((cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT)))
     failed = []
     for cmd, p in procs:
         out, _ = p.communicate()
