@@ -180,17 +180,21 @@ __global__ void __launch_bounds__(FLD_THREADS) field_eval_kernel(const double *p
 //     p, ip (real parts of i p), -q, -iq,   columns (re, im) of each side,
 // staged once per chunk.  So neither factors nor sums move between lanes.
 // NB: blocks of 8 real columns, 4 NB right-hand sides.  Each warp holds PG
-// groups of 8 points, so a B operand feeds PG products.
-// Bound: the FP64 units (about 45 + 32 NB FP64 instructions' worth per (point,
+// groups of 8 points.  The four products of four sources are summed from zero
+// and added to the running sum once: with the running sum as their accumulator
+// it is rounded 16 times for four sources, and the error against long double was
+// 10 % above a thread per point's (F = 11,864, 16 sides: 4.4 -> 4.9e-13; this 4.2).
+// Bound: the FP64 units (about 45 + 34 NB FP64 instructions' worth per (point,
 // source)); a thread per point with 16 sides in registers read 32 broadcast
 // 16-byte values of shared memory per source and was held by those: field at
-// 2,000 points, 16 sides, 71,184 sources 2.9 ms, this 2.05.
+// 2,000 points, 16 sides, 71,184 sources 2.9 ms, this 2.2.  Three CTAs per SM
+// with 16 sides, by registers.
 constexpr int FLD_PG = FLD_POINTS / 8;
 template <int NB> struct FieldB {
     static constexpr int LD = NB == 1 ? 8 : 8 * NB + 8;  // row stride: 8 mod 16 doubles, two wavefronts a load
 };
 template <bool FAR, int NB>
-__global__ void __launch_bounds__(FLD_THREADS) field_mma_kernel(const double *pts, int M, const double *ys,
+__global__ void __launch_bounds__(FLD_THREADS, NB == 4 ? 3 : 4) field_mma_kernel(const double *pts, int M, const double *ys,
                                                                 const double *ns, const double2 *ps,
                                                                 const double2 *qs, int S, int R, int r0, int per_cta,
                                                                 double k, double2 *out) {
@@ -243,17 +247,22 @@ __global__ void __launch_bounds__(FLD_THREADS) field_mma_kernel(const double *pt
                     for (int i = 0; i < 4; ++i) f[a][i] = 0.0;
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int b = 0; b < NB; ++b) {
+                double bv[4];
 #pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    const double bv = ch.b[i][(j0 + t) * LD + 8 * b + g];
+                for (int i = 0; i < 4; ++i) bv[i] = ch.b[i][(j0 + t) * LD + 8 * b + g];
 #pragma unroll
-                    for (int a = 0; a < FLD_PG; ++a)
-                        asm volatile(
-                            "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                            : "+d"(c[a][b][0]), "+d"(c[a][b][1])
-                            : "d"(f[a][i]), "d"(bv));
+                for (int a = 0; a < FLD_PG; ++a) {
+                    double d[2] = {0.0, 0.0};  // four sources' sum, apart from the others'
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                            : "+d"(d[0]), "+d"(d[1])
+                            : "d"(f[a][i]), "d"(bv[i]));
+                    c[a][b][0] += d[0];
+                    c[a][b][1] += d[1];
                 }
+            }
         }
     }
     // the warps' sums meet in shared memory, half of the points at a time:
@@ -341,7 +350,7 @@ static StagedSources stage_sources(beat_b200_ctx *c, int M, const double *pts_ho
 // The source range in as many parts as fill whole waves of resident CTAs best
 // (a part has at least four chunks): with 63 tiles of points and 444 CTAs
 // resident, 9 parts leave the second wave 28 % full (2.68 ms for the product
-// kernel above), 7 make one wave (2.05 ms).
+// kernel above with one running sum), 7 make one wave (2.05 ms).
 struct SourceSplit {
     dim3 grid;
     int per;  // sources per CTA

@@ -86,3 +86,36 @@ def test_mapping_times_columns(faces, columns):
         _, b = c.assemble(k, 1.0 / k, q, _lib.FP64, want_matrix=False)
     ref = B.astype(np.clongdouble) @ q.astype(np.clongdouble)
     assert _distance(b, ref) <= U / np.sqrt(3.0) * np.sqrt(16.0 + n / 32.0)
+
+
+def test_field_sums():
+    """A field whose terms all have one sign and about one size (no pressure,
+    positive Neumann data, a wavenumber near zero), at so many points that a warp
+    sums a quarter of the sources by itself: m additions to a sum that grows
+    with them have an error of sqrt(m / 3) roundings in rms relative to it, of u /
+    sqrt(3) at most each, and the four warps' errors are independent.  Four
+    sources make one addition."""
+    mesh = M.rounded_box_enclosure(5228, seed=5228)
+    S, R, k = 6 * mesh.num_faces, 16, 1e-3
+    rng = np.random.default_rng(1)
+    q = rng.uniform(0.5, 1.5, (mesh.num_faces, R)) + 0j
+    x = M.fibonacci_sphere(32 * 148 * 3, 2.0)
+    with _lib.Context(0) as c:
+        c.set_mesh(mesh.vertices, mesh.faces, 4, 4)
+        got = c.field(k, x, np.zeros((mesh.num_vertices, R), complex), q)
+    rule, w = oracle.triangle_rule(4)
+    tri = np.asarray(mesh.vertices).astype(np.longdouble)[np.asarray(mesh.faces)]
+    y = np.einsum("qa,fad->fqd", np.column_stack([1 - rule.sum(axis=1), rule]).astype(np.longdouble), tri)
+    normal = np.cross(tri[:, 1] - tri[:, 0], tri[:, 2] - tri[:, 0])
+    weight = np.sqrt((normal * normal).sum(axis=1))[:, None] * w.astype(np.longdouble)
+    at = np.arange(0, len(x), len(x) // 25)
+    ref = []
+    for m in at:
+        r = np.sqrt(((y - x[m].astype(np.longdouble)) ** 2).sum(axis=2))
+        g = weight / (4 * np.arctan2(np.longdouble(0), np.longdouble(-1)) * r)
+        ref.append([-((g * np.cos(k * r)).sum(axis=1) @ q.real.astype(np.longdouble)),
+                    -((g * np.sin(k * r)).sum(axis=1) @ q.real.astype(np.longdouble))])
+    ref = np.array(ref)
+    error = got[at].real - ref[:, 0]
+    assert np.linalg.norm(error.astype(float)) <= \
+        U / np.sqrt(3.0) * np.sqrt(S / 16 / 3) / 2 * np.linalg.norm(ref[:, 0].astype(float))
