@@ -689,7 +689,8 @@ void set_mesh(beat_b200_ctx *c, int V, const double *verts, int F, const int32_t
     upload(c->rule_start, rstart);
     c->npoints = (int64_t)rdata.size() / 5;  // coordinate by coordinate, so that a warp's points are coalesced
     std::vector<double> rsoa(rdata.size());
-    for (size_t i = 0; i < rdata.size(); ++i) rsoa[(i % 5) * c->npoints + i / 5] = rdata[i];
+    for (int d = 0; d < 5; ++d)
+        for (int64_t i = 0; i < c->npoints; ++i) rsoa[d * c->npoints + i] = rdata[5 * i + d];
     upload(c->rule_data, rsoa);
 }
 
