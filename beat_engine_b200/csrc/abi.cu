@@ -90,8 +90,9 @@ __global__ void export_matrix_kernel(const Cx<T> *A, int64_t ld, int n, double2 
     }
 }
 
+// (beside: other lanes of a sweep may be at work)
 void solve_core(beat_b200_ctx *c, double k, double eta, int R, const double *d_q, const beat_b200_opts &o,
-                double *d_x, beat_b200_diag *diag) {
+                double *d_x, beat_b200_diag *diag, bool beside) {
     BB_REQUIRE(c->F > 0, BEAT_B200_STATE, "no mesh: call beat_b200_set_mesh first");
     BB_REQUIRE(R >= 1, BEAT_B200_INVALID_ARG, "R must be >= 1");
     BB_REQUIRE(std::isfinite(k) && k != 0.0 && std::isfinite(eta), BEAT_B200_INVALID_ARG,
@@ -106,12 +107,20 @@ void solve_core(beat_b200_ctx *c, double k, double eta, int R, const double *d_q
     // One solve is queued as far as the refinement's first residual before the
     // host waits: the status words of the factorisation are read there (the
     // substitutions end whatever the factors hold), the stage times at the end.
+    // Beside other lanes the host waits for the assembly first: with every
+    // lane's factorisation queued behind its assembly, some lanes' assemblies
+    // began only when other lanes' factorisations had ended (18 and 50 ms into a
+    // sweep of six instead of 35 each), and the latency-bound factorisations no
+    // longer ran beside each other.  Six frequencies at F = 5,228 / 9,605 /
+    // 20,480: 29-33 / 77 / 285 ms without the wait, 21 / 57.5 / 275 with it; three
+    // uneven meshes of up to 6,000 faces, four frequencies each: 47 and 33.
     float ms_asm = 0, ms_sing = 0, ms_reg = 0, ms_lu = 0, ms_solve = 0, ms_ir = 0;
     assemble(c, k, eta, o.precision, R, d_q);
     apply_admittance_lhs(c, o.precision);  // A += B diag(a) P when an admittance is set
     if (o.precision != BEAT_B200_FP64)
         BB_CUDA(cudaMemcpyAsync(w.Aop.p, w.A.p, (size_t)n * w.ld * 8, cudaMemcpyDeviceToDevice, c->stream));
     BB_CUDA(cudaEventRecord(c->ev[4], c->stream));
+    if (beside) BB_CUDA(cudaEventSynchronize(c->ev[4]));
     lu_factor(c, o.precision, o.lu_block, o.lu_split_terms);
     BB_CUDA(cudaEventRecord(c->ev[5], c->stream));
     keep_status(c);
@@ -167,7 +176,7 @@ void solve_core(beat_b200_ctx *c, double k, double eta, int R, const double *d_q
     beat_b200_opts o64 = o;
     o64.precision = BEAT_B200_FP64;
     o64.lu_block = 128;
-    solve_core(c, k, eta, R, d_q, o64, d_x, diag);
+    solve_core(c, k, eta, R, d_q, o64, d_x, diag, beside);
     if (diag) {
         diag->ir_iterations = ir.iterations;
         diag->ir_converged = 0;
@@ -485,7 +494,7 @@ int32_t beat_b200_solve_device(beat_b200_ctx *c, double k, double eta, int32_t R
     return guarded(c, [&] {
         BB_REQUIRE(d_q && d_p, BEAT_B200_INVALID_ARG, "null device pointer");
         const beat_b200_opts o = resolve_opts(opts);
-        solve_core(c, k, eta, R, (const double *)d_q, o, (double *)d_p, diag);
+        solve_core(c, k, eta, R, (const double *)d_q, o, (double *)d_p, diag, false);
     });
 }
 
@@ -502,7 +511,7 @@ int32_t beat_b200_solve(beat_b200_ctx *c, double k, double eta, int32_t R, const
         DevBuf &out = w.io;
         out.alloc((size_t)c->V * R * 16);
         try {
-            solve_core(c, k, eta, R, w.q.as<double>(), o, out.as<double>(), diag);
+            solve_core(c, k, eta, R, w.q.as<double>(), o, out.as<double>(), diag, false);
             BB_CUDA(cudaMemcpyAsync(p_out, out.p, (size_t)c->V * R * 16, cudaMemcpyDeviceToHost, c->stream));
             BB_CUDA(cudaStreamSynchronize(c->stream));
         } catch (...) {
@@ -675,7 +684,7 @@ int32_t beat_b200_sweep_device(beat_b200_ctx *c, int32_t nfreq, const double *k_
         run_sweep(c, nfreq, sweep_lane_count(c, nfreq, o, R), [&](beat_b200_ctx *l, int f) {
             const double *q = (const double *)d_q + f * qs;
             double *p = (double *)d_p + f * ps;
-            solve_core(l, k_signed[f], eta_im[f], R, q, o, p, diags ? diags + f : nullptr);
+            solve_core(l, k_signed[f], eta_im[f], R, q, o, p, diags ? diags + f : nullptr, true);
             if (M > 0) farfield(l, k_signed[f], M, dirs, R, p, q, (double *)d_ff + f * fs, true);
         });
     });
@@ -698,7 +707,7 @@ int32_t beat_b200_sweep(beat_b200_ctx *c, int32_t nfreq, const double *k_signed,
             BB_CUDA(cudaMemcpyAsync(w.q.p, q + f * qs, qs * sizeof(double), cudaMemcpyHostToDevice, l->stream));
             w.io.alloc((ps + fs) * sizeof(double));
             double *dp = w.io.as<double>(), *dff = dp + ps;
-            solve_core(l, k_signed[f], eta_im[f], R, w.q.as<double>(), o, dp, diags ? diags + f : nullptr);
+            solve_core(l, k_signed[f], eta_im[f], R, w.q.as<double>(), o, dp, diags ? diags + f : nullptr, true);
             if (M > 0) farfield(l, k_signed[f], M, dirs, R, dp, w.q.as<double>(), dff, true);
             BB_CUDA(cudaMemcpyAsync(p_out + f * ps, dp, ps * sizeof(double), cudaMemcpyDeviceToHost, l->stream));
             if (M > 0)
@@ -757,7 +766,7 @@ int32_t beat_b200_sweep_batch(int32_t nmesh, beat_b200_ctx *const *ctxs, const i
             w.io.alloc((ps + fs) * sizeof(double));
             double *dp = w.io.as<double>(), *dff = dp + ps;
             solve_core(l, k_signed[m][f], eta_im[m][f], Rm, w.q.as<double>(), o[m], dp,
-                       diags && diags[m] ? diags[m] + f : nullptr);
+                       diags && diags[m] ? diags[m] + f : nullptr, true);
             if (M > 0) farfield(l, k_signed[m][f], M, dirs, Rm, dp, w.q.as<double>(), dff, true);
             BB_CUDA(cudaMemcpyAsync(p_out[m] + f * ps, dp, ps * sizeof(double), cudaMemcpyDeviceToHost, l->stream));
             if (M > 0)
@@ -792,7 +801,8 @@ int32_t beat_b200_sweep_batch_device(int32_t nmesh, beat_b200_ctx *const *ctxs, 
             const size_t qs = (size_t)cs[m]->F * Rm * 2, ps = (size_t)cs[m]->V * Rm * 2, fs = (size_t)M * Rm * 2;
             const double *qd = (const double *)d_q[m] + f * qs;
             double *pd = (double *)d_p[m] + f * ps;
-            solve_core(l, k_signed[m][f], eta_im[m][f], Rm, qd, o[m], pd, diags && diags[m] ? diags[m] + f : nullptr);
+            solve_core(l, k_signed[m][f], eta_im[m][f], Rm, qd, o[m], pd, diags && diags[m] ? diags[m] + f : nullptr,
+                       true);
             if (M > 0) farfield(l, k_signed[m][f], M, dirs, Rm, pd, qd, (double *)d_ff[m] + f * fs, true);
         });
     });
