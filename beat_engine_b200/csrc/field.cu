@@ -348,7 +348,8 @@ static StagedSources stage_sources(beat_b200_ctx *c, int M, const double *pts_ho
 }
 
 // The source range in as many parts as fill whole waves of resident CTAs best
-// (a part has at least four chunks): with 63 tiles of points and 444 CTAs
+// (a part has at least two chunks; with four, one point's gradient at F = 300
+// took 79 us instead of 76, ten points' 78 instead of 67): with 63 tiles of points and 444 CTAs
 // resident, 9 parts leave the second wave 28 % full (2.68 ms for the product
 // kernel above with one running sum), 7 make one wave (2.05 ms).
 struct SourceSplit {
@@ -359,7 +360,7 @@ template <typename K> static SourceSplit resident_split(const beat_b200_ctx *c, 
     int per_sm = 1;
     BB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, FLD_THREADS, 0));
     const int mt = (M + FLD_POINTS - 1) / FLD_POINTS, chunks = (S + FLD_CHUNK - 1) / FLD_CHUNK;
-    const int per = chunks_per_slice(mt, chunks, (int64_t)std::max(1, per_sm) * c->sm_count, 4) * FLD_CHUNK;
+    const int per = chunks_per_slice(mt, chunks, (int64_t)std::max(1, per_sm) * c->sm_count, 2) * FLD_CHUNK;
     return {dim3(mt, (S + per - 1) / per), per};
 }
 
@@ -787,6 +788,8 @@ void field_gradient(beat_b200_ctx *c, double k, int M, const double *pts_host, i
     const GradRule coarse = grad_rule(c->rule_pts, c->rule_w), fine = grad_rule(p4, w4);
     const int face_blocks = (int)(((int64_t)F * images.n + 255) / 256);
     const int parts = std::min(M, std::max(1, 8 * c->sm_count / face_blocks)), per = (M + parts - 1) / parts;
+    const int near_blocks = (int)std::min<int64_t>(
+        4 * c->sm_count, ((int64_t)M * F * images.n + FG_NEAR_WARPS - 1) / FG_NEAR_WARPS);  // a warp per possible pair
     struct {
         unsigned long long count;
         int err, pad;
@@ -800,7 +803,7 @@ void field_gradient(beat_b200_ctx *c, double k, int M, const double *pts_host, i
             st.pts, M, c->d_verts.as<double>(), c->d_faces.as<int>(), F, images, per, items, cap, d_count);
         BB_CUDA(cudaGetLastError());
         auto correct = [&](auto *kernel, int groups) {
-            kernel<<<dim3(4 * c->sm_count, groups), 32 * FG_NEAR_WARPS, 0, c->stream>>>(
+            kernel<<<dim3(near_blocks, groups), 32 * FG_NEAR_WARPS, 0, c->stream>>>(
                 st.pts, M, c->d_verts.as<double>(), c->d_faces.as<int>(), c->d_normals.as<double>(), F, N, images,
                 items, d_count, cap, reinterpret_cast<const double2 *>(p_dev), st.q, R, coarse, fine, k, out, d_err);
             BB_CUDA(cudaGetLastError());
